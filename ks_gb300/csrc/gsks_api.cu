@@ -414,6 +414,9 @@ int enqueue_fused(Ctx *c, const ks_t *ker, int m, int n, int k,
     return enqueue_split(c, ker, m, n, k, u, umap, XA, XA2, amap, nxa, XB, XB2, bmap, nxb,
                          w, wmap, hi, hj, s, stream_ordered_alloc, std::max(nrhs, 1));
   if (precision != GSKS_FP64) return GSKS_ERR_PRECISION;
+  if (sliced_takes(k))
+    return enqueue_sliced(c, ker, m, n, k, u, umap, XA, XA2, amap, nxa, XB, XB2, bmap, nxb,
+                          w, wmap, hi, hj, s, stream_ordered_alloc, std::max(nrhs, 1));
 
   Fp64Plan p = fp64_plan(m, n, k, c->num_sms);
   const size_t pbytes = p.partial_elems * sizeof(double) * (size_t)std::max(nrhs, 1);
