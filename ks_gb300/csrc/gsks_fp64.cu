@@ -121,14 +121,8 @@ int fp64_launch(const FusedArgs &a0, const Fp64Plan &p, double *u, const int *um
     case KS_EPANECHNIKOV: launch_tiles<KS_EPANECHNIKOV>(a, p.grid, s); break;
     default: return -1;
   }
-  fp64_reduce_launch(a.m, p.nsc, p.ldp, a.nrhs, a.rstride, a.partial, u, umap, s);
+  fp64_reduce<<<(a.m + 255) / 256, 256, 0, s>>>(a.m, p.nsc, p.ldp, a.nrhs, a.rstride, a.partial, u, umap);
   return 2;
-}
-
-void fp64_reduce_launch(int m, int nsc, int ldp, int R, long long rstride, const double *partial, double *u,
-                        const int *umap, cudaStream_t s)
-{
-  fp64_reduce<<<(m + 255) / 256, 256, 0, s>>>(m, nsc, ldp, R, rstride, partial, u, umap);
 }
 
 cudaError_t norms_launch(int N, int k, const double *X, double *X2, cudaStream_t s)

@@ -108,6 +108,23 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k,
                    const double *w, const int *wmap, const double *hi, const double *hj,
                    cudaStream_t s, bool stream_ordered_alloc, int nrhs);
 
+// The same for dgsks_list, planned once for a set of lists: row sums of every
+// (task t, target position r, source chunk sc) into partial[pbase[t] + sc * m_t
+// + r].  kps: ntask device-side descriptors; hoff_a / hoff_b: host offsets.
+// sliced_list_run takes device pointers and only launches kernels.
+struct SlicedListPlan {
+  int ntask = 0, k = 0, kpad = 0, n_ta = 0, n_tb = 0, n_items = 0;
+  bool any_gauss = false;
+  DevBuf ws;
+  size_t o_next = 0, o_ta = 0, o_tat = 0, o_tb = 0, o_tbt = 0, o_items = 0, o_tg = 0, o_tp = 0;
+  size_t o_aa = 0, o_hi = 0, o_e = 0, o_a = 0, o_b = 0;
+};
+int sliced_list_plan(SlicedListPlan &P, const KParams *kps, int ntask, int k, const int *hoff_a, const int *hoff_b,
+                     const long long *pbase, int chunk, cudaStream_t s);
+int sliced_list_run(const SlicedListPlan &P, Ctx *c, const double *XA, const double *XA2, const int *a_idx, int nxa,
+                    const double *XB, const double *XB2, const int *b_idx, int nxb, const double *w, const int *w_idx,
+                    double *partial, int *err, cudaStream_t s, int *launches);
+
 // Split-precision form (gsks_split.cu).  nrhs <= 4 interleaved columns of u
 // and w in one sweep; GSKS_ERR_TOO_LARGE when k or the shared memory of that
 // sweep does not fit (the caller then sweeps once per column).

@@ -139,10 +139,6 @@ struct Fp64Plan {
 Fp64Plan fp64_plan(int m, int n, int k, int num_sms);
 int fp64_launch(const FusedArgs &a, const Fp64Plan &p, double *u, const int *umap,
                 cudaStream_t s);
-// u[umap[i] R + q] += the nsc partials of row i and column q (ldp and rstride
-// apart), in order.
-void fp64_reduce_launch(int m, int nsc, int ldp, int R, long long rstride, const double *partial, double *u,
-                        const int *umap, cudaStream_t s);
 cudaError_t norms_launch(int N, int k, const double *X, double *X2, cudaStream_t s);
 
 }  // namespace gsks

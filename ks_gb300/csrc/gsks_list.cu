@@ -10,8 +10,9 @@
 // positions that name it in ascending position order -- the same order on
 // every run, so the result is deterministic without floating-point atomics.
 // With the split-precision form selected, the same partial layout is filled
-// by the tensor-core kernel of gsks_split.cu (split_list_run) and merged by
-// the same merge kernel.  A plan (gsks_list_plan_*) keeps the lists' tables
+// by the tensor-core kernel of gsks_split.cu (split_list_run), in the FP64 form
+// up to k = 1024 by that of gsks_sliced.cu (sliced_list_run); the same merge
+// kernel adds them up.  A plan (gsks_list_plan_*) keeps the lists' tables
 // on the device and replays its evaluation as a CUDA graph.
 #include "gsks.h"
 #include "gsks_internal.cuh"
@@ -131,6 +132,8 @@ struct ListPlan {
   DevBuf XA2, XB2;                      // norms computed on the device
   std::vector<DevBuf> bandwidths;       // device copies of host bandwidth arrays
   SplitListPlan sp;
+  SlicedListPlan lp;                    // FP64 on the tensor cores (sliced)
+  bool sliced = false;
   // graph of the last run: replayed while the pointers and the stream stay the same
   cudaGraphExec_t gexec = nullptr;
   const void *gkey[7] = {};
@@ -139,7 +142,7 @@ struct ListPlan {
     if (gexec) cudaGraphExecDestroy(gexec);
     gexec = nullptr;
     for (DevBuf *b : {&items, &tasks, &kps, &counter, &partial, &ent_u, &own_off, &own_pos, &sort_work, &a_off,
-                      &err, &l_a, &l_b, &l_w, &l_u, &XA2, &XB2, &sp.ws})
+                      &err, &l_a, &l_b, &l_w, &l_u, &XA2, &XB2, &sp.ws, &lp.ws})
       b->release();
     for (auto &b : bandwidths) b.release();
     bandwidths.clear();
@@ -158,6 +161,7 @@ int list_plan_build(ListPlan &L, Ctx *c, ks_t *kernel, ks_t *kernels, int ntask,
   if (L.gexec) { cudaGraphExecDestroy(L.gexec); L.gexec = nullptr; }
   L.ntask = ntask; L.k = k; L.nu = nu; L.nxa = nxa; L.nxb = nxb; L.nw = nw;
   L.split = prec == GSKS_SPLIT_BF16X3;
+  L.sliced = !L.split && sliced_takes(k);
   L.per_task = kernels != nullptr;
   L.same_pool = same_pool;
   if (!u_idx) u_idx = a_idx;
@@ -245,7 +249,7 @@ int list_plan_build(ListPlan &L, Ctx *c, ks_t *kernel, ks_t *kernels, int ntask,
     const int m = hoff_a[t + 1] - hoff_a[t], n = hoff_b[t + 1] - hoff_b[t];
     const int nsc = (m > 0 && n > 0) ? (n + LIST_CHUNK - 1) / LIST_CHUNK : 0;
     tasks[t] = ListTask{pbase, m, nsc};
-    if (L.split) { pbase += (long long)nsc * m; continue; }   // the split form plans its own items
+    if (L.split || L.sliced) { pbase += (long long)nsc * m; continue; }   // these plan their own items
     for (int sc = 0; sc < nsc; sc++)
       for (int i0 = 0; i0 < m; i0 += fp64cfg::BM) {
         ListItem it{};
@@ -270,7 +274,7 @@ int list_plan_build(ListPlan &L, Ctx *c, ks_t *kernel, ks_t *kernels, int ntask,
   }
   L.pbase = pbase;
   L.nitems = (int)items.size();
-  bool ok = (L.split || upload(L.items, items.data(), items.size(), s)) &&
+  bool ok = (L.split || L.sliced || upload(L.items, items.data(), items.size(), s)) &&
             upload(L.tasks, tasks.data(), tasks.size(), s) && upload(L.kps, kps.data(), kps.size(), s) &&
             upload(L.a_off, hoff_a.data(), (size_t)ntask + 1, s) &&
             L.partial.ensure(std::max<long long>(pbase, 1) * sizeof(double)) && L.counter.ensure(2 * sizeof(int)) &&
@@ -285,12 +289,14 @@ int list_plan_build(ListPlan &L, Ctx *c, ks_t *kernel, ks_t *kernels, int ntask,
                                (int *)L.own_off.p, (int *)L.counter.p + 1, (int *)L.err.p, s, launches);
     if (st) return st;
   }
-  if (L.split) {
+  if (L.split || L.sliced) {
     std::vector<KParams> kpt(ntask);
     std::vector<long long> pb(ntask);
     for (int t = 0; t < ntask; t++) { kpt[t] = kps[kernels ? t : 0]; pb[t] = tasks[t].pbase; }
-    const int st = split_list_plan(L.sp, kpt.data(), ntask, k, hoff_a.data(), hoff_b.data(), pb.data(), LIST_CHUNK,
-                                   nxa, nxb, same_pool, s);
+    const int st = L.split ? split_list_plan(L.sp, kpt.data(), ntask, k, hoff_a.data(), hoff_b.data(), pb.data(),
+                                             LIST_CHUNK, nxa, nxb, same_pool, s)
+                           : sliced_list_plan(L.lp, kpt.data(), ntask, k, hoff_a.data(), hoff_b.data(), pb.data(),
+                                              LIST_CHUNK, s);
     if (st) return st;
   }
   // the host vectors above die here: every copy from them must have left
@@ -309,7 +315,7 @@ int list_plan_run(ListPlan &L, Ctx *c, double *u, const double *XA, const double
     const int st = split_list_run(L.sp, c, XA, L.a_idx, XB, L.b_idx, w, L.w_idx, (double *)L.partial.p, err, s,
                                   launches);
     if (st) return st;
-  } else if (L.nitems > 0) {
+  } else if (L.sliced ? L.lp.n_items > 0 : L.nitems > 0) {
     const double *dXA2 = nullptr, *dXB2 = nullptr;
     if (L.any_norms) {
       // caller-supplied norms are used as given; missing ones are computed on
@@ -320,6 +326,11 @@ int list_plan_run(ListPlan &L, Ctx *c, double *u, const double *XA, const double
       else if (XB2) dXB2 = XB2;
       else { norms_launch(L.nxb, L.k, XB, (double *)L.XB2.p, s); (*launches)++; dXB2 = (const double *)L.XB2.p; }
     }
+    if (L.sliced) {
+      const int st = sliced_list_run(L.lp, c, XA, dXA2, L.a_idx, L.nxa, XB, dXB2, L.b_idx, L.nxb, w, L.w_idx,
+                                     (double *)L.partial.p, err, s, launches);
+      if (st) return st;
+    } else {
     FusedArgs a{};
     a.k = L.k; a.XA = XA; a.XA2 = dXA2; a.amap = L.a_idx; a.XB = XB; a.XB2 = dXB2; a.bmap = L.b_idx;
     a.w = w; a.wmap = L.w_idx; a.nxa = L.nxa; a.nxb = L.nxb; a.err = err;
@@ -329,6 +340,7 @@ int list_plan_run(ListPlan &L, Ctx *c, double *u, const double *XA, const double
                                                   (const ListItem *)L.items.p, L.nitems, (int *)L.counter.p,
                                                   (double *)L.partial.p);
     *launches += 2;
+    }
   }
   if (na > 0) {
     list_merge<<<(na + 127) / 128, 128, 0, s>>>((const int *)L.counter.p + 1, (const int *)L.ent_u.p,

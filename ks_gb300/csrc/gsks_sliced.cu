@@ -29,19 +29,28 @@
 // the range of their norms), slice_kernel (the digits, written as tile images
 // in the layout the MMA reads, one block per 32 points).  Then sliced_tiles,
 // one persistent CTA of 18 warps per SM over items (target tile of 128, run of
-// source tiles of 64):
+// source tiles of 32):
 //   warp 0       bulk copies: the target tile resident for k <= 64 (96 KB at
-//                k = 64), source tiles through two stages; beyond k = 64 both
-//                operands in 32-wide chunks
-//   warp 1       MMA issue: 21 tcgen05.mma (M 128, N 64) per 16 coordinates
-//                into six accumulators (384 TMEM columns)
-//   warps 2..17  epilogue: each 32 rows x 16 columns; the accumulators become
-//                16 integers W per thread, the tensor memory is handed back,
-//                and the kernel values are formed while the next tile's
-//                products run
-// Each epilogue group writes its own row sums, one per (row, run, group);
-// fp64_reduce adds them in a fixed order (deterministic).  Every wait is
-// bounded, as in gsks_split.cu.
+//                k = 64), source tiles through four stages; beyond k = 64 two
+//                source tiles and the targets in 32-wide chunks
+//   warp 1       MMA issue: the source slices lie stacked along N, so that
+//                target slice i times slices 0 .. 5 - i is one tcgen05.mma of
+//                N = 32 (6 - i) whose columns are the accumulators of levels
+//                i .. 5: six instructions per 16 coordinates, each target
+//                slice read once (21 of N = 64 read it six times over and took
+//                4032 SM cycles of shared-memory bandwidth per 64 columns at
+//                k = 64 where these take 2816)
+//   warps 2..17  epilogue, in two halves of eight, each with an accumulator
+//                buffer (192 TMEM columns) of its own: a half turns its
+//                accumulators into integers W (bound by the float-to-integer
+//                conversions, 16 per SM cycle) while the other forms kernel
+//                values (bound by the FP64 pipe) and the tensor cores fill the
+//                buffer handed back
+// A work item's row sums (the four groups' in order) go to one partial per (row,
+// run) -- with several right-hand sides one per group too -- and the last of a
+// row's runs to arrive adds them in run order (deterministic).  Every wait is
+// bounded, as in gsks_split.cu; no wait is on another CTA.  The batched form (KS_LIST) runs the same kernels over tables of
+// tiles and items from many tasks, each with its own kernel and frame.
 #include "gsks.h"
 #include "gsks_internal.cuh"
 #include "gsks_host.h"
@@ -50,20 +59,26 @@
 
 #include <cuda_fp16.h>
 #include <algorithm>
+#include <climits>
 #include <cmath>
+#include <cstring>
+#include <vector>
 
 namespace gsks {
 namespace sliced {
 
 using namespace sm100;
 
-constexpr int GROUPS = 4;                        // column groups of the epilogue
-constexpr int COLS = BN / GROUPS;                // columns per thread and tile
+constexpr int GROUPS = 4;                        // epilogue groups of four warps
+constexpr int HALVES = 2;                        // accumulator buffers, each with two of the groups
+constexpr int COLS = BN * HALVES / GROUPS;       // columns per thread and tile
 constexpr int EPI_WARPS = 4 * GROUPS;
+constexpr int HALF_WARPS = EPI_WARPS / HALVES;
 constexpr int NTHREADS = 32 * (2 + EPI_WARPS);
-constexpr int NMETA = 3;                         // source metadata slots
-constexpr int NSTAGE = 2;                        // operand stages
-constexpr uint32_t TMEM_COLS = 512;              // six accumulators of 64 columns (allocation: a power of two)
+constexpr int NMETA = 4;                         // source metadata slots
+constexpr int NSTAGE_RES = 4, NSTAGE_STR = 2;    // operand stages (resident, streaming)
+constexpr uint32_t TMEM_COLS = 512;              // two buffers of six accumulators (allocation: a power of two)
+constexpr uint32_t TBUF = NS * BN;               // columns of one buffer
 constexpr size_t SMEM_MAX = 232448;
 constexpr long long WAIT_LIMIT = 1LL << 32;      // clock cycles (~2 s) per wait
 
@@ -74,9 +89,34 @@ static __device__ const ExpTable g_exp_table = ExpTable();
 struct CallParam {
   int fixed;             // the fixed-point form applies
   int e, F;
-  int shl;               // 53 - F: y to units of 2^-53
-  int lim, end;          // high words of 1021 2^F and (at most 2^31 - 1) of 1088 2^F
+  int pre;               // left shift of y where F is below 43 (exp2_neg's least), else 0
+  int lim, end;          // high words of 1021 2^F and 1088 2^F, at most 2^31 - 1
   double alpha, ah, al;  // alpha^2 = ah + al
+};
+
+// Kernel selector of the batched (list) form: the epilogue dispatches on each
+// task's type.
+constexpr int KS_LIST = 99;
+
+// One task of the list form (copied into shared memory with its items): the
+// kernel and the Gaussian's frame from the task's own points.
+struct __align__(16) TaskParam {
+  KParams kp;
+  CallParam cp;
+};
+static_assert(sizeof(TaskParam) % 16 == 0, "TaskParam is copied by the bulk-copy engine");
+
+// One work item of the list form: target tile a_tile (list positions ia ..
+// ia + rows - 1), source tiles b0 .. b1 - 1 (positions jb .. jb + cols - 1); the
+// row sums go to partial[out + row].
+struct Item {
+  int a_tile, rows, ia, b0, b1, jb, cols, task;
+  long long out;
+};
+
+// One task's target and source list positions.
+struct TaskGeo {
+  int a0, m, b0, n;
 };
 
 // One block's share of the scan: largest |coordinate| (as ordered bits), the
@@ -87,19 +127,28 @@ struct ScanPart {
   int bad, pad;
 };
 constexpr int SCAN_MAX = 256;
+// Coordinates up to which every block of slice_kernel scans all points itself
+// (32 loads a thread) instead of a launch of its own.
+constexpr long long SCAN_SELF = 8192;
 
 struct SliceArgs {
   int m, n, k, kpad, kt, nrhs, nr;
   const double *XA, *XA2, *hi; const int *amap; int nxa;
   const double *XB, *XB2, *hj; const int *bmap; int nxb;
   const double *w; const int *wmap;
-  double scal;
+  CallParam frame;         // gauss_frame of the call
   uint8_t *imgA, *imgB;
-  double *row_aa, *row_hi; int *row_e;
-  const ScanPart *scan; int nscan;
+  double *row_aa, *row_hi; int *row_e, *row_n;
+  const ScanPart *scan; int nscan;   // partials; 0: few points, -1: no Gaussian
   CallParam *cp;
   int *next_item;
   int *err;
+  // list form: tile t of a side packs list positions tiles[t].x .. + tiles[t].y - 1
+  // of task tile_task[t]
+  const int2 *tilesA, *tilesB;
+  const int *taskA, *taskB;
+  const TaskParam *tp;
+  int nta;                 // target tiles
 };
 
 // k coordinates are processed in chunks: the whole padded k when the target
@@ -124,75 +173,141 @@ __device__ __forceinline__ int pool_index(const int *map, int pos, int npool, in
   return p;
 }
 
-// ---------------------------------------------------------------------------
-// Largest |coordinate| and norm range of the gathered points (one warp per
-// point): HBM-bound, 8 k bytes a point.
-__global__ void __launch_bounds__(256) scan_kernel(SliceArgs a, ScanPart *__restrict__ part)
+// Programmatic dependent launch: a kernel launched with launch_after may start
+// when every block of the one before it has called launch_dependents, and
+// calls wait_primary before it touches anything that one reads or writes.  It
+// overlaps launch and set-up (tensor memory, barriers, the table) with the
+// preparation: calls of a few tens of microseconds gain.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_primary() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... A>
+cudaError_t launch_after(void (*kernel)(A...), int grid, int block, size_t smem, cudaStream_t s, A... args)
 {
-  __shared__ unsigned long long s_mx[8];
-  __shared__ double s_lo[8], s_hi[8];
-  __shared__ int s_bad[8];
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  unsigned long long mx = 0;
-  double lo = 1e300, hi = -1e300;
-  bool bad = false;
-  for (int i = blockIdx.x * 8 + wp; i < a.m + a.n; i += gridDim.x * 8) {
-    const bool A = i < a.m;
-    const int p = A ? pool_index(a.amap, i, a.nxa, a.err) : pool_index(a.bmap, i - a.m, a.nxb, a.err);
-    const double *x = (A ? a.XA : a.XB) + (size_t)p * a.k;
-    for (int c = lane; c < a.k; c += 32)
-      mx = max(mx, (unsigned long long)__double_as_longlong(x[c]) & 0x7fffffffffffffffull);
-    const double nn = A ? a.XA2[p] : a.XB2[p];
-    bad |= !(nn >= 0.0 && nn < 1e300);
-    lo = fmin(lo, nn);
-    hi = fmax(hi, nn);
-  }
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, args...);
+}
+
+// ---------------------------------------------------------------------------
+// A block's fold of its threads' scan values (256 threads, every thread calls;
+// the result in every thread).
+__device__ __forceinline__ ScanPart scan_fold(ScanPart r)
+{
+  __shared__ ScanPart part[8];
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
-    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    r.maxabs = max(r.maxabs, __shfl_xor_sync(0xffffffffu, r.maxabs, o));
+    r.nmin = fmin(r.nmin, __shfl_xor_sync(0xffffffffu, r.nmin, o));
+    r.nmax = fmax(r.nmax, __shfl_xor_sync(0xffffffffu, r.nmax, o));
   }
-  bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) { s_mx[wp] = mx; s_lo[wp] = lo; s_hi[wp] = hi; s_bad[wp] = bad; }
+  r.bad = __any_sync(0xffffffffu, r.bad);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = r;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    ScanPart r{0, 1e300, -1e300, 0, 0};
-    for (int q = 0; q < 8; q++) {
-      r.maxabs = max(r.maxabs, s_mx[q]);
-      r.nmin = fmin(r.nmin, s_lo[q]);
-      r.nmax = fmax(r.nmax, s_hi[q]);
-      r.bad |= s_bad[q];
-    }
-    part[blockIdx.x] = r;
+  r = part[0];
+#pragma unroll
+  for (int q = 1; q < 8; q++) {
+    r.maxabs = max(r.maxabs, part[q].maxabs);
+    r.nmin = fmin(r.nmin, part[q].nmin);
+    r.nmax = fmax(r.nmax, part[q].nmax);
+    r.bad |= part[q].bad;
   }
+  return r;
+}
+
+// Scan values of points first, first + step, ... of a target list (m positions
+// of amap from a0) followed by a source list (n of bmap from b0): the block's
+// threads take one coordinate of every (256 / k)-th point (a point at a time for
+// long rows).
+__device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int m, int b0, int n, int first, int step)
+{
+  ScanPart r{0, 1e300, -1e300, 0, 0};
+  const int lanes = min(a.k, 256), per = 256 / lanes, c0 = threadIdx.x % lanes, sub = threadIdx.x / lanes;
+  if (sub < per) {
+#pragma unroll 4
+    for (int i = first * per + sub; i < m + n; i += step * per) {
+      const bool A = i < m;
+      const int p = A ? pool_index(a.amap, a0 + i, a.nxa, a.err) : pool_index(a.bmap, b0 + i - m, a.nxb, a.err);
+      const double *x = (A ? a.XA : a.XB) + (size_t)p * a.k;
+      for (int c = c0; c < a.k; c += lanes)
+        r.maxabs = max(r.maxabs, (unsigned long long)__double_as_longlong(x[c]) & 0x7fffffffffffffffull);
+      if (c0 == 0) {
+        const double nn = A ? a.XA2[p] : a.XB2[p];
+        r.bad |= !(nn >= 0.0 && nn < 1e300);
+        r.nmin = fmin(r.nmin, nn);
+        r.nmax = fmax(r.nmax, nn);
+      }
+    }
+  }
+  return r;
+}
+
+// Largest |coordinate| and norm range of the call's points: HBM-bound, 8 k bytes
+// a point.
+__global__ void __launch_bounds__(256) scan_kernel(SliceArgs a, ScanPart *__restrict__ part)
+{
+  launch_dependents();
+  const ScanPart r = scan_fold(scan_points(a, 0, a.m, 0, a.n, blockIdx.x, gridDim.x));
+  if (threadIdx.x == 0) part[blockIdx.x] = r;
+}
+
+__device__ CallParam call_param(const ScanPart &s, CallParam c, int kpad);
+
+// The same over one task's points, one block per Gaussian task: its frame.
+__global__ void __launch_bounds__(256) list_scan_kernel(SliceArgs a, int ntask, const TaskGeo *__restrict__ tg,
+                                                        TaskParam *__restrict__ tp)
+{
+  const int t = blockIdx.x;
+  launch_dependents();
+  if (t == 0 && threadIdx.x == 0) *a.next_item = 0;
+  if (t >= ntask || tp[t].kp.type != KS_GAUSSIAN) return;
+  const TaskGeo G = tg[t];
+  const ScanPart r = scan_fold(scan_points(a, G.a0, G.m, G.b0, G.n, 0, 1));
+  if (threadIdx.x == 0) tp[t].cp = call_param(r, tp[t].cp, a.kpad);
 }
 
 // The Gaussian's frame from the points' range.  The form applies when every
 // value is finite, the exponent leaves 33 <= F, the norms fit their points,
 // and an absolute error of a few 2^-F in y is no more than FP64's own rounding
 // of the pairs' norms: F >= 52, or every norm sum at least 2^(52 - F).
-__device__ CallParam call_param(const ScanPart &s, double scal, int kpad)
+// c: alpha, ah, al set (gauss_frame), the rest filled in.
+__device__ CallParam call_param(const ScanPart &s, CallParam c, int kpad)
 {
-  CallParam c;
-  c.fixed = 0; c.e = 0; c.F = 0; c.shl = 0; c.lim = 0; c.end = 0;
-  const double c2 = -scal * 1.4426950408889634;     // y = c2 d^2
+  auto pow2 = [](int e) { return __hiloint2double((1023 + e) << 20, 0); };
+  c.fixed = 0;
+  const double mx = __longlong_as_double((long long)s.maxabs) * c.alpha;
+  if (c.alpha == 0.0 || s.bad || !(mx < 0x1p30)) return c;
+  // e as low as the points allow (mx < 2^e), F = 51 + g - 2 e at most 62
+  const int g = guard_bits(kpad);
+  c.e = max((g - 11 + 1) / 2, (__double2hiint(mx) >> 20) - 1022);
+  c.F = 51 + g - 2 * c.e;
+  if (c.F < 33) return c;
+  if (s.nmax * c.ah > (double)kpad * pow2(2 * c.e)) return c;
+  if (c.F < 52 && 2.0 * s.nmin * c.ah < pow2(52 - c.F)) return c;
+  c.pre = max(0, 43 - c.F);
+  c.lim = c.F < 54 ? (int)(1021u << (c.F - 32)) : 0x7fffffff;
+  c.end = c.F < 53 ? (int)(1088u << (c.F - 32)) : 0x7fffffff;
+  c.fixed = 1;
+  return c;
+}
+
+// The part of the frame that the kernel alone sets: y = alpha^2 d2 (alpha 0: not
+// a decaying Gaussian, no fixed-point form).
+CallParam gauss_frame(double scal)
+{
+  CallParam c{};
+  const double c2 = -scal * 1.4426950408889634;
+  if (!(c2 > 0x1p-300 && c2 < 0x1p300)) return c;
   c.alpha = sqrt(c2);
   c.ah = c.alpha * c.alpha;
   c.al = fma(c.alpha, c.alpha, -c.ah);
-  const double mx = __longlong_as_double((long long)s.maxabs) * c.alpha;
-  if (!(c2 > 0.0 && c2 < 1e100) || s.bad || !(mx < 0x1p30)) return c;
-  int e = max(0, (guard_bits(kpad) - 1) / 2);       // F at most 53
-  while (mx >= ldexp(1.0, e)) e++;
-  c.e = e;
-  c.F = 51 + guard_bits(kpad) - 2 * e;
-  if (c.F < 33 || c.F > 53) return c;
-  if (s.nmax * c.ah > (double)kpad * ldexp(1.0, 2 * e)) return c;
-  if (c.F < 52 && 2.0 * s.nmin * c.ah < ldexp(1.0, 52 - c.F)) return c;
-  c.shl = 53 - c.F;
-  c.lim = (int)(1021u << (c.F - 32));
-  c.end = (int)min(1088u << (c.F - 32), 0x7fffffffu);
-  c.fixed = 1;
   return c;
 }
 
@@ -236,33 +351,24 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
 {
   __shared__ uint32_t s_max[8][32];
   __shared__ CallParam s_cp;
-  __shared__ ScanPart s_part[8];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-  const int nbA = (a.m + BM - 1) / BM * (BM / 32);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.next_item = 0;
+  const int nbA = a.nta * (BM / 32);
+  launch_dependents();
+  wait_primary();
+  const bool listed = a.tp != nullptr;
   bool fixed = false;
-  if (a.nscan > 0) {
-    // every block folds the scan's partials (at most one per thread)
+  if (!listed && blockIdx.x == 0 && threadIdx.x == 0) *a.next_item = 0;
+  if (listed) {
+    // (below, from the tile's task)
+  } else if (a.nscan >= 0) {
+    // every block folds the scan's partials (at most one per thread) or, for
+    // few points, scans them all itself
     ScanPart r{0, 1e300, -1e300, 0, 0};
-    if ((int)threadIdx.x < a.nscan) r = a.scan[threadIdx.x];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      r.maxabs = max(r.maxabs, __shfl_xor_sync(0xffffffffu, r.maxabs, o));
-      r.nmin = fmin(r.nmin, __shfl_xor_sync(0xffffffffu, r.nmin, o));
-      r.nmax = fmax(r.nmax, __shfl_xor_sync(0xffffffffu, r.nmax, o));
-      r.bad |= __shfl_xor_sync(0xffffffffu, r.bad, o);
-    }
-    if (lane == 0) s_part[wp] = r;
-    __syncthreads();
+    if (a.nscan == 0) r = scan_points(a, 0, a.m, 0, a.n, 0, 1);
+    else if ((int)threadIdx.x < a.nscan) r = a.scan[threadIdx.x];
+    r = scan_fold(r);
     if (threadIdx.x == 0) {
-      r = s_part[0];
-      for (int q = 1; q < 8; q++) {
-        r.maxabs = max(r.maxabs, s_part[q].maxabs);
-        r.nmin = fmin(r.nmin, s_part[q].nmin);
-        r.nmax = fmax(r.nmax, s_part[q].nmax);
-        r.bad |= s_part[q].bad;
-      }
-      s_cp = call_param(r, a.scal, a.kpad);
+      s_cp = call_param(r, a.frame, a.kpad);
       if (blockIdx.x == 0) *a.cp = s_cp;
     }
     __syncthreads();
@@ -275,8 +381,23 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
   const int blk = side ? blockIdx.x - nbA : blockIdx.x;
   const int rows = side ? BN : BM, per = rows / 32;       // rows per tile, blocks per tile
   const int tile = blk / per, r = (blk - tile * per) * 32 + lane;
-  const int pt = tile * rows + r;
-  const bool valid = pt < (side ? a.n : a.m);
+  int pt = tile * rows + r, kt = a.kt;     // position in the call's maps
+  bool valid = pt < (side ? a.n : a.m);
+  const int slot = pt;                     // row of the metadata
+  const double *hv = side ? a.hj : a.hi;
+  if (listed) {
+    const int2 tl = side ? a.tilesB[tile] : a.tilesA[tile];
+    const TaskParam *T = a.tp + (side ? a.taskB[tile] : a.taskA[tile]);
+    pt = tl.x + r;
+    valid = r < tl.y;
+    kt = T->kp.type;
+    hv = side ? T->kp.hj : T->kp.hi;
+    if (kt == KS_GAUSSIAN) {
+      if (threadIdx.x == 0) s_cp = T->cp;
+      __syncthreads();
+      fixed = s_cp.fixed != 0;
+    }
+  }
   const int p = valid ? (side ? pool_index(a.bmap, pt, a.nxb, a.err) : pool_index(a.amap, pt, a.nxa, a.err)) : 0;
   const double *x = (side ? a.XB : a.XA) + (size_t)p * a.k;
   const double mul = fixed ? s_cp.alpha : 1.0;
@@ -332,30 +453,33 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     uint4 out[NS];
     slice8(v, e, !flag, out);
     const int c = kg / gpc, kgc = kg - c * gpc;
-    uint8_t *dst = base + (size_t)c * op_bytes(rows, kc) + (size_t)kgc * rows * 16 + (size_t)r * 16;
+    // targets: slice, then k-group, row; sources: k-group, then slice, row
+    uint8_t *dst = base + (size_t)c * op_bytes(rows, kc) + (size_t)kgc * (side ? NS : 1) * rows * 16 + (size_t)r * 16;
+    const size_t step = side ? (size_t)rows * 16 : (size_t)rows * kc * 2;
 #pragma unroll
-    for (int s = 0; s < NS; s++) *(uint4 *)(dst + (size_t)s * rows * kc * 2) = out[s];
+    for (int s = 0; s < NS; s++) *(uint4 *)(dst + s * step) = out[s];
   }
 
   if (wp == 0) {
-    const bool norms = kt_uses_norms(a.kt), varbw = a.kt == KS_GAUSSIAN_VAR_BANDWIDTH;
+    const bool norms = kt_uses_norms(kt), varbw = kt == KS_GAUSSIAN_VAR_BANDWIDTH;
     double nn = (valid && norms) ? (side ? a.XB2[p] : a.XA2[p]) : 0.0;
     if (fixed) {
       const double y = fma(nn, s_cp.ah, nn * s_cp.al) * ldexp(1.0, s_cp.F);
       nn = __longlong_as_double(__double2ll_rn(y));
     }
-    const double h = (valid && varbw) ? (side ? a.hj[p] : a.hi[p]) : 0.0;
+    const double h = (valid && varbw) ? hv[p] : 0.0;
     if (!side) {
-      a.row_aa[pt] = nn;
-      a.row_hi[pt] = h;
-      a.row_e[pt] = flag ? EFLAG : e;
+      a.row_aa[slot] = nn;
+      a.row_hi[slot] = h;
+      a.row_e[slot] = flag ? EFLAG : e;
+      if (a.row_n) a.row_n[slot] = 0;
     } else {
       ColMeta *cm = (ColMeta *)(base + op_bytes(BN, a.kpad));
       cm->bb[r] = nn;
       cm->hj[r] = h;
       cm->e[r] = flag ? EFLAG : e;
       const bool any = __any_sync(0xffffffffu, flag);
-      if (lane == 0) { cm->flag[r >> 5] = any ? 1 : 0; cm->pad[r >> 5] = 0; }
+      if (lane == 0) { cm->flag = any ? 1 : 0; cm->pad[0] = cm->pad[1] = cm->pad[2] = 0; }
       const size_t wi = valid ? (size_t)(a.wmap ? a.wmap[pt] : pt) * a.nrhs : 0;
       for (int q = 0; q < a.nr; q++) cm->w[q][r] = (valid && q < a.nrhs) ? a.w[wi + q] : 0.0;
     }
@@ -373,18 +497,46 @@ struct TileArgs {
   int nxa, nxb;
   KParams kp;
   const CallParam *cp;
-  double *partial;                  // [nrhs][nsc][GROUPS][ldp]
+  double *partial;                  // [nsc][ldp]; several right-hand sides: [nrhs][nsc][GROUPS][ldp]
+  int *row_n;                       // arrivals per row (nullptr: the list form)
+  double *u; const int *umap;
   int ldp;
   int *err, *next_item;
   long long wait_limit;
+  // list form
+  const Item *tab;
+  int ntab;
+  const TaskParam *tp;
 };
 
-struct SlicedSmem {
+// Geometry of a work item: target tile, source tiles, list positions of its
+// first row and column and how many are valid, the partial offset of row 0.
+__device__ __forceinline__ Item item_geo(const TileArgs &a, int item)
+{
+  if (a.tab) return a.tab[item];
+  Item g;
+  g.a_tile = item % a.ntm;
+  const int sc = item / a.ntm;
+  g.b0 = sc * a.chunk_tiles;
+  g.b1 = min(a.ntn, g.b0 + a.chunk_tiles);
+  g.ia = g.a_tile * BM;
+  g.rows = min(BM, a.m - g.ia);
+  g.jb = g.b0 * BN;
+  g.cols = a.n - g.jb;
+  g.task = 0;
+  g.out = (long long)sc * a.ldp + g.ia;
+  return g;
+}
+
+struct __align__(16) SlicedSmem {
   uint64_t a_full, a_empty;
-  uint64_t b_full[NSTAGE], b_empty[NSTAGE];
+  uint64_t b_full[NSTAGE_RES], b_empty[NSTAGE_RES];
   uint64_t m_full[NMETA], m_empty[NMETA];
-  uint64_t t_full, t_empty;
+  uint64_t t_full[HALVES], t_empty[HALVES];
+  uint64_t r_full[2], r_empty[2];       // row-sum exchange of the epilogue groups, by item parity
   uint64_t drain;
+  double rsum[2][GROUPS - 1][BM];       // row sums of groups 1 .., by item parity
+  TaskParam tslot[2];                   // list form: the items' task parameters, by item parity
   uint32_t tmem_base;
   int abort;
   int never;             // stays 0: an abort flag for the drain waits
@@ -394,7 +546,8 @@ struct SlicedSmem {
 struct SmemLayout {
   bool resident;
   int kc, nch;               // k-chunk, chunks per tile
-  size_t a_chunk, b_chunk;   // operand bytes of one chunk
+  int nstage;
+  size_t a_chunk, b_chunk;   // operand bytes of one chunk (one source tile)
   size_t a_region, stage, meta, table;
 };
 __host__ __device__ inline SmemLayout smem_layout(int kpad, int nr, bool table)
@@ -403,52 +556,46 @@ __host__ __device__ inline SmemLayout smem_layout(int kpad, int nr, bool table)
   L.kc = kchunk(kpad);
   L.nch = kpad / L.kc;
   L.resident = L.nch == 1;
+  L.nstage = L.resident ? NSTAGE_RES : NSTAGE_STR;
   L.a_chunk = op_bytes(BM, L.kc);
   L.b_chunk = op_bytes(BN, L.kc);
   L.a_region = L.resident ? L.a_chunk : 0;
-  L.stage = L.b_chunk + (L.resident ? 0 : L.a_chunk);
+  L.stage = L.resident ? L.b_chunk : L.a_chunk + HALVES * L.b_chunk;
   L.meta = colmeta_bytes(nr);
   L.table = table ? ETAB * sizeof(uint64_t) : 0;
   return L;
 }
 inline size_t smem_bytes(const SmemLayout &L)
 {
-  return 1024 + L.a_region + NSTAGE * L.stage + NMETA * L.meta + L.table + sizeof(SlicedSmem) + 64;
+  return 1024 + L.a_region + L.nstage * L.stage + NMETA * L.meta + L.table + sizeof(SlicedSmem) + 64;
 }
-static_assert(1024 + NS * (size_t)BM * KRES * 2 + NSTAGE * NS * (size_t)BN * KRES * 2 +
-                      NMETA * colmeta_bytes(RMAX) + ETAB * 8 + sizeof(SlicedSmem) + 64 <= SMEM_MAX,
+static_assert(1024 + NS * (size_t)BM * KRES * 2 + NSTAGE_RES * NS * (size_t)BN * KRES * 2 + NMETA * colmeta_bytes(RMAX) +
+                      ETAB * 8 + sizeof(SlicedSmem) + 64 <= SMEM_MAX,
               "sliced_tiles shared memory (resident)");
-static_assert(1024 + NSTAGE * NS * (size_t)(BM + BN) * KST * 2 + NMETA * colmeta_bytes(RMAX) +
+static_assert(1024 + NSTAGE_STR * NS * (size_t)(BM + HALVES * BN) * KST * 2 + NMETA * colmeta_bytes(RMAX) +
                       ETAB * 8 + sizeof(SlicedSmem) + 64 <= SMEM_MAX,
               "sliced_tiles shared memory (streaming)");
 
-// a 2^s sign-extended to 64 bits, m = 2^s: one integer multiply (a 64-bit
-// shift of a sign-extended value would be three instructions).
-__device__ __forceinline__ long long mulw_s(int a, int m)
+// The high word that takes the bias of combine's level 0 back out.
+template <int SIGN>
+__device__ __forceinline__ uint32_t combine_bias(int g) { return 0u - 0x4B400000u * (uint32_t)(SIGN * (1 << (4 + g))); }
+// w + SIGN W of one pair, from its six level sums, with g guard bits: four
+// 32 x 32 + 64 bit multiply-adds and one into the high word.  Levels 4 and 5
+// join in FP32 (the sum of level 5 is not exact to begin with, and its last
+// bits lie below W's).  Level 0, at most 2^22 over 64 coordinates, becomes an
+// integer by adding 1.5 2^23 to it (w starts with combine_bias in its high
+// word); the others, up to 2^24, need the conversion instruction.
+template <int SIGN>
+__device__ __forceinline__ long long combine(const uint32_t (&r)[NS], int g, long long w)
 {
-  long long d;
-  asm("mul.wide.s32 %0, %1, %2;" : "=l"(d) : "r"(a), "r"(m));
-  return d;
-}
-
-// W of one pair from its six level sums, with g guard bits (2 or more when
-// k <= 64; possibly negative beyond).
-template <bool STREAM>
-__device__ __forceinline__ long long combine(const uint32_t (&r)[NS], int g)
-{
-  int a[NS];
-#pragma unroll
-  for (int l = 0; l < NS; l++) a[l] = __float2int_rn(__uint_as_float(r[l]));
-  long long w = mulw_s(a[1], 1 << (27 + g)) + mulw_s(a[2], 1 << (18 + g)) + mulw_s(a[3], 1 << (9 + g));
-  if constexpr (!STREAM) {
-    // |a4| 2^g <= 5 2^22 2^2 at k = 64, 5 2^21 2^3 at k = 32: 32 bits hold it
-    w += (long long)((a[4] << g) + ((a[5] + (1 << (8 - g))) >> (9 - g)));
-    return w + ((long long)(a[0] << (4 + g)) << 32);
-  } else {
-    const long long v = mulw_s(a[4], 512) + a[5];
-    w += (v + (1ll << (8 - g))) >> (9 - g);
-    return w + ((long long)a[0] << (36 + g));
-  }
+  const float f4 = SIGN * __int_as_float((127 + g) << 23), f5 = SIGN * __int_as_float((118 + g) << 23);   // 2^g, 2^(g-9)
+  const float v = fmaf(__uint_as_float(r[5]), f5, __uint_as_float(r[4]) * f4);
+  w = madws(__float2int_rn(v), 1, w);
+  w = madws(__float2int_rn(__uint_as_float(r[3])), SIGN * (1 << (9 + g)), w);
+  w = madws(__float2int_rn(__uint_as_float(r[2])), SIGN * (1 << (18 + g)), w);
+  w = madws(__float2int_rn(__uint_as_float(r[1])), SIGN * (1 << (27 + g)), w);
+  const int hi = (int)(w >> 32) + __float_as_int(__uint_as_float(r[0]) + 12582912.0f) * (SIGN * (1 << (4 + g)));
+  return (long long)(((uint64_t)(uint32_t)hi << 32) | (uint32_t)w);
 }
 
 // 4 consecutive 32-bit columns of this thread's TMEM lane.
@@ -487,27 +634,42 @@ __device__ __noinline__ double near_d2(const TileArgs &a, int i, int j, double d
   return s;
 }
 
-// Row side of a pair.
+// Row side of a pair: metadata, and the row's position in the call's maps (-1:
+// a padding row).
 struct RowMeta {
   double aa, hi;
-  int e;
+  int e, i;
 };
+
+// The fixed-point Gaussian's value of a pair outside the common range: nearly
+// coincident points, and exponents of 1021 and more.  j: the column's position
+// (-1: a padding column).
+__device__ __noinline__ double rare_value(const TileArgs &a, const CallParam &cp, uint32_t tab, long long y, long long A,
+                                          int i, int j)
+{
+  if (y <= (A >> 38) && i >= 0 && j >= 0)
+    y = __double2ll_rn(near_d2(a, i, j, 0.0) * cp.ah * ldexp(1.0, cp.F));
+  if (y <= 0) return 1.0;
+  if ((int)(y >> 32) < cp.lim) return exp2_neg((uint64_t)y << cp.pre, exp_frame(max(cp.F, 43), tab));
+  if ((int)(y >> 32) >= cp.end) return 0.0;
+  return exp2_neg_wide((double)y * ldexp(1.0, -cp.F));
+}
 
 // Kernel value from the inner product: the functions of kfun64, with the
 // exponentials through exp2_neg and the comparisons of rare cases on the
 // doubles' high words (an FP64 comparison costs as much as an FP64 add).
+// cfold: y 2^53 per unit of d2 (Gaussian), times h_i (variable bandwidth).
 template <int KT>
-__device__ __forceinline__ double kvalue(const TileArgs &a, int i, int j, double dot, const RowMeta &am, double bb,
-                                         double hj, double cfold, const uint64_t *__restrict__ tab)
+__device__ __forceinline__ double kvalue(const TileArgs &a, const KParams &kp, int j, double dot, const RowMeta &am,
+                                         double bb, double hj, double cfold, uint32_t tab)
 {
-  const KParams &kp = a.kp;
   double d2 = 0.0;
   bool near = false;
   if constexpr (kt_uses_norms(KT)) {
     d2 = fma(-2.0, dot, am.aa) + bb;
     // d2 at most about 2^-39 of the larger norm, by the high words
     near = __double2hiint(d2) <= max(__double2hiint(am.aa), __double2hiint(bb)) - (39 << 20);
-    if (KT != KS_LAPLACE && near && i < a.m) d2 = near_d2(a, i, j, d2);
+    if (KT != KS_LAPLACE && near && am.i >= 0) d2 = near_d2(a, am.i, j, d2);
   }
   if constexpr (KT == KS_GAUSSIAN || KT == KS_GAUSSIAN_VAR_BANDWIDTH) {
     // max(d2, 0), also of NaN (fmax): anything not in (0, inf] becomes 0
@@ -516,9 +678,11 @@ __device__ __forceinline__ double kvalue(const TileArgs &a, int i, int j, double
     else return exp2_neg64((d2 * cfold) * hj, tab);
   } else if constexpr (KT == KS_POLYNOMIAL) {
     const double c = fma(dot, kp.scal, kp.cons);
-    if (kp.powe == 2.0) return c * c;
-    if (kp.powe == 3.0) return (c * c) * c;
-    if (kp.powe == 4.0) { const double q = c * c; return q * q; }
+    if (kp.pmode == POW_INT) {
+      if (kp.pint == 2) return c * c;
+      if (kp.pint == 3) return (c * c) * c;
+      if (kp.pint == 4) { const double q = c * c; return q * q; }
+    }
     return pow_call(c, kp);
   } else if constexpr (KT == KS_LAPLACE) {
     // coincidence only where the high words allow it (coinc < 2^-40)
@@ -538,27 +702,166 @@ __device__ __forceinline__ double kvalue(const TileArgs &a, int i, int j, double
   }
 }
 
-template <int KT, int NR, bool STREAM>
+// Where a thread stands in an item: its row's position in the call's maps (-1: a
+// padding row), and for a tile its first column's position and how many are
+// valid.  Formed anew where it is needed (the common path does not).
+struct Place {
+  int i, j0, nv;
+};
+__device__ __forceinline__ Place place_of(const TileArgs &a, int item, int row, int tj, int c0)
+{
+  const Item g = item_geo(a, item);
+  const int done = (tj - g.b0) * BN + c0;
+  return Place{row < g.rows ? g.ia + row : -1, g.jb + done, min(COLS, g.cols - done)};
+}
+
+// One thread's columns of a tile, fixed-point Gaussian: W holds y; A: the row's
+// norm in the same units.
+template <int NR>
+__device__ __forceinline__ void fixed_cols(const TileArgs &a, const CallParam &cp, const ExpFrame &E, long long (&W)[COLS],
+                                           long long A, uint32_t cmS, int item, int row, int tj, int c0,
+                                           double (&sum)[NR])
+{
+  const uint32_t wS = cmS + (uint32_t)offsetof(ColMeta, w);
+  const int lim = cp.lim;
+  // straight-line code where every y of the thread's columns lies in [2^32,
+  // 1021 2^F): independent chains for the schedulers
+  bool rare = false;
+#pragma unroll
+  for (int c = 0; c < COLS; c++) rare |= (uint32_t)((int)(W[c] >> 32) - 1) >= (uint32_t)(lim - 1);
+  if (cp.pre && !rare) {
+#pragma unroll
+    for (int c = 0; c < COLS; c++) W[c] <<= cp.pre;
+  }
+  if (!rare) {
+#pragma unroll
+    for (int c = 0; c < COLS; c += 2) {
+      const double k0 = exp2_neg((uint64_t)W[c], E), k1 = exp2_neg((uint64_t)W[c + 1], E);
+#pragma unroll
+      for (int r = 0; r < NR; r++) {
+        if (r > 0 && r >= a.nrhs) continue;
+        double w0, w1;
+        lds2(wS + (r * BN + c) * 8, w0, w1);
+        sum[r] = fma(k1, w1, fma(k0, w0, sum[r]));
+      }
+    }
+    return;
+  }
+  // the common columns one by one (values of 1088 and more are 0, times w), the
+  // others after them, each lane at a column of its own: their loads take long
+  const int yend = cp.end;
+  uint32_t mask = 0;
+#pragma unroll
+  for (int c = 0; c < COLS; c++) {
+    const int yh = (int)(W[c] >> 32);
+    if (yh < yend && (uint32_t)(yh - 1) >= (uint32_t)(lim - 1)) {
+      mask |= 1u << c;
+    } else {
+      const double kv = yh < yend ? exp2_neg((uint64_t)W[c] << cp.pre, E) : 0.0;
+#pragma unroll
+      for (int r = 0; r < NR; r++) {
+        if (r > 0 && r >= a.nrhs) continue;
+        double w0;
+        lds1(wS + (r * BN + c) * 8, w0);
+        sum[r] = fma(kv, w0, sum[r]);
+      }
+    }
+  }
+  if (!mask) return;
+  const Place P = place_of(a, item, row, tj, c0);
+  for (; mask; mask &= mask - 1) {
+    const int c = __ffs(mask) - 1;
+    long long y = W[0];
+#pragma unroll
+    for (int q = 1; q < COLS; q++) y = c == q ? W[q] : y;
+    const double kv = rare_value(a, cp, E.tab, y, A, P.i, c < P.nv ? P.j0 + c : -1);
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+      if (r > 0 && r >= a.nrhs) continue;
+      double w0;
+      lds1(wS + (r * BN + c) * 8, w0);
+      sum[r] = fma(kv, w0, sum[r]);
+    }
+  }
+}
+
+// One thread's columns of a tile through x.y in FP64; W holds SIGN W.  slow: a
+// point of the row or of the tile has no digits (EFLAG).
+template <int KT, int NR, int SIGN>
+__device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, const long long (&W)[COLS],
+                                         const RowMeta &am, const ColMeta *cm, int c0, const Place &P, int gb, bool slow,
+                                         uint32_t tab, double (&sum)[NR])
+{
+  double cfold = 0.0;
+  if (KT == KS_GAUSSIAN) cfold = -kp.scal * (1.4426950408889634 * 0x1p53);
+  if (KT == KS_GAUSSIAN_VAR_BANDWIDTH) cfold = am.hi * (0.5 * 1.4426950408889634 * 0x1p53);
+#pragma unroll
+  for (int c = 0; c < COLS; c++) {
+    if (c < P.nv) {
+      const int ej = cm->e[c0 + c], j = P.j0 + c;
+      double dot = (double)(SIGN * W[c]);
+      dot = __hiloint2double(__double2hiint(dot) + (W[c] != 0 ? (am.e + ej - 52 - gb) << 20 : 0), __double2loint(dot));
+      if (slow && (am.e == EFLAG || ej == EFLAG) && am.i >= 0) {
+        int pa = a.amap ? a.amap[am.i] : am.i, pb = a.bmap ? a.bmap[j] : j;
+        if (a.nxa >= 0 && (pa < 0 || pa >= a.nxa)) pa = 0;   // flagged by slice_kernel
+        if (a.nxb >= 0 && (pb < 0 || pb >= a.nxb)) pb = 0;
+        dot = dot_direct(a.XA + (size_t)pa * a.k, a.XB + (size_t)pb * a.k, a.k);
+      }
+      const double kv = kvalue<KT>(a, kp, j, dot, am, cm->bb[c0 + c], cm->hj[c0 + c], cfold, tab);
+#pragma unroll
+      for (int r = 0; r < NR; r++)
+        if (r == 0 || r < a.nrhs) sum[r] = fma(kv, cm->w[r][c0 + c], sum[r]);
+    }
+  }
+}
+
+constexpr bool uses_table(int kt) { return kt == KS_GAUSSIAN || kt == KS_GAUSSIAN_VAR_BANDWIDTH || kt == KS_LIST; }
+
+// G: guard bits of the resident layouts (k <= 32: 3, k <= 64: 2), -1: streaming.
+// A thread's partial sums of row i are stored; the last of the row's parts
+// (count in all) adds them in order into u.  (A reduction kernel of its own cost
+// a launch: 3 us of a 40 us call.)
+template <int NR>
+__device__ __forceinline__ void row_done(const TileArgs &a, int i, int parts)
+{
+  __threadfence();
+  if (atomicAdd(&a.row_n[i], 1) != parts - 1) return;
+  __threadfence();
+  const size_t q = (size_t)(a.umap ? a.umap[i] : i) * (NR > 1 ? a.nrhs : 1);
+#pragma unroll
+  for (int r = 0; r < NR; r++) {
+    if (r > 0 && r >= a.nrhs) continue;
+    double s = 0.0;
+    for (int c = 0; c < parts; c++) s += __ldcg(&a.partial[((size_t)r * parts + c) * a.ldp + i]);
+    a.u[q + r] += s;
+  }
+}
+
+template <int KT, int NR, int G>
 __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
 {
-  constexpr bool TABLE = KT == KS_GAUSSIAN || KT == KS_GAUSSIAN_VAR_BANDWIDTH;
+  constexpr bool STREAM = G < 0;
+  constexpr bool TABLE = uses_table(KT);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *sm = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const SmemLayout L = smem_layout(a.kpad, NR, TABLE);
-  uint8_t *sA = sm, *sStage = sm + L.a_region, *sMeta = sStage + NSTAGE * L.stage;
+  uint8_t *sA = sm, *sStage = sm + L.a_region, *sMeta = sStage + L.nstage * L.stage;
   uint64_t *sTab = (uint64_t *)(sMeta + NMETA * L.meta);
   SlicedSmem *S = (SlicedSmem *)((uint8_t *)sTab + L.table);
   volatile int *abort = &S->abort;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int items = a.ntm * a.nsc;
+  const int items = KT == KS_LIST ? a.ntab : a.ntm * a.nsc;
 
   if (threadIdx.x == 0) {
     mbar_init(&S->a_full, 1);
     mbar_init(&S->a_empty, 1 + EPI_WARPS);
-    for (int s = 0; s < NSTAGE; s++) { mbar_init(&S->b_full[s], 1); mbar_init(&S->b_empty[s], 1); }
-    for (int s = 0; s < NMETA; s++) { mbar_init(&S->m_full[s], 1); mbar_init(&S->m_empty[s], EPI_WARPS); }
-    mbar_init(&S->t_full, 1);
-    mbar_init(&S->t_empty, EPI_WARPS);
+    for (int s = 0; s < NSTAGE_RES; s++) { mbar_init(&S->b_full[s], 1); mbar_init(&S->b_empty[s], 1); }
+    for (int s = 0; s < NMETA; s++) { mbar_init(&S->m_full[s], 1); mbar_init(&S->m_empty[s], HALF_WARPS); }
+    for (int h = 0; h < HALVES; h++) { mbar_init(&S->t_full[h], 1); mbar_init(&S->t_empty[h], HALF_WARPS); }
+    for (int b = 0; b < 2; b++) {   // one arrive per thread: groups 1 .. fill, group 0 empties
+      mbar_init(&S->r_full[b], 32 * 4 * (GROUPS - 1));
+      mbar_init(&S->r_empty[b], 32 * 4);
+    }
     mbar_init(&S->drain, 1);
     S->abort = 0;
     S->never = 0;
@@ -567,6 +870,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
   if (warp == 0) { tmem_alloc(&S->tmem_base, TMEM_COLS); tmem_relinquish(); }
   if constexpr (TABLE)
     for (int i = threadIdx.x; i < ETAB; i += NTHREADS) sTab[i] = g_exp_table.v[i];
+  wait_primary();        // slice_kernel's results from here on
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -576,8 +880,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     // ---------------- producer ----------------
     if (lane == 0) {
       int g = 0, tt = 0, a_issued = -1;
-      int b_last[NSTAGE], m_last[NMETA];
-      for (int s = 0; s < NSTAGE; s++) b_last[s] = -1;
+      int b_last[NSTAGE_RES], m_last[NMETA];
+      for (int s = 0; s < NSTAGE_RES; s++) b_last[s] = -1;
       for (int s = 0; s < NMETA; s++) m_last[s] = -1;
       bool stop = false;
       int item = blockIdx.x;
@@ -591,34 +895,46 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
         }
         S->islot[it & 1] = item;
         const int next = atomicAdd(a.next_item, 1) + (int)gridDim.x;
-        const int ti = item % a.ntm, sc = item / a.ntm;
-        const int t0 = sc * a.chunk_tiles, t1 = min(a.ntn, t0 + a.chunk_tiles);
-        const uint8_t *imgA = a.imgA + (size_t)ti * op_bytes(BM, a.kpad);
-        if (L.resident) {
-          mbar_arrive_expect_tx(&S->a_full, (uint32_t)L.a_chunk);
-          bulk_g2s(sA, imgA, (uint32_t)L.a_chunk, &S->a_full);
-        } else {
-          mbar_arrive(&S->a_full);
-        }
+        const Item G_ = item_geo(a, item);
+        const int t0 = G_.b0, t1 = G_.b1;
+        const uint8_t *imgA = a.imgA + (size_t)G_.a_tile * op_bytes(BM, a.kpad);
+        // (a task slot was last read for item it - 2, which every epilogue warp
+        // has finished once it arrived on a_empty for item it - 1)
+        const uint32_t tp_bytes = KT == KS_LIST ? (uint32_t)sizeof(TaskParam) : 0u;
+        const uint32_t a_bytes = STREAM ? 0u : (uint32_t)L.a_chunk;
+        if (a_bytes + tp_bytes) mbar_arrive_expect_tx(&S->a_full, a_bytes + tp_bytes);
+        else mbar_arrive(&S->a_full);
+        if (a_bytes) bulk_g2s(sA, imgA, a_bytes, &S->a_full);
+        if (tp_bytes) bulk_g2s(&S->tslot[it & 1], a.tp + G_.task, tp_bytes, &S->a_full);
         a_issued = it;
-        for (int tj = t0; tj < t1 && !stop; tj++, tt++) {
+        // resident: a stage per source tile; streaming: a stage per k-chunk of
+        // the targets and of two source tiles
+        const int step = STREAM ? HALVES : 1;
+        for (int tj = t0; tj < t1 && !stop; tj += step) {
           const uint8_t *imgB = a.imgB + (size_t)tj * bt;
-          for (int c = 0; c < L.nch; c++, g++) {
-            const int st = g % NSTAGE, u = g / NSTAGE;
+          const int nt = min(step, t1 - tj);
+          // the metadata first: the epilogue waits for it before it takes the
+          // first accumulators, which the copies below wait for in turn
+          for (int q = 0; q < nt && !stop; q++, tt++) {
+            const int ms = tt % NMETA, mu = tt / NMETA;
+            if (mu > 0 && !mbar_wait(&S->m_empty[ms], (mu - 1) & 1, abort, a.wait_limit)) { stop = true; break; }
+            mbar_arrive_expect_tx(&S->m_full[ms], (uint32_t)L.meta);
+            bulk_g2s(sMeta + ms * L.meta, imgB + q * bt + op_bytes(BN, a.kpad), (uint32_t)L.meta, &S->m_full[ms]);
+            m_last[ms] = mu;
+          }
+          for (int c = 0; c < L.nch && !stop; c++, g++) {
+            const int st = g % L.nstage, u = g / L.nstage;
             if (u > 0 && !mbar_wait(&S->b_empty[st], (u - 1) & 1, abort, a.wait_limit)) { stop = true; break; }
             uint8_t *dst = sStage + st * L.stage;
-            mbar_arrive_expect_tx(&S->b_full[st], (uint32_t)L.stage);
-            bulk_g2s(dst, imgB + (size_t)c * L.b_chunk, (uint32_t)L.b_chunk, &S->b_full[st]);
-            if (!L.resident)
-              bulk_g2s(dst + L.b_chunk, imgA + (size_t)c * L.a_chunk, (uint32_t)L.a_chunk, &S->b_full[st]);
+            mbar_arrive_expect_tx(&S->b_full[st], (uint32_t)((STREAM ? L.a_chunk : 0) + nt * L.b_chunk));
+            if (STREAM) {
+              bulk_g2s(dst, imgA + (size_t)c * L.a_chunk, (uint32_t)L.a_chunk, &S->b_full[st]);
+              dst += L.a_chunk;
+            }
+            for (int q = 0; q < nt; q++)
+              bulk_g2s(dst + q * L.b_chunk, imgB + q * bt + (size_t)c * L.b_chunk, (uint32_t)L.b_chunk, &S->b_full[st]);
             b_last[st] = u;
           }
-          if (stop) break;
-          const int ms = tt % NMETA, mu = tt / NMETA;
-          if (mu > 0 && !mbar_wait(&S->m_empty[ms], (mu - 1) & 1, abort, a.wait_limit)) break;
-          mbar_arrive_expect_tx(&S->m_full[ms], (uint32_t)L.meta);
-          bulk_g2s(sMeta + ms * L.meta, imgB + op_bytes(BN, a.kpad), (uint32_t)L.meta, &S->m_full[ms]);
-          m_last[ms] = mu;
         }
         item = next;
       }
@@ -626,7 +942,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
       if (*abort) {
         volatile int *nev = &S->never;
         if (a_issued >= 0) mbar_wait(&S->a_full, a_issued & 1, nev, 1LL << 28);
-        for (int s = 0; s < NSTAGE; s++)
+        for (int s = 0; s < NSTAGE_RES; s++)
           if (b_last[s] >= 0) mbar_wait(&S->b_full[s], b_last[s] & 1, nev, 1LL << 28);
         for (int s = 0; s < NMETA; s++)
           if (m_last[s] >= 0) mbar_wait(&S->m_full[s], m_last[s] & 1, nev, 1LL << 28);
@@ -635,46 +951,51 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
   } else if (warp == 1) {
     // ---------------- MMA issuer (whole warp, one elected lane issues) ----------------
     const unsigned full = 0xffffffffu;
-    const uint32_t idesc = idesc_f16_f32(BM, BN);
-    const uint64_t ablk = (uint64_t)(BM * L.kc * 2) >> 4, bblk = (uint64_t)(BN * L.kc * 2) >> 4;   // one slice
-    const uint64_t astep = (2 * BM * 16) >> 4, bstep = (2 * BN * 16) >> 4;                         // 16 coordinates
-    const int nks = L.kc / 16, gch = STREAM ? KRES / KST : 1;   // chunks per accumulation
-    int g = 0, tg = 0;
+    const uint64_t ablk = (uint64_t)(BM * L.kc * 2) >> 4;                           // one target slice
+    const uint64_t astep = (2 * BM * 16) >> 4, bstep = (2 * NS * BN * 16) >> 4;     // 16 coordinates
+    const int nks = L.kc / 16, gch = STREAM ? KRES / KST : 1;                       // chunks per accumulation
+    int g = 0, use[HALVES] = {0, 0};
     bool stop = false;
     for (int it = 0; !stop; it++) {
       if (!__all_sync(full, *abort == 0 && mbar_wait(&S->a_full, it & 1, abort, a.wait_limit))) break;
       const int item = __shfl_sync(full, ((volatile int *)S->islot)[it & 1], 0);
       if (item < 0) break;
-      const int sc = item / a.ntm, t0 = sc * a.chunk_tiles, t1 = min(a.ntn, t0 + a.chunk_tiles);
-      for (int tj = t0; tj < t1 && !stop; tj++) {
-        for (int c = 0; c < L.nch; c++, g++) {
+      const Item G_ = item_geo(a, item);
+      const int t0 = G_.b0, t1 = G_.b1;
+      const int step = STREAM ? HALVES : 1;
+      for (int tj = t0; tj < t1 && !stop; tj += step) {
+        for (int c = 0; c < L.nch && !stop; c++, g++) {
           const bool first = c % gch == 0, last = c % gch == gch - 1;
-          if (first) {
-            if (tg > 0 && !__all_sync(full, mbar_wait(&S->t_empty, (tg - 1) & 1, abort, a.wait_limit))) { stop = true; break; }
-            tg++;
-          }
-          const int st = g % NSTAGE;
-          if (!__all_sync(full, mbar_wait(&S->b_full[st], (g / NSTAGE) & 1, abort, a.wait_limit))) { stop = true; break; }
-          tc_fence_after();
+          const int st = g % L.nstage;
+          if (!__all_sync(full, mbar_wait(&S->b_full[st], (g / L.nstage) & 1, abort, a.wait_limit))) { stop = true; break; }
           const uint32_t sb = smem_addr(sStage + st * L.stage);
-          const uint32_t sa = L.resident ? smem_addr(sA) : sb + (uint32_t)L.b_chunk;
-          const uint64_t dA = desc_noswizzle(sa, BM * 16, 128), dB = desc_noswizzle(sb, BN * 16, 128);
-          if (elect_one()) {
+          const uint64_t dA = desc_noswizzle(STREAM ? sb : smem_addr(sA), BM * 16, 128);
 #pragma unroll
-            for (int s = 0; s < KRES / 16; s++) {
-              if (s < nks) {
-                const uint64_t As = dA + (uint64_t)s * astep, Bs = dB + (uint64_t)s * bstep;
-#pragma unroll
-                for (int l = 0; l < NS; l++)
-#pragma unroll
-                  for (int i = 0; i <= l; i++)
-                    umma_f16(tmem + l * BN, As + i * ablk, Bs + (l - i) * bblk, idesc,
-                             (i > 0 || s > 0 || !first) ? 1u : 0u);
-              }
+          for (int q = 0; q < (STREAM ? HALVES : 1); q++) {
+            if (tj + q >= t1) continue;
+            const int h = STREAM ? q : (tj - t0) & 1;      // the accumulator buffer
+            if (first) {
+              const int u = h ? use[1]++ : use[0]++;
+              if (u > 0 && !__all_sync(full, mbar_wait(&S->t_empty[h], (u - 1) & 1, abort, a.wait_limit))) { stop = true; break; }
             }
-            umma_commit(&S->b_empty[st]);
-            if (last) umma_commit(&S->t_full);
+            tc_fence_after();
+            const uint64_t dB = desc_noswizzle(sb + (STREAM ? (uint32_t)(L.a_chunk + q * L.b_chunk) : 0u), NS * BN * 16, 128);
+            if (elect_one()) {
+#pragma unroll
+              for (int s = 0; s < KRES / 16; s++) {
+                if (s < nks) {
+#pragma unroll
+                  for (int i = 0; i < NS; i++)
+                    umma_f16(tmem + h * TBUF + i * BN, dA + (uint64_t)s * astep + i * ablk, dB + (uint64_t)s * bstep,
+                             idesc_f16_f32(BM, BN * (NS - i)), (i > 0 || s > 0 || !first) ? 1u : 0u);
+                }
+              }
+              if (last) umma_commit(&S->t_full[h]);
+            }
+            __syncwarp();
           }
+          if (stop) break;
+          if (elect_one()) umma_commit(&S->b_empty[st]);
           __syncwarp();
         }
       }
@@ -686,110 +1007,138 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     mbar_wait(&S->drain, 0, &S->never, 1LL << 30);
   } else {
     // ---------------- epilogue ----------------
-    const int grp = (warp - 2) >> 2, qd = warp & 3;
-    const int row = qd * 32 + lane, c0 = grp * COLS;
-    const uint32_t tT = tmem + ((uint32_t)(qd * 32) << 16) + c0;
-    const int gb = guard_bits(a.kpad);
-    const CallParam cp = *a.cp;
-    const bool fixed = KT == KS_GAUSSIAN && cp.fixed != 0;
-    int g = 0, tg = 0;
+    const int grp = (warp - 2) >> 2, qd = warp & 3, half = grp >> 1;
+    const int row = qd * 32 + lane, c0 = (grp & 1) * COLS;
+    const uint32_t tT = tmem + ((uint32_t)(qd * 32) << 16) + half * TBUF + c0;
+    const int gb = G >= 0 ? G : guard_bits(a.kpad);
+    constexpr int SIGN = KT == KS_GAUSSIAN || KT == KS_LIST ? -1 : 1;   // W or -W
+    const uint32_t bias = combine_bias<SIGN>(gb);
+    const uint32_t tabS = smem_addr(sTab);
+    int tbase = 0, tg = 0;                          // tiles before this item, accumulations taken
     for (int it = 0; !*abort; it++) {
       if (!mbar_wait(&S->a_full, it & 1, abort, a.wait_limit)) break;
       const int item = ((volatile int *)S->islot)[it & 1];
       if (item < 0) break;
       __syncwarp();
       if (lane == 0) mbar_arrive(&S->a_empty);
-      const int ti = item % a.ntm, sc = item / a.ntm;
-      const int t0 = sc * a.chunk_tiles, t1 = min(a.ntn, t0 + a.chunk_tiles);
-      const int i = ti * BM + row;
-      RowMeta am;
-      am.aa = a.row_aa[i];
-      am.hi = a.row_hi[i];
-      am.e = a.row_e[i];
-      const bool rflag = am.e == EFLAG;
-      const bool anyrow = __any_sync(0xffffffffu, rflag);
-      // the exponent of 2^-y per unit of d2, in units of 2^-53 (variable bandwidth: times h_i)
-      double cfold = 0.0;
-      if constexpr (KT == KS_GAUSSIAN) cfold = -a.kp.scal * (1.4426950408889634 * 0x1p53);
-      if constexpr (KT == KS_GAUSSIAN_VAR_BANDWIDTH) cfold = am.hi * (0.5 * 1.4426950408889634 * 0x1p53);
+      int t0, t1, i0;
+      {
+        const Item g = item_geo(a, item);
+        t0 = g.b0; t1 = g.b1; i0 = g.a_tile * BM + row;
+      }
+      const KParams &kp = KT == KS_LIST ? S->tslot[it & 1].kp : a.kp;
+      const CallParam &cp = KT == KS_LIST ? S->tslot[it & 1].cp : *a.cp;
+      const int type = KT == KS_LIST ? kp.type : KT;
+      const bool fixed = (KT == KS_GAUSSIAN || (KT == KS_LIST && type == KS_GAUSSIAN)) && cp.fixed != 0;
+      const ExpFrame E = exp_frame(max(fixed ? cp.F : 43, 43), tabS);
+      const long long arow = __double_as_longlong(a.row_aa[i0]);
+      const bool anyrow = __any_sync(0xffffffffu, a.row_e[i0] == EFLAG);
       double racc[NR];
 #pragma unroll
       for (int r = 0; r < NR; r++) racc[r] = 0.0;
       bool ok = true;
-      for (int tj = t0; tj < t1; tj++, g++) {
+      for (int tj = t0 + half; tj < t1; tj += HALVES) {
+        const int tt = tbase + tj - t0, ms = tt % NMETA;
+        if (!mbar_wait(&S->m_full[ms], (tt / NMETA) & 1, abort, a.wait_limit)) { ok = false; break; }
+        const ColMeta *cm = (const ColMeta *)(sMeta + ms * L.meta);
+        const uint32_t cmS = smem_addr(cm) + c0 * 8;   // the group's first column
+        // Accumulators -> W (the fixed form: y = A + B - W), four columns at a
+        // time; the tensor memory is free again after the last load.
         long long W[COLS];
-        // accumulators -> integers; the tensor memory is free again after the last load
         const int ngr = STREAM ? a.kpad / KRES : 1;
         for (int c = 0; c < ngr; c++, tg++) {
-          if (!mbar_wait(&S->t_full, tg & 1, abort, a.wait_limit)) { ok = false; break; }
+          if (!mbar_wait(&S->t_full[half], tg & 1, abort, a.wait_limit)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int q = 0; q < COLS; q += 4) {
             uint32_t r[4][NS];
 #pragma unroll
             for (int l = 0; l < NS; l++) tmem_ld4(tT + l * BN + q, r[0][l], r[1][l], r[2][l], r[3][l]);
+            const long long b0 = (long long)((uint64_t)bias << 32);
+            long long w0[4] = {b0, b0, b0, b0};
+            if (STREAM && c > 0) {
+#pragma unroll
+              for (int s = 0; s < 4; s++) w0[s] += W[q + s];
+            } else if ((KT == KS_GAUSSIAN || KT == KS_LIST) && fixed) {
+              lds2(cmS + q * 8, w0[0], w0[1]);
+              lds2(cmS + q * 8 + 16, w0[2], w0[3]);
+#pragma unroll
+              for (int s = 0; s < 4; s++) w0[s] += arow + b0;
+            }
             tmem_ld_wait();
 #pragma unroll
-            for (int s = 0; s < 4; s++) {
-              const long long w = combine<STREAM>(r[s], gb);
-              W[q + s] = STREAM && c > 0 ? W[q + s] + w : w;
-            }
+            for (int s = 0; s < 4; s++) W[q + s] = combine<SIGN>(r[s], gb, w0[s]);
           }
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&S->t_empty);
+          if (lane == 0) mbar_arrive(&S->t_empty[half]);
         }
         if (!ok) break;
-        const int ms = g % NMETA;
-        if (!mbar_wait(&S->m_full[ms], (g / NMETA) & 1, abort, a.wait_limit)) { ok = false; break; }
-        const ColMeta *cm = (const ColMeta *)(sMeta + ms * L.meta);
-        const int nv = min(COLS, a.n - tj * BN - c0);   // valid columns of this group
-        if (fixed) {
-          const long long A = __double_as_longlong(am.aa);
+        // the tile's sum first: a chain of 16 and one of the tiles, not one of
+        // all the row's columns (its rounding)
+        double tsum[NR];
 #pragma unroll
-          for (int c = 0; c < COLS; c++) {
-            long long y = A + __double_as_longlong(cm->bb[c0 + c]) - W[c];
-            if (y <= (A >> 38) && c < nv && i < a.m)
-              y = __double2ll_rn(near_d2(a, i, tj * BN + c0 + c, 0.0) * cp.ah * ldexp(1.0, cp.F));
-            double kv;
-            if ((int)(y >> 32) < cp.lim) kv = exp2_neg((uint64_t)y << cp.shl, sTab);
-            else if ((int)(y >> 32) >= cp.end) kv = 0.0;
-            else kv = exp2_neg_wide((double)y * ldexp(1.0, -cp.F));
-#pragma unroll
-            for (int r = 0; r < NR; r++)
-              if (r == 0 || r < a.nrhs) racc[r] = fma(kv, cm->w[r][c0 + c], racc[r]);
-          }
+        for (int r = 0; r < NR; r++) tsum[r] = 0.0;
+        if ((KT == KS_GAUSSIAN || KT == KS_LIST) && fixed) {
+          fixed_cols<NR>(a, cp, E, W, arow, cmS, item, row, tj, c0, tsum);
         } else {
-          const bool slow = anyrow || cm->flag[c0 >> 5] != 0;
-#pragma unroll
-          for (int c = 0; c < COLS; c++) {
-            const int ej = cm->e[c0 + c];
-            double dot = (double)W[c];
-            dot = __hiloint2double(__double2hiint(dot) + (W[c] != 0 ? (am.e + ej - 52 - gb) << 20 : 0),
-                                   __double2loint(dot));
-            if (slow && (rflag || ej == EFLAG) && c < nv && i < a.m) {
-              const int j = tj * BN + c0 + c;
-              int pa = a.amap ? a.amap[i] : i, pb = a.bmap ? a.bmap[j] : j;
-              if (a.nxa >= 0 && (pa < 0 || pa >= a.nxa)) pa = 0;   // flagged by slice_kernel
-              if (a.nxb >= 0 && (pb < 0 || pb >= a.nxb)) pb = 0;
-              dot = dot_direct(a.XA + (size_t)pa * a.k, a.XB + (size_t)pb * a.k, a.k);
+          const Place P = place_of(a, item, row, tj, c0);
+          const RowMeta am{__longlong_as_double(arow), a.row_hi[i0], a.row_e[i0], P.i};
+          const bool slow = anyrow || cm->flag != 0;
+#define GSKS_COLS(T) dot_cols<T, NR, SIGN>(a, kp, W, am, cm, c0, P, gb, slow, tabS, tsum)
+          if constexpr (KT == KS_LIST) {
+            switch (type) {
+              case KS_GAUSSIAN: GSKS_COLS(KS_GAUSSIAN); break;
+              case KS_GAUSSIAN_VAR_BANDWIDTH: GSKS_COLS(KS_GAUSSIAN_VAR_BANDWIDTH); break;
+              case KS_POLYNOMIAL: GSKS_COLS(KS_POLYNOMIAL); break;
+              case KS_LAPLACE: GSKS_COLS(KS_LAPLACE); break;
+              case KS_TANH: GSKS_COLS(KS_TANH); break;
+              case KS_QUARTIC: GSKS_COLS(KS_QUARTIC); break;
+              case KS_MULTIQUADRATIC: GSKS_COLS(KS_MULTIQUADRATIC); break;
+              default: GSKS_COLS(KS_EPANECHNIKOV); break;
             }
-            if (c < nv) {
-              const double kv = kvalue<KT>(a, i, tj * BN + c0 + c, dot, am, cm->bb[c0 + c], cm->hj[c0 + c], cfold, sTab);
-#pragma unroll
-              for (int r = 0; r < NR; r++)
-                if (r == 0 || r < a.nrhs) racc[r] = fma(kv, cm->w[r][c0 + c], racc[r]);
-            }
+          } else {
+            GSKS_COLS(KT);
           }
+#undef GSKS_COLS
         }
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+          if (r == 0 || r < a.nrhs) racc[r] += tsum[r];
         __syncwarp();
         if (lane == 0) mbar_arrive(&S->m_empty[ms]);
       }
       if (!ok) break;
-      if (i < a.m) {
+      tbase += t1 - t0;
+      const Item g = item_geo(a, item);
+      if constexpr (NR > 1) {
+        // every group writes its own partials; the reduction adds them in order
+        const int sc = item / a.ntm;
+        if (row < g.rows) {
 #pragma unroll
-        for (int r = 0; r < NR; r++)
-          if (r == 0 || r < a.nrhs) a.partial[(((size_t)r * a.nsc + sc) * GROUPS + grp) * a.ldp + i] = racc[r];
+          for (int r = 0; r < NR; r++)
+            if (r < a.nrhs) a.partial[(((size_t)r * a.nsc + sc) * GROUPS + grp) * a.ldp + g.ia + row] = racc[r];
+          row_done<NR>(a, g.ia + row, a.nsc * GROUPS);
+        }
+      } else {
+        // the groups' row sums in group order, through a slot per item parity:
+        // groups 1 .. write theirs and arrive on r_full, group 0 waits, adds
+        // and arrives on r_empty
+        const int rb = it & 1, ru = it >> 1;   // slot, and its earlier uses
+        if (grp > 0) {
+          if (ru > 0 && !mbar_wait(&S->r_empty[rb], (ru - 1) & 1, abort, a.wait_limit)) break;
+          S->rsum[rb][grp - 1][row] = racc[0];
+          mbar_arrive(&S->r_full[rb]);
+        } else {
+          if (!mbar_wait(&S->r_full[rb], ru & 1, abort, a.wait_limit)) break;
+          double s = racc[0];
+          for (int q = 0; q < GROUPS - 1; q++) s += S->rsum[rb][q][row];
+          mbar_arrive(&S->r_empty[rb]);
+          if (row < g.rows) {
+            a.partial[g.out + row] = s;
+            if (KT != KS_LIST) row_done<1>(a, g.ia + row, a.nsc);
+          }
+        }
       }
     }
   }
@@ -799,34 +1148,38 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
   if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
 }
 
-template <int KT, int NR, bool STREAM>
+template <int KT, int NR, int G>
 cudaError_t launch_t(const TileArgs &a, int grid, cudaStream_t s)
 {
-  const size_t smem = smem_bytes(smem_layout(a.kpad, NR, KT == KS_GAUSSIAN || KT == KS_GAUSSIAN_VAR_BANDWIDTH));
+  const size_t smem = smem_bytes(smem_layout(a.kpad, NR, uses_table(KT)));
   // The attribute is per function and device; raised once to the most any launch takes.
   static bool raised[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !raised[dev]) {
     const cudaError_t e =
-        cudaFuncSetAttribute(sliced_tiles<KT, NR, STREAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
+        cudaFuncSetAttribute(sliced_tiles<KT, NR, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) raised[dev] = true;
   }
-  sliced_tiles<KT, NR, STREAM><<<grid, NTHREADS, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_after(sliced_tiles<KT, NR, G>, grid, NTHREADS, smem, s, a);
 }
 
+template <int KT, int NR>
+cudaError_t launch_g(const TileArgs &a, int grid, cudaStream_t s)
+{
+  if (a.kpad > KRES) return launch_t<KT, NR, -1>(a, grid, s);
+  return a.kpad > 32 ? launch_t<KT, NR, 2>(a, grid, s) : launch_t<KT, NR, 3>(a, grid, s);
+}
 template <int KT>
 cudaError_t launch_k(const TileArgs &a, int grid, int nr, cudaStream_t s)
 {
-  const bool stream = a.kpad > KRES;
-  if (nr > 1) return stream ? launch_t<KT, RMAX, true>(a, grid, s) : launch_t<KT, RMAX, false>(a, grid, s);
-  return stream ? launch_t<KT, 1, true>(a, grid, s) : launch_t<KT, 1, false>(a, grid, s);
+  return nr > 1 ? launch_g<KT, RMAX>(a, grid, s) : launch_g<KT, 1>(a, grid, s);
 }
 
 cudaError_t launch_tiles(const TileArgs &a, int grid, int nr, cudaStream_t s)
 {
+  if (a.tab) return launch_g<KS_LIST, 1>(a, grid, s);
   switch (a.kp.type) {
     case KS_GAUSSIAN: return launch_k<KS_GAUSSIAN>(a, grid, nr, s);
     case KS_GAUSSIAN_VAR_BANDWIDTH: return launch_k<KS_GAUSSIAN_VAR_BANDWIDTH>(a, grid, nr, s);
@@ -859,21 +1212,22 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   const int nr = nrhs > 1 ? RMAX : 1;
   const int kpad = sliced_kpad(k);
   const int ntm = (m + BM - 1) / BM, ntn = (n + BN - 1) / BN, sms = std::max(1, c->num_sms);
-  // Runs of source tiles: the slowest CTA's work, waves x (run + one tile of
-  // per-item overhead), over up to 16 items per SM (as enqueue_split).
-  int nsc = 1, chunk = ntn;
+  const int ntp = (ntn + 1) / 2;   // pairs of source tiles (one for each half of the epilogue)
+  // Runs of source tiles, in pairs: the slowest CTA's work, waves x (run + one
+  // pair of per-item overhead), over up to 16 items per SM (as enqueue_split).
+  int nsc = 1, chunk = ntp;
   {
-    const int cmax = (int)std::min<long long>(ntn, std::max<long long>(1, (16LL * sms + ntm - 1) / ntm));
+    const int cmax = (int)std::min<long long>(ntp, std::max<long long>(1, (16LL * sms + ntm - 1) / ntm));
     long long best = -1;
     for (int q = 1; q <= cmax; q++) {
-      const int ch = (ntn + q - 1) / q;
-      if ((ntn + ch - 1) / ch != q) continue;
+      const int ch = (ntp + q - 1) / q;
+      if ((ntp + ch - 1) / ch != q) continue;
       const long long cost = (((long long)ntm * q + sms - 1) / sms) * (ch + 1);
       if (best < 0 || cost < best) { best = cost; nsc = q; chunk = ch; }
     }
   }
   const int ldp = ntm * BM;
-  const bool scan = ker->type == KS_GAUSSIAN;
+  const bool gauss = ker->type == KS_GAUSSIAN, scan = gauss && ((long long)m + n) * k > SCAN_SELF;
   const int nscan = scan ? (int)std::min<long long>(SCAN_MAX, ((long long)m + n + 7) / 8) : 0;
 
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -885,8 +1239,10 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   const size_t o_aa = o_b + al((size_t)ntn * btile_bytes(kpad, nr));
   const size_t o_hi = o_aa + al((size_t)ldp * 8);
   const size_t o_e = o_hi + al((size_t)ldp * 8);
-  const size_t o_p = o_e + al((size_t)ldp * 4);
-  const size_t total = o_p + al((size_t)nrhs * nsc * GROUPS * ldp * 8);
+  const size_t o_n = o_e + al((size_t)ldp * 4);
+  const size_t o_p = o_n + al((size_t)ldp * 4);
+  const int nparts = nr > 1 ? nsc * GROUPS : nsc;          // partials per row and column
+  const size_t total = o_p + al((size_t)nrhs * nparts * ldp * 8);
   uint8_t *ws = nullptr;
   if (stream_ordered_alloc) {
     const cudaError_t e = cudaMallocAsync((void **)&ws, total, s);
@@ -900,19 +1256,28 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   p.m = m; p.n = n; p.k = k; p.kpad = kpad; p.kt = ker->type; p.nrhs = nrhs; p.nr = nr;
   p.XA = XA; p.XA2 = XA2; p.hi = hi; p.amap = amap; p.nxa = nxa;
   p.XB = XB; p.XB2 = XB2; p.hj = hj; p.bmap = bmap; p.nxb = nxb;
-  p.w = w; p.wmap = wmap; p.scal = ker->scal;
+  p.w = w; p.wmap = wmap;
+  p.frame = gauss_frame(ker->scal);
+  p.nta = ntm;
   p.imgA = ws + o_a; p.imgB = ws + o_b;
   p.row_aa = (double *)(ws + o_aa); p.row_hi = (double *)(ws + o_hi); p.row_e = (int *)(ws + o_e);
-  p.scan = (const ScanPart *)(ws + o_scan); p.nscan = nscan;
+  p.row_n = (int *)(ws + o_n);
+  p.scan = (const ScanPart *)(ws + o_scan); p.nscan = gauss ? nscan : -1;
   p.cp = (CallParam *)(ws + o_cp);
   p.next_item = (int *)(ws + o_next);
   p.err = err_word(c);
-  if (scan) scan_kernel<<<nscan, 256, 0, s>>>(p, (ScanPart *)(ws + o_scan));
-  slice_kernel<<<ntm * (BM / 32) + ntn * (BN / 32), 256, 0, s>>>(p);
+  const int blocks = ntm * (BM / 32) + ntn * (BN / 32);
+  cudaError_t e = cudaSuccess;
+  if (scan) {
+    scan_kernel<<<nscan, 256, 0, s>>>(p, (ScanPart *)(ws + o_scan));
+    e = launch_after(slice_kernel, blocks, 256, 0, s, p);
+  } else {
+    slice_kernel<<<blocks, 256, 0, s>>>(p);
+  }
 
   TileArgs a{};
   a.m = m; a.n = n; a.k = k; a.kpad = kpad; a.nrhs = nrhs;
-  a.ntm = ntm; a.ntn = ntn; a.nsc = nsc; a.chunk_tiles = chunk;
+  a.ntm = ntm; a.ntn = ntn; a.nsc = nsc; a.chunk_tiles = 2 * chunk;
   a.imgA = p.imgA; a.imgB = p.imgB;
   a.row_aa = p.row_aa; a.row_hi = p.row_hi; a.row_e = p.row_e;
   a.XA = XA; a.XB = XB; a.amap = amap; a.bmap = bmap; a.nxa = nxa; a.nxb = nxb;
@@ -920,19 +1285,171 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   a.kp.coinc = coincidence_eps(k);
   a.cp = p.cp;
   a.partial = (double *)(ws + o_p);
+  a.row_n = p.row_n;
+  a.u = u; a.umap = umap;
   a.ldp = ldp;
   a.err = p.err;
   a.next_item = p.next_item;
   a.wait_limit = WAIT_LIMIT;
-  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_tiles(a, std::min(ntm * nsc, sms), nr, s);
-  if (e == cudaSuccess) {
-    fp64_reduce_launch(m, nsc * GROUPS, ldp, nrhs, (long long)nsc * GROUPS * ldp, a.partial, u, umap, s);
-    e = cudaGetLastError();
-  }
   if (stream_ordered_alloc) cudaFreeAsync(ws, s);
   if (e != cudaSuccess) return cuda_status(e, "sliced launch");
-  note_launches(scan ? 4 : 3);
+  note_launches(scan ? 3 : 2);
+  return GSKS_OK;
+}
+
+// ---------------------------------------------------------------------------
+// Batched form: every task's targets and sources in tiles of their own; an item
+// is (task, target tile, chunk of source tiles), its row sums go to
+// partial[pbase[t] + sc m_t + r], the layout the list merge reads.
+// sliced_list_plan builds the tile and item tables of a fixed set of lists on
+// the device, sliced_list_run evaluates them (launches only).
+int sliced_list_plan(SlicedListPlan &Pl, const KParams *kps, int ntask, int k, const int *hoff_a, const int *hoff_b,
+                     const long long *pbase, int chunk, cudaStream_t s)
+{
+  using namespace sliced;
+  if (chunk % BN) return GSKS_ERR_ARG;
+  const int kpad = sliced_kpad(k), chunk_tiles = chunk / BN;
+  std::vector<int> ota(ntask + 1, 0), otb(ntask + 1, 0);
+  std::vector<long long> oit(ntask + 1, 0);
+  for (int t = 0; t < ntask; t++) {
+    const int m = hoff_a[t + 1] - hoff_a[t], n = hoff_b[t + 1] - hoff_b[t];
+    const bool live = m > 0 && n > 0;
+    const int ca = live ? (m + BM - 1) / BM : 0, cb = live ? (n + BN - 1) / BN : 0;
+    ota[t + 1] = ota[t] + ca;
+    otb[t + 1] = otb[t] + cb;
+    oit[t + 1] = oit[t] + (long long)ca * ((cb + chunk_tiles - 1) / chunk_tiles);
+  }
+  if (oit[ntask] > INT32_MAX) return GSKS_ERR_TOO_LARGE;
+  std::vector<int2> ta(ota[ntask]), tb(otb[ntask]);
+  std::vector<int> ta_task(ota[ntask]), tb_task(otb[ntask]), cost(oit[ntask]);
+  std::vector<Item> items(oit[ntask]);
+  std::vector<TaskGeo> tg(ntask);
+  std::vector<TaskParam> tp(ntask);
+#pragma omp parallel for schedule(dynamic, 64) if (ntask > 512)
+  for (int t = 0; t < ntask; t++) {
+    const int m = hoff_a[t + 1] - hoff_a[t], n = hoff_b[t + 1] - hoff_b[t];
+    tg[t] = TaskGeo{hoff_a[t], m, hoff_b[t], n};
+    memset(&tp[t], 0, sizeof(TaskParam));
+    tp[t].kp = kps[t];
+    if (kps[t].type == KS_GAUSSIAN) tp[t].cp = gauss_frame(kps[t].scal);
+    if (m <= 0 || n <= 0) continue;
+    for (int q = ota[t]; q < ota[t + 1]; q++) {
+      const int i0 = (q - ota[t]) * BM;
+      ta[q] = make_int2(hoff_a[t] + i0, std::min(BM, m - i0));
+      ta_task[q] = t;
+    }
+    for (int q = otb[t]; q < otb[t + 1]; q++) {
+      const int j0 = (q - otb[t]) * BN;
+      tb[q] = make_int2(hoff_b[t] + j0, std::min(BN, n - j0));
+      tb_task[q] = t;
+    }
+    // relative epilogue cost of a tile: FP64 instructions of a value
+    const int wkt = kps[t].type == KS_LAPLACE ? 10 : kps[t].type == KS_GAUSSIAN ? 2 : kps[t].type == KS_TANH ? 12 : 4;
+    long long q = oit[t];
+    for (int b0 = otb[t]; b0 < otb[t + 1]; b0 += chunk_tiles)
+      for (int i0 = 0; i0 < m; i0 += BM, q++) {
+        Item it{};
+        it.a_tile = ota[t] + i0 / BM;
+        it.rows = std::min(BM, m - i0);
+        it.ia = hoff_a[t] + i0;
+        it.b0 = b0;
+        it.b1 = std::min(otb[t + 1], b0 + chunk_tiles);
+        it.jb = hoff_b[t] + (b0 - otb[t]) * BN;
+        it.cols = std::min(hoff_b[t + 1] - it.jb, chunk);
+        it.task = t;
+        it.out = pbase[t] + (long long)((b0 - otb[t]) / chunk_tiles) * m + i0;
+        items[q] = it;
+        cost[q] = wkt * (it.b1 - it.b0);
+      }
+  }
+  {
+    // largest cost first, ties in build order: a counting sort
+    int cmax = 0;
+    for (const int c : cost) cmax = std::max(cmax, c);
+    std::vector<size_t> start((size_t)cmax + 2, 0);
+    for (const int c : cost) start[(size_t)(cmax - c) + 1]++;
+    for (int b = 0; b <= cmax; b++) start[b + 1] += start[b];
+    std::vector<Item> sorted(items.size());
+    for (size_t i = 0; i < items.size(); i++) sorted[start[cmax - cost[i]]++] = items[i];
+    items.swap(sorted);
+  }
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  Pl.ntask = ntask; Pl.k = k; Pl.kpad = kpad;
+  Pl.n_ta = (int)ta.size(); Pl.n_tb = (int)tb.size(); Pl.n_items = (int)items.size();
+  Pl.any_gauss = false;
+  for (int t = 0; t < ntask && !Pl.any_gauss; t++) Pl.any_gauss = kps[t].type == KS_GAUSSIAN;
+  const size_t rows = (size_t)Pl.n_ta * BM;
+  Pl.o_next = 0;
+  Pl.o_ta = al(4);
+  Pl.o_tat = Pl.o_ta + al(ta.size() * sizeof(int2));
+  Pl.o_tb = Pl.o_tat + al(ta.size() * 4);
+  Pl.o_tbt = Pl.o_tb + al(tb.size() * sizeof(int2));
+  Pl.o_items = Pl.o_tbt + al(tb.size() * 4);
+  Pl.o_tg = Pl.o_items + al(items.size() * sizeof(Item));
+  Pl.o_tp = Pl.o_tg + al(tg.size() * sizeof(TaskGeo));
+  Pl.o_aa = Pl.o_tp + al(tp.size() * sizeof(TaskParam));
+  Pl.o_hi = Pl.o_aa + al(rows * 8);
+  Pl.o_e = Pl.o_hi + al(rows * 8);
+  Pl.o_a = Pl.o_e + al(rows * 4);
+  Pl.o_b = Pl.o_a + al((size_t)Pl.n_ta * op_bytes(BM, kpad));
+  const size_t total = Pl.o_b + al((size_t)Pl.n_tb * btile_bytes(kpad, 1));
+  if (!Pl.ws.ensure(total)) return GSKS_ERR_ALLOC;
+  uint8_t *ws = (uint8_t *)Pl.ws.p;
+  auto up = [&](size_t off, const void *src, size_t bytes) {
+    return bytes == 0 || cudaMemcpyAsync(ws + off, src, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
+  };
+  if (!(up(Pl.o_ta, ta.data(), ta.size() * sizeof(int2)) && up(Pl.o_tat, ta_task.data(), ta_task.size() * 4) &&
+        up(Pl.o_tb, tb.data(), tb.size() * sizeof(int2)) && up(Pl.o_tbt, tb_task.data(), tb_task.size() * 4) &&
+        up(Pl.o_items, items.data(), items.size() * sizeof(Item)) && up(Pl.o_tg, tg.data(), tg.size() * sizeof(TaskGeo)) &&
+        up(Pl.o_tp, tp.data(), tp.size() * sizeof(TaskParam))))
+    return cuda_status(cudaGetLastError(), "sliced list tables");
+  // the host vectors above die here: the copies must have left them
+  const cudaError_t e = cudaStreamSynchronize(s);
+  return e == cudaSuccess ? GSKS_OK : cuda_status(e, "sliced list tables");
+}
+
+int sliced_list_run(const SlicedListPlan &Pl, Ctx *c, const double *XA, const double *XA2, const int *a_idx, int nxa,
+                    const double *XB, const double *XB2, const int *b_idx, int nxb, const double *w, const int *w_idx,
+                    double *partial, int *err, cudaStream_t s, int *launches)
+{
+  using namespace sliced;
+  if (Pl.n_items == 0) return GSKS_OK;
+  uint8_t *ws = (uint8_t *)Pl.ws.p;
+  TaskParam *tp = (TaskParam *)(ws + Pl.o_tp);
+  SliceArgs p{};
+  p.k = Pl.k; p.kpad = Pl.kpad; p.kt = KS_LIST; p.nrhs = 1; p.nr = 1;
+  p.XA = XA; p.XA2 = XA2; p.amap = a_idx; p.nxa = nxa;
+  p.XB = XB; p.XB2 = XB2; p.bmap = b_idx; p.nxb = nxb;
+  p.w = w; p.wmap = w_idx;
+  p.imgA = ws + Pl.o_a; p.imgB = ws + Pl.o_b;
+  p.row_aa = (double *)(ws + Pl.o_aa); p.row_hi = (double *)(ws + Pl.o_hi); p.row_e = (int *)(ws + Pl.o_e);
+  p.next_item = (int *)(ws + Pl.o_next);
+  p.err = err;
+  p.tilesA = (const int2 *)(ws + Pl.o_ta); p.taskA = (const int *)(ws + Pl.o_tat);
+  p.tilesB = (const int2 *)(ws + Pl.o_tb); p.taskB = (const int *)(ws + Pl.o_tbt);
+  p.tp = tp;
+  p.nta = Pl.n_ta;
+  // (also clears the work counter)
+  list_scan_kernel<<<Pl.any_gauss ? Pl.ntask : 1, 256, 0, s>>>(p, Pl.ntask, (const TaskGeo *)(ws + Pl.o_tg), tp);
+  cudaError_t e = launch_after(slice_kernel, Pl.n_ta * (BM / 32) + Pl.n_tb * (BN / 32), 256, 0, s, p);
+  TileArgs a{};
+  a.k = Pl.k; a.kpad = Pl.kpad; a.nrhs = 1; a.ntm = 1;
+  a.imgA = p.imgA; a.imgB = p.imgB;
+  a.row_aa = p.row_aa; a.row_hi = p.row_hi; a.row_e = p.row_e;
+  a.XA = XA; a.XB = XB; a.amap = a_idx; a.bmap = b_idx; a.nxa = nxa; a.nxb = nxb;
+  a.partial = partial;
+  a.err = err;
+  a.next_item = p.next_item;
+  a.wait_limit = WAIT_LIMIT;
+  a.tab = (const Item *)(ws + Pl.o_items);
+  a.ntab = Pl.n_items;
+  a.tp = tp;
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch_tiles(a, std::min(Pl.n_items, std::max(1, c->num_sms)), 1, s);
+  if (e != cudaSuccess) return cuda_status(e, "sliced list launch");
+  *launches += 3;
   return GSKS_OK;
 }
 

@@ -174,3 +174,44 @@ def test_infinite_and_nan_coordinates(gpu):
     for ktype, params in [(0, dict(scal=-1.0)), (1, dict(scal=0.1, cons=1.0, powe=2.0)), (5, {}), (6, dict(cons=1.0))]:
         u, ref = _run(gpu, gsks, ktype, params, g), _run(gpu, gsks, ktype, params, g, noalloc=True)
         np.testing.assert_allclose(u, ref, rtol=1e-10, atol=1e-12)
+
+
+@pytest.mark.parametrize("k", [3, 16, 33, 64, 65, 200])
+def test_lists_of_all_kernels(gpu, oracle_mod, k):
+    """A batch of tasks of every kernel type, of sizes around the tiles and the source
+    chunk (1024), empty ones among them; shared u entries add up."""
+    from ks_gb300 import gsks
+    O = oracle_mod
+    rng = np.random.default_rng(k)
+    N = 3000
+    X = rng.random((N, k)) * (6.0 / k) ** 0.5
+    g = dict(X=X, X2=O.norms(X), w=rng.standard_normal((N, 1)), h=rng.uniform(0.5, 2.0, N))
+    sizes = [(1, 1), (127, 31), (128, 32), (129, 33), (0, 40), (40, 0), (300, 1100), (64, 1024), (200, 1025), (5, 2500)]
+    tasks = []
+    for t in range(2 * len(sizes)):
+        ktype, params = KINDS[t % len(KINDS)]
+        if ktype == 2 and k < 3:
+            continue
+        m, n = sizes[t % len(sizes)]
+        p = _params(ktype, params, 6) if ktype in (0, 1, 4) else dict(params)
+        tasks.append((ktype, p, rng.choice(N, m, replace=False).astype(np.int32), rng.choice(N, n, replace=False).astype(np.int32)))
+    a_off = np.cumsum([0] + [len(t[2]) for t in tasks]).astype(np.int32)
+    b_off = np.cumsum([0] + [len(t[3]) for t in tasks]).astype(np.int32)
+    a_idx = np.concatenate([t[2] for t in tasks]).astype(np.int32)
+    b_idx = np.concatenate([t[3] for t in tasks]).astype(np.int32)
+    kers = [gsks.make_kernel(t[0], **t[1], **(dict(hi=g["h"], hj=g["h"]) if t[0] == 3 else {})) for t in tasks]
+    u = np.zeros(N)
+    gsks.set_precision(gsks.GSKS_FP64)
+    gsks.dgsks_list(kers[0], u, a_off, a_idx, b_off, b_idx, X, g["X2"], X, g["X2"], np.ascontiguousarray(g["w"][:, 0]),
+                    kers=kers)
+    ref, bound = np.zeros(N), np.zeros(N)
+    for ktype, p, a, b in tasks:
+        if not len(a) or not len(b):
+            continue
+        kp = dict(p, **(dict(hi=g["h"], hj=g["h"]) if ktype == 3 else {}))
+        s, c = O.rows(O.make_kernel(ktype, **kp), np.arange(len(a), dtype=np.int32), X, g["X2"], a, X, g["X2"], b,
+                      np.ascontiguousarray(g["w"][:, 0]), b)
+        ref[a] += s
+        gg = dict(g, amap=a, bmap=b)
+        bound[a] += 2.0 * EPS * ((k + 4) * _slope(ktype, p, gg, k) + 64 + 2 * k) * c
+    assert np.all(np.abs(u - ref) <= bound + 32 * EPS * np.abs(ref))
