@@ -84,14 +84,19 @@ constexpr long long WAIT_LIMIT = 1LL << 32;      // clock cycles (~2 s) per wait
 
 static __device__ const ExpTable g_exp_table = ExpTable();
 
-// What the Gaussian's fixed-point form needs, per call (written by
-// slice_kernel): all points on the exponent e, y = A + B - W in units of 2^-F.
+// What the fixed-point form of the Gaussian, variable-bandwidth Gaussian and
+// Laplace kernels needs, per call or task: all points on the exponent e, their
+// distance (the Gaussian: its exponent y) A + B - W in units of 2^-F.
 struct CallParam {
   int fixed;             // the fixed-point form applies
   int e, F;
   int pre;               // left shift of y where F is below 43 (exp2_neg's least), else 0
   int lim, end;          // high words of 1021 2^F and 1088 2^F, at most 2^31 - 1
-  double alpha, ah, al;  // alpha^2 = ah + al
+  int small;             // high word of 2^51, or 0: two norms below it, the pair is formed directly
+  int pad;
+  double alpha, ah, al;  // coordinates are scaled by alpha; alpha^2 = ah + al
+  double pad2;
+  PowFrame pw;           // Laplace
 };
 
 // Kernel selector of the batched (list) form: the epilogue dispatches on each
@@ -136,9 +141,9 @@ struct SliceArgs {
   const double *XA, *XA2, *hi; const int *amap; int nxa;
   const double *XB, *XB2, *hj; const int *bmap; int nxb;
   const double *w; const int *wmap;
-  CallParam frame;         // gauss_frame of the call
+  CallParam frame;         // kernel_frame of the call
   uint8_t *imgA, *imgB;
-  double *row_aa, *row_hi; int *row_e, *row_n;
+  double *row_aa; uint64_t *row_hi; int *row_e, *row_n;
   const ScanPart *scan; int nscan;   // partials; 0: few points, -1: no Gaussian
   CallParam *cp;
   int *next_item;
@@ -223,10 +228,12 @@ __device__ __forceinline__ ScanPart scan_fold(ScanPart r)
 }
 
 // Scan values of points first, first + step, ... of a target list (m positions
-// of amap from a0) followed by a source list (n of bmap from b0): the block's
+// of amap from a0) followed by a source list (n of bmap from b0), with the
+// bandwidth factors hi, hj of the variable-bandwidth kernel: the block's
 // threads take one coordinate of every (256 / k)-th point (a point at a time for
 // long rows).
-__device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int m, int b0, int n, int first, int step)
+__device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int m, int b0, int n, const double *hi,
+                                                const double *hj, int first, int step)
 {
   ScanPart r{0, 1e300, -1e300, 0, 0};
   const int lanes = min(a.k, 256), per = 256 / lanes, c0 = threadIdx.x % lanes, sub = threadIdx.x / lanes;
@@ -241,6 +248,10 @@ __device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int 
       if (c0 == 0) {
         const double nn = A ? a.XA2[p] : a.XB2[p];
         r.bad |= !(nn >= 0.0 && nn < 1e300);
+        if (hi) {            // bandwidth factors: positive and far from the ends of the range
+          const double h = A ? hi[p] : hj[p];
+          r.bad |= !(h > 0x1p-300 && h < 0x1p300);
+        }
         r.nmin = fmin(r.nmin, nn);
         r.nmax = fmax(r.nmax, nn);
       }
@@ -254,31 +265,35 @@ __device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int 
 __global__ void __launch_bounds__(256) scan_kernel(SliceArgs a, ScanPart *__restrict__ part)
 {
   launch_dependents();
-  const ScanPart r = scan_fold(scan_points(a, 0, a.m, 0, a.n, blockIdx.x, gridDim.x));
+  const ScanPart r = scan_fold(scan_points(a, 0, a.m, 0, a.n, a.hi, a.hj, blockIdx.x, gridDim.x));
   if (threadIdx.x == 0) part[blockIdx.x] = r;
 }
 
-__device__ CallParam call_param(const ScanPart &s, CallParam c, int kpad);
+__device__ CallParam call_param(const ScanPart &s, CallParam c, int kt, int kpad);
 
-// The same over one task's points, one block per Gaussian task: its frame.
+// The same over one task's points, one block per task with a frame.
 __global__ void __launch_bounds__(256) list_scan_kernel(SliceArgs a, int ntask, const TaskGeo *__restrict__ tg,
                                                         TaskParam *__restrict__ tp)
 {
   const int t = blockIdx.x;
   launch_dependents();
   if (t == 0 && threadIdx.x == 0) *a.next_item = 0;
-  if (t >= ntask || tp[t].kp.type != KS_GAUSSIAN) return;
+  if (t >= ntask || tp[t].cp.alpha == 0.0) return;
   const TaskGeo G = tg[t];
-  const ScanPart r = scan_fold(scan_points(a, G.a0, G.m, G.b0, G.n, 0, 1));
-  if (threadIdx.x == 0) tp[t].cp = call_param(r, tp[t].cp, a.kpad);
+  const KParams &kp = tp[t].kp;
+  const bool vb = kp.type == KS_GAUSSIAN_VAR_BANDWIDTH;
+  const ScanPart r = scan_fold(scan_points(a, G.a0, G.m, G.b0, G.n, vb ? kp.hi : nullptr, kp.hj, 0, 1));
+  if (threadIdx.x == 0) tp[t].cp = call_param(r, tp[t].cp, tp[t].kp.type, a.kpad);
 }
 
-// The Gaussian's frame from the points' range.  The form applies when every
-// value is finite, the exponent leaves 33 <= F, the norms fit their points,
-// and an absolute error of a few 2^-F in y is no more than FP64's own rounding
-// of the pairs' norms: F >= 52, or every norm sum at least 2^(52 - F).
-// c: alpha, ah, al set (gauss_frame), the rest filled in.
-__device__ CallParam call_param(const ScanPart &s, CallParam c, int kpad)
+// The frame from the points' range.  The form applies when every value is
+// finite, the exponent leaves 33 <= F and the norms fit their points.  An error
+// of a few 2^-F is no more than FP64's own rounding of a pair's norms where
+// their sum is at least 2^(52 - F); a Gaussian's y with F >= 52 needs no more
+// than that anyway.  Pairs of two smaller norms are formed directly; where there
+// may be many (a norm 64 times smaller) the form does not apply.
+// c: what the kernel alone sets (kernel_frame), the rest filled in.
+__device__ CallParam call_param(const ScanPart &s, CallParam c, int kt, int kpad)
 {
   auto pow2 = [](int e) { return __hiloint2double((1023 + e) << 20, 0); };
   c.fixed = 0;
@@ -290,7 +305,10 @@ __device__ CallParam call_param(const ScanPart &s, CallParam c, int kpad)
   c.F = 51 + g - 2 * c.e;
   if (c.F < 33) return c;
   if (s.nmax * c.ah > (double)kpad * pow2(2 * c.e)) return c;
-  if (c.F < 52 && 2.0 * s.nmin * c.ah < pow2(52 - c.F)) return c;
+  const bool relative = kt != KS_GAUSSIAN || c.F < 52;
+  if (relative && s.nmin * c.ah < pow2(45 - c.F)) return c;
+  c.small = relative ? 1 << 19 : 0;
+  if (kt != KS_GAUSSIAN && c.F < 43) return c;
   c.pre = max(0, 43 - c.F);
   c.lim = c.F < 54 ? (int)(1021u << (c.F - 32)) : 0x7fffffff;
   c.end = c.F < 53 ? (int)(1088u << (c.F - 32)) : 0x7fffffff;
@@ -298,17 +316,34 @@ __device__ CallParam call_param(const ScanPart &s, CallParam c, int kpad)
   return c;
 }
 
-// The part of the frame that the kernel alone sets: y = alpha^2 d2 (alpha 0: not
-// a decaying Gaussian, no fixed-point form).
-CallParam gauss_frame(double scal)
+// The part of the frame that the kernel alone sets (alpha 0: no fixed-point
+// form).  Gaussian: y = alpha^2 d2.  Laplace: exponents up to 64 (P <= 128 keeps
+// pow_neg_half's products in 32 bits).
+CallParam kernel_frame(const KParams &kp)
 {
   CallParam c{};
-  const double c2 = -scal * 1.4426950408889634;
-  if (!(c2 > 0x1p-300 && c2 < 0x1p300)) return c;
-  c.alpha = sqrt(c2);
-  c.ah = c.alpha * c.alpha;
-  c.al = fma(c.alpha, c.alpha, -c.ah);
+  if (kp.type == KS_GAUSSIAN) {
+    const double c2 = -kp.scal * 1.4426950408889634;
+    if (!(c2 > 0x1p-300 && c2 < 0x1p300)) return c;
+    c.alpha = sqrt(c2);
+    c.ah = c.alpha * c.alpha;
+    c.al = fma(c.alpha, c.alpha, -c.ah);
+  } else if (kp.type == KS_GAUSSIAN_VAR_BANDWIDTH) {
+    c.alpha = c.ah = 1.0;
+  } else if (kp.type == KS_LAPLACE) {
+    const double P = -2.0 * kp.powe;
+    if (!(P >= 1.0 && P <= 128.0 && P == rint(P))) return c;
+    c.alpha = c.ah = 1.0;
+    c.pw.p8 = (int)P << 8;
+    const uint64_t q = (uint64_t)(0.5L * P * 1.442695040888963407359924681001892137L * 0x1p56L);
+    c.pw.qh = (uint32_t)(q >> 32);
+    c.pw.ql = (uint32_t)q;
+  }
   return c;
+}
+__host__ __device__ constexpr bool has_frame(int kt)
+{
+  return kt == KS_GAUSSIAN || kt == KS_GAUSSIAN_VAR_BANDWIDTH || kt == KS_LAPLACE;
 }
 
 // Digits of eight coordinates as six 16-byte rows of FP16 integers.
@@ -364,11 +399,11 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     // every block folds the scan's partials (at most one per thread) or, for
     // few points, scans them all itself
     ScanPart r{0, 1e300, -1e300, 0, 0};
-    if (a.nscan == 0) r = scan_points(a, 0, a.m, 0, a.n, 0, 1);
+    if (a.nscan == 0) r = scan_points(a, 0, a.m, 0, a.n, a.hi, a.hj, 0, 1);
     else if ((int)threadIdx.x < a.nscan) r = a.scan[threadIdx.x];
     r = scan_fold(r);
     if (threadIdx.x == 0) {
-      s_cp = call_param(r, a.frame, a.kpad);
+      s_cp = call_param(r, a.frame, a.kt, a.kpad);
       if (blockIdx.x == 0) *a.cp = s_cp;
     }
     __syncthreads();
@@ -392,7 +427,7 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     valid = r < tl.y;
     kt = T->kp.type;
     hv = side ? T->kp.hj : T->kp.hi;
-    if (kt == KS_GAUSSIAN) {
+    if (has_frame(kt)) {
       if (threadIdx.x == 0) s_cp = T->cp;
       __syncthreads();
       fixed = s_cp.fixed != 0;
@@ -468,15 +503,24 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
       nn = __longlong_as_double(__double2ll_rn(y));
     }
     const double h = (valid && varbw) ? hv[p] : 0.0;
+    uint64_t hb = (uint64_t)__double_as_longlong(h);
+    if (fixed && varbw) {
+      // the factor (a row's times log2(e) / 2) as a 64-bit mantissa and an
+      // exponent; the words are kept as integers (as FP64 some would be NaN)
+      const double f = valid ? h : 1.0;
+      hb = (uint64_t)__double_as_longlong(side ? f : f * (0.5 * 1.4426950408889634));
+      e = (int)(hb >> 52) - 1023;
+      hb = (hb | 0x10000000000000ull) << 11;
+    }
     if (!side) {
       a.row_aa[slot] = nn;
-      a.row_hi[slot] = h;
+      a.row_hi[slot] = hb;
       a.row_e[slot] = flag ? EFLAG : e;
       if (a.row_n) a.row_n[slot] = 0;
     } else {
       ColMeta *cm = (ColMeta *)(base + op_bytes(BN, a.kpad));
       cm->bb[r] = nn;
-      cm->hj[r] = h;
+      cm->hj[r] = hb;
       cm->e[r] = flag ? EFLAG : e;
       const bool any = __any_sync(0xffffffffu, flag);
       if (lane == 0) { cm->flag = any ? 1 : 0; cm->pad[0] = cm->pad[1] = cm->pad[2] = 0; }
@@ -491,7 +535,7 @@ struct TileArgs {
   int m, n, k, kpad, nrhs;
   int ntm, ntn, nsc, chunk_tiles;   // items = ntm * nsc, chunk_tiles source tiles each
   const uint8_t *imgA, *imgB;
-  const double *row_aa, *row_hi; const int *row_e;
+  const double *row_aa; const uint64_t *row_hi; const int *row_e;
   const double *XA, *XB;            // pools and maps, for the points with EFLAG
   const int *amap, *bmap;
   int nxa, nxb;
@@ -641,20 +685,6 @@ struct RowMeta {
   int e, i;
 };
 
-// The fixed-point Gaussian's value of a pair outside the common range: nearly
-// coincident points, and exponents of 1021 and more.  j: the column's position
-// (-1: a padding column).
-__device__ __noinline__ double rare_value(const TileArgs &a, const CallParam &cp, uint32_t tab, long long y, long long A,
-                                          int i, int j)
-{
-  if (y <= (A >> 38) && i >= 0 && j >= 0)
-    y = __double2ll_rn(near_d2(a, i, j, 0.0) * cp.ah * ldexp(1.0, cp.F));
-  if (y <= 0) return 1.0;
-  if ((int)(y >> 32) < cp.lim) return exp2_neg((uint64_t)y << cp.pre, exp_frame(max(cp.F, 43), tab));
-  if ((int)(y >> 32) >= cp.end) return 0.0;
-  return exp2_neg_wide((double)y * ldexp(1.0, -cp.F));
-}
-
 // Kernel value from the inner product: the functions of kfun64, with the
 // exponentials through exp2_neg and the comparisons of rare cases on the
 // doubles' high words (an FP64 comparison costs as much as an FP64 add).
@@ -715,55 +745,137 @@ __device__ __forceinline__ Place place_of(const TileArgs &a, int item, int row, 
   return Place{row < g.rows ? g.ia + row : -1, g.jb + done, min(COLS, g.cols - done)};
 }
 
-// One thread's columns of a tile, fixed-point Gaussian: W holds y; A: the row's
-// norm in the same units.
-template <int NR>
-__device__ __forceinline__ void fixed_cols(const TileArgs &a, const CallParam &cp, const ExpFrame &E, long long (&W)[COLS],
-                                           long long A, uint32_t cmS, int item, int row, int tj, int c0,
-                                           double (&sum)[NR])
+// A pair's distance where the fixed-point one does not do: nearly coincident
+// points (D at most about 2^-38 of the norms), two small norms.
+__device__ __forceinline__ double direct_d2(const TileArgs &a, const CallParam &cp, long long D, long long A, int i, int j)
+{
+  if (D <= (A >> 38) || (cp.small && (int)(A >> 32) < cp.small)) return near_d2(a, i, j, 0.0);
+  return (double)D * ldexp(1.0, -cp.F);
+}
+
+// The fixed-point value of a pair outside the common range.  j: the column's
+// position (-1: a padding column).
+template <int KT>
+__device__ __noinline__ double rare_value(const TileArgs &a, const KParams &kp, const CallParam &cp, uint32_t tab,
+                                          long long y, long long A, int i, int j)
+{
+  if (i < 0 || j < 0) return 0.0;   // padding: its weight is 0
+  if constexpr (KT == KS_GAUSSIAN) {
+    if (y <= (A >> 38) || (cp.small && (int)(A >> 32) < cp.small))
+      y = __double2ll_rn(near_d2(a, i, j, 0.0) * cp.ah * ldexp(1.0, cp.F));
+    if (y <= 0) return 1.0;
+    if ((int)(y >> 32) >= cp.end) return 0.0;
+    return exp2_neg_deep((uint64_t)y << cp.pre, (int)(y >> 32), cp.lim, exp_frame(max(cp.F, 43), tab));
+  } else {
+    double d2 = direct_d2(a, cp, y, A, i, j);
+    if constexpr (KT == KS_LAPLACE) {
+      // (two coincident points have the same norm)
+      if (d2 < fmax(1e-15, kp.coinc * 2.0 * ((double)A * ldexp(1.0, -cp.F)))) d2 = 1.79e308;
+      return pow_call(d2, kp);      // the row's sum is multiplied by scal
+    } else {
+      const int pa = a.amap ? a.amap[i] : i, pb = a.bmap ? a.bmap[j] : j;
+      return exp2_neg64(((d2 * (0.5 * 1.4426950408889634 * 0x1p53)) * kp.hi[pa]) * kp.hj[pb], tab);
+    }
+  }
+}
+
+// One thread's columns of a tile in the fixed-point form: W holds the distance D
+// (the Gaussian: y); A: the row's norm in the same units; i0: its metadata.
+// Columns outside the common range are left for a loop in which each lane takes
+// a column of its own, since their loads take long.
+template <int KT, int NR>
+__device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp, const CallParam &cp, const ExpFrame &E,
+                                           long long (&W)[COLS], long long A, const ColMeta *cm, uint32_t cmS, int item,
+                                           int row, int i0, int tj, int c0, double (&sum)[NR])
 {
   const uint32_t wS = cmS + (uint32_t)offsetof(ColMeta, w);
   const int lim = cp.lim;
-  // straight-line code where every y of the thread's columns lies in [2^32,
-  // 1021 2^F): independent chains for the schedulers
-  bool rare = false;
-#pragma unroll
-  for (int c = 0; c < COLS; c++) rare |= (uint32_t)((int)(W[c] >> 32) - 1) >= (uint32_t)(lim - 1);
-  if (cp.pre && !rare) {
-#pragma unroll
-    for (int c = 0; c < COLS; c++) W[c] <<= cp.pre;
+  uint32_t mask = 0;
+  // a row of small norm: its columns of small norm too (bb >= 0)
+  if ((int)(A >> 32) < cp.small) {
+#pragma unroll 1
+    for (int c = 0; c < COLS; c++)
+      if (__double2hiint(cm->bb[c0 + c]) < cp.small) mask |= 1u << c;
   }
-  if (!rare) {
+  if constexpr (KT == KS_GAUSSIAN) {
+    // straight-line code where every y of the thread's columns lies in [2^32,
+    // 1021 2^F): independent chains for the schedulers
+    bool rare = mask != 0;
+#pragma unroll
+    for (int c = 0; c < COLS; c++) rare |= (uint32_t)((int)(W[c] >> 32) - 1) >= (uint32_t)(lim - 1);
+    if (cp.pre && !rare) {
+#pragma unroll
+      for (int c = 0; c < COLS; c++) W[c] <<= cp.pre;
+    }
+    if (!rare) {
+#pragma unroll
+      for (int c = 0; c < COLS; c += 2) {
+        const double k0 = exp2_neg((uint64_t)W[c], E), k1 = exp2_neg((uint64_t)W[c + 1], E);
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+          if (r > 0 && r >= a.nrhs) continue;
+          double w0, w1;
+          lds2(wS + (r * BN + c) * 8, w0, w1);
+          sum[r] = fma(k1, w1, fma(k0, w0, sum[r]));
+        }
+      }
+      return;
+    }
+    // the common columns one by one (values of 1088 and more are 0, times w)
+    const int yend = cp.end;
+#pragma unroll
+    for (int c = 0; c < COLS; c++) {
+      const int yh = (int)(W[c] >> 32);
+      if (yh <= 0 || (mask >> c & 1u)) {
+        mask |= 1u << c;
+      } else {
+        const double kv = yh < yend ? exp2_neg_deep((uint64_t)W[c] << cp.pre, yh, lim, E) : 0.0;
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+          if (r > 0 && r >= a.nrhs) continue;
+          double w0;
+          lds1(wS + (r * BN + c) * 8, w0);
+          sum[r] = fma(kv, w0, sum[r]);
+        }
+      }
+    }
+  } else {
+    uint64_t Mi = 0;
+    int ei = 0;
+    if constexpr (KT == KS_GAUSSIAN_VAR_BANDWIDTH) {
+      Mi = a.row_hi[i0];
+      ei = a.row_e[i0];
+    }
+    const PowFrame pw = cp.pw;
+    const int F = cp.F;
 #pragma unroll
     for (int c = 0; c < COLS; c += 2) {
-      const double k0 = exp2_neg((uint64_t)W[c], E), k1 = exp2_neg((uint64_t)W[c + 1], E);
+      double kv[2];
+      bool good[2];
+#pragma unroll
+      for (int s = 0; s < 2; s++) {
+        const long long D = W[c + s];
+        good[s] = (int)(D >> 32) > 0 && !(mask >> (c + s) & 1u);
+        if constexpr (KT == KS_LAPLACE) {
+          bool ok;
+          kv[s] = pow_neg_half((uint64_t)D, F, pw, E, ok);
+          good[s] = good[s] && ok;
+        } else {
+          int zh;
+          kv[s] = exp2_neg_scaled((uint64_t)D, F, Mi, cm->hj[c0 + c + s],
+                                  ei + cm->e[c0 + c + s], E, zh);
+          if (good[s] && zh >= (1088 << 20)) kv[s] = 0.0;      // beyond 2^-1088: 0, times w
+          else good[s] = good[s] && zh > 0;
+        }
+        mask = good[s] ? mask : mask | (1u << (c + s));
+      }
 #pragma unroll
       for (int r = 0; r < NR; r++) {
         if (r > 0 && r >= a.nrhs) continue;
         double w0, w1;
         lds2(wS + (r * BN + c) * 8, w0, w1);
-        sum[r] = fma(k1, w1, fma(k0, w0, sum[r]));
-      }
-    }
-    return;
-  }
-  // the common columns one by one (values of 1088 and more are 0, times w), the
-  // others after them, each lane at a column of its own: their loads take long
-  const int yend = cp.end;
-  uint32_t mask = 0;
-#pragma unroll
-  for (int c = 0; c < COLS; c++) {
-    const int yh = (int)(W[c] >> 32);
-    if (yh < yend && (uint32_t)(yh - 1) >= (uint32_t)(lim - 1)) {
-      mask |= 1u << c;
-    } else {
-      const double kv = yh < yend ? exp2_neg((uint64_t)W[c] << cp.pre, E) : 0.0;
-#pragma unroll
-      for (int r = 0; r < NR; r++) {
-        if (r > 0 && r >= a.nrhs) continue;
-        double w0;
-        lds1(wS + (r * BN + c) * 8, w0);
-        sum[r] = fma(kv, w0, sum[r]);
+        if (good[0]) sum[r] = fma(kv[0], w0, sum[r]);
+        if (good[1]) sum[r] = fma(kv[1], w1, sum[r]);
       }
     }
   }
@@ -774,7 +886,7 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const CallParam &c
     long long y = W[0];
 #pragma unroll
     for (int q = 1; q < COLS; q++) y = c == q ? W[q] : y;
-    const double kv = rare_value(a, cp, E.tab, y, A, P.i, c < P.nv ? P.j0 + c : -1);
+    const double kv = rare_value<KT>(a, kp, cp, E.tab, y, A, P.i, c < P.nv ? P.j0 + c : -1);
 #pragma unroll
     for (int r = 0; r < NR; r++) {
       if (r > 0 && r >= a.nrhs) continue;
@@ -807,7 +919,8 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
         if (a.nxb >= 0 && (pb < 0 || pb >= a.nxb)) pb = 0;
         dot = dot_direct(a.XA + (size_t)pa * a.k, a.XB + (size_t)pb * a.k, a.k);
       }
-      const double kv = kvalue<KT>(a, kp, j, dot, am, cm->bb[c0 + c], cm->hj[c0 + c], cfold, tab);
+      const double kv = kvalue<KT>(a, kp, j, dot, am, cm->bb[c0 + c],
+                                    __longlong_as_double((long long)cm->hj[c0 + c]), cfold, tab);
 #pragma unroll
       for (int r = 0; r < NR; r++)
         if (r == 0 || r < a.nrhs) sum[r] = fma(kv, cm->w[r][c0 + c], sum[r]);
@@ -815,7 +928,7 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
   }
 }
 
-constexpr bool uses_table(int kt) { return kt == KS_GAUSSIAN || kt == KS_GAUSSIAN_VAR_BANDWIDTH || kt == KS_LIST; }
+constexpr bool uses_table(int kt) { return has_frame(kt) || kt == KS_LIST; }
 
 // G: guard bits of the resident layouts (k <= 32: 3, k <= 64: 2), -1: streaming.
 // A thread's partial sums of row i are stored; the last of the row's parts
@@ -1011,7 +1124,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     const int row = qd * 32 + lane, c0 = (grp & 1) * COLS;
     const uint32_t tT = tmem + ((uint32_t)(qd * 32) << 16) + half * TBUF + c0;
     const int gb = G >= 0 ? G : guard_bits(a.kpad);
-    constexpr int SIGN = KT == KS_GAUSSIAN || KT == KS_LIST ? -1 : 1;   // W or -W
+    constexpr bool FRAMED = has_frame(KT) || KT == KS_LIST;
+    constexpr int SIGN = FRAMED ? -1 : 1;           // W or -W
     const uint32_t bias = combine_bias<SIGN>(gb);
     const uint32_t tabS = smem_addr(sTab);
     int tbase = 0, tg = 0;                          // tiles before this item, accumulations taken
@@ -1029,8 +1143,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
       const KParams &kp = KT == KS_LIST ? S->tslot[it & 1].kp : a.kp;
       const CallParam &cp = KT == KS_LIST ? S->tslot[it & 1].cp : *a.cp;
       const int type = KT == KS_LIST ? kp.type : KT;
-      const bool fixed = (KT == KS_GAUSSIAN || (KT == KS_LIST && type == KS_GAUSSIAN)) && cp.fixed != 0;
-      const ExpFrame E = exp_frame(max(fixed ? cp.F : 43, 43), tabS);
+      const bool fixed = FRAMED && cp.fixed != 0;
+      const ExpFrame E = type == KS_GAUSSIAN ? exp_frame(max(fixed ? cp.F : 43, 43), tabS) : exp_frame52(tabS);
       const long long arow = __double_as_longlong(a.row_aa[i0]);
       const bool anyrow = __any_sync(0xffffffffu, a.row_e[i0] == EFLAG);
       double racc[NR];
@@ -1059,7 +1173,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
             if (STREAM && c > 0) {
 #pragma unroll
               for (int s = 0; s < 4; s++) w0[s] += W[q + s];
-            } else if ((KT == KS_GAUSSIAN || KT == KS_LIST) && fixed) {
+            } else if (FRAMED && fixed) {
               lds2(cmS + q * 8, w0[0], w0[1]);
               lds2(cmS + q * 8 + 16, w0[2], w0[3]);
 #pragma unroll
@@ -1079,11 +1193,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
         double tsum[NR];
 #pragma unroll
         for (int r = 0; r < NR; r++) tsum[r] = 0.0;
-        if ((KT == KS_GAUSSIAN || KT == KS_LIST) && fixed) {
-          fixed_cols<NR>(a, cp, E, W, arow, cmS, item, row, tj, c0, tsum);
+        if (FRAMED && fixed) {
+#define GSKS_COLS(T) fixed_cols<T, NR>(a, kp, cp, E, W, arow, cm, cmS, item, row, i0, tj, c0, tsum)
+          if constexpr (KT == KS_LIST) {
+            if (type == KS_GAUSSIAN) GSKS_COLS(KS_GAUSSIAN);
+            else if (type == KS_LAPLACE) GSKS_COLS(KS_LAPLACE);
+            else GSKS_COLS(KS_GAUSSIAN_VAR_BANDWIDTH);
+          } else if constexpr (FRAMED) {
+            GSKS_COLS(KT);
+          }
+#undef GSKS_COLS
         } else {
           const Place P = place_of(a, item, row, tj, c0);
-          const RowMeta am{__longlong_as_double(arow), a.row_hi[i0], a.row_e[i0], P.i};
+          const RowMeta am{__longlong_as_double(arow), __longlong_as_double((long long)a.row_hi[i0]), a.row_e[i0], P.i};
           const bool slow = anyrow || cm->flag != 0;
 #define GSKS_COLS(T) dot_cols<T, NR, SIGN>(a, kp, W, am, cm, c0, P, gb, slow, tabS, tsum)
           if constexpr (KT == KS_LIST) {
@@ -1111,6 +1233,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
       if (!ok) break;
       tbase += t1 - t0;
       const Item g = item_geo(a, item);
+      if ((KT == KS_LAPLACE || KT == KS_LIST) && fixed && type == KS_LAPLACE) {
+#pragma unroll
+        for (int r = 0; r < NR; r++) racc[r] *= kp.scal;
+      }
       if constexpr (NR > 1) {
         // every group writes its own partials; the reduction adds them in order
         const int sc = item / a.ntm;
@@ -1227,7 +1353,9 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
     }
   }
   const int ldp = ntm * BM;
-  const bool gauss = ker->type == KS_GAUSSIAN, scan = gauss && ((long long)m + n) * k > SCAN_SELF;
+  const KParams kp = make_kparams(ker, hi, hj);
+  const CallParam frame = kernel_frame(kp);
+  const bool framed = frame.alpha != 0.0, scan = framed && ((long long)m + n) * k > SCAN_SELF;
   const int nscan = scan ? (int)std::min<long long>(SCAN_MAX, ((long long)m + n + 7) / 8) : 0;
 
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -1254,15 +1382,16 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
 
   SliceArgs p{};
   p.m = m; p.n = n; p.k = k; p.kpad = kpad; p.kt = ker->type; p.nrhs = nrhs; p.nr = nr;
-  p.XA = XA; p.XA2 = XA2; p.hi = hi; p.amap = amap; p.nxa = nxa;
-  p.XB = XB; p.XB2 = XB2; p.hj = hj; p.bmap = bmap; p.nxb = nxb;
+  const bool varbw = ker->type == KS_GAUSSIAN_VAR_BANDWIDTH;
+  p.XA = XA; p.XA2 = XA2; p.hi = varbw ? hi : nullptr; p.amap = amap; p.nxa = nxa;
+  p.XB = XB; p.XB2 = XB2; p.hj = varbw ? hj : nullptr; p.bmap = bmap; p.nxb = nxb;
   p.w = w; p.wmap = wmap;
-  p.frame = gauss_frame(ker->scal);
   p.nta = ntm;
   p.imgA = ws + o_a; p.imgB = ws + o_b;
-  p.row_aa = (double *)(ws + o_aa); p.row_hi = (double *)(ws + o_hi); p.row_e = (int *)(ws + o_e);
+  p.row_aa = (double *)(ws + o_aa); p.row_hi = (uint64_t *)(ws + o_hi); p.row_e = (int *)(ws + o_e);
   p.row_n = (int *)(ws + o_n);
-  p.scan = (const ScanPart *)(ws + o_scan); p.nscan = gauss ? nscan : -1;
+  p.scan = (const ScanPart *)(ws + o_scan); p.nscan = framed ? nscan : -1;
+  p.frame = frame;
   p.cp = (CallParam *)(ws + o_cp);
   p.next_item = (int *)(ws + o_next);
   p.err = err_word(c);
@@ -1281,7 +1410,7 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   a.imgA = p.imgA; a.imgB = p.imgB;
   a.row_aa = p.row_aa; a.row_hi = p.row_hi; a.row_e = p.row_e;
   a.XA = XA; a.XB = XB; a.amap = amap; a.bmap = bmap; a.nxa = nxa; a.nxb = nxb;
-  a.kp = make_kparams(ker, hi, hj);
+  a.kp = kp;
   a.kp.coinc = coincidence_eps(k);
   a.cp = p.cp;
   a.partial = (double *)(ws + o_p);
@@ -1333,7 +1462,7 @@ int sliced_list_plan(SlicedListPlan &Pl, const KParams *kps, int ntask, int k, c
     tg[t] = TaskGeo{hoff_a[t], m, hoff_b[t], n};
     memset(&tp[t], 0, sizeof(TaskParam));
     tp[t].kp = kps[t];
-    if (kps[t].type == KS_GAUSSIAN) tp[t].cp = gauss_frame(kps[t].scal);
+    tp[t].cp = kernel_frame(kps[t]);
     if (m <= 0 || n <= 0) continue;
     for (int q = ota[t]; q < ota[t + 1]; q++) {
       const int i0 = (q - ota[t]) * BM;
@@ -1345,8 +1474,8 @@ int sliced_list_plan(SlicedListPlan &Pl, const KParams *kps, int ntask, int k, c
       tb[q] = make_int2(hoff_b[t] + j0, std::min(BN, n - j0));
       tb_task[q] = t;
     }
-    // relative epilogue cost of a tile: FP64 instructions of a value
-    const int wkt = kps[t].type == KS_LAPLACE ? 10 : kps[t].type == KS_GAUSSIAN ? 2 : kps[t].type == KS_TANH ? 12 : 4;
+    // relative epilogue cost of a tile
+    const int wkt = kps[t].type == KS_TANH ? 12 : kps[t].type == KS_GAUSSIAN ? 2 : 3;
     long long q = oit[t];
     for (int b0 = otb[t]; b0 < otb[t + 1]; b0 += chunk_tiles)
       for (int i0 = 0; i0 < m; i0 += BM, q++) {
@@ -1378,8 +1507,8 @@ int sliced_list_plan(SlicedListPlan &Pl, const KParams *kps, int ntask, int k, c
   auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
   Pl.ntask = ntask; Pl.k = k; Pl.kpad = kpad;
   Pl.n_ta = (int)ta.size(); Pl.n_tb = (int)tb.size(); Pl.n_items = (int)items.size();
-  Pl.any_gauss = false;
-  for (int t = 0; t < ntask && !Pl.any_gauss; t++) Pl.any_gauss = kps[t].type == KS_GAUSSIAN;
+  Pl.any_frame = false;
+  for (int t = 0; t < ntask && !Pl.any_frame; t++) Pl.any_frame = has_frame(kps[t].type);
   const size_t rows = (size_t)Pl.n_ta * BM;
   Pl.o_next = 0;
   Pl.o_ta = al(4);
@@ -1424,7 +1553,7 @@ int sliced_list_run(const SlicedListPlan &Pl, Ctx *c, const double *XA, const do
   p.XB = XB; p.XB2 = XB2; p.bmap = b_idx; p.nxb = nxb;
   p.w = w; p.wmap = w_idx;
   p.imgA = ws + Pl.o_a; p.imgB = ws + Pl.o_b;
-  p.row_aa = (double *)(ws + Pl.o_aa); p.row_hi = (double *)(ws + Pl.o_hi); p.row_e = (int *)(ws + Pl.o_e);
+  p.row_aa = (double *)(ws + Pl.o_aa); p.row_hi = (uint64_t *)(ws + Pl.o_hi); p.row_e = (int *)(ws + Pl.o_e);
   p.next_item = (int *)(ws + Pl.o_next);
   p.err = err;
   p.tilesA = (const int2 *)(ws + Pl.o_ta); p.taskA = (const int *)(ws + Pl.o_tat);
@@ -1432,7 +1561,7 @@ int sliced_list_run(const SlicedListPlan &Pl, Ctx *c, const double *XA, const do
   p.tp = tp;
   p.nta = Pl.n_ta;
   // (also clears the work counter)
-  list_scan_kernel<<<Pl.any_gauss ? Pl.ntask : 1, 256, 0, s>>>(p, Pl.ntask, (const TaskGeo *)(ws + Pl.o_tg), tp);
+  list_scan_kernel<<<Pl.any_frame ? Pl.ntask : 1, 256, 0, s>>>(p, Pl.ntask, (const TaskGeo *)(ws + Pl.o_tg), tp);
   cudaError_t e = launch_after(slice_kernel, Pl.n_ta * (BM / 32) + Pl.n_tb * (BN / 32), 256, 0, s, p);
   TileArgs a{};
   a.k = Pl.k; a.kpad = Pl.kpad; a.nrhs = 1; a.ntm = 1;

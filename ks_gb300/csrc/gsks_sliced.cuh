@@ -26,7 +26,7 @@ constexpr int ETAB = 2048;           // entries of the 2^-f table
 // tile holds a point with EFLAG, and the weight columns.
 struct ColMeta {
   double bb[BN];
-  double hj[BN];
+  uint64_t hj[BN];      // FP64 bits, or (fixed-point form) the mantissa
   int e[BN];
   int flag;
   int pad[3];
@@ -37,7 +37,7 @@ static_assert(colmeta_bytes(1) % 16 == 0 && sizeof(ColMeta) % 16 == 0, "ColMeta 
 
 // ---------------------------------------------------------------------------
 // 2^-(i / ETAB) in units of 2^-64, i = 0 .. ETAB - 1 (the first one unit short
-// of 1), plus 1300: half of 2^-53 for exp2_neg's last shift and the mean of its
+// of 1), plus EXP_BIAS: half of 2^-53 for exp2_neg's last shift and the mean of its
 // floors.  Products of the eleven constants 2^(-2^b / ETAB) in 64-bit fixed point,
 // evaluated by the compiler.
 constexpr uint64_t mulhi64c(uint64_t a, uint64_t b)
@@ -47,6 +47,7 @@ constexpr uint64_t mulhi64c(uint64_t a, uint64_t b)
   const uint64_t n = al * bh + (m & 0xffffffffu);
   return ah * bh + (m >> 32) + (n >> 32);
 }
+constexpr uint64_t EXP_BIAS = 1300;
 struct ExpTable {
   uint64_t v[ETAB];
   constexpr ExpTable() : v()
@@ -63,7 +64,7 @@ struct ExpTable {
           p = first ? c[b] : mulhi64c(p, c[b]);
           first = false;
         }
-      v[i] = p + 1300;
+      v[i] = p + EXP_BIAS;
     }
   }
 };
@@ -102,7 +103,7 @@ __device__ __forceinline__ void lds1(uint32_t addr, double &a)
   asm volatile("ld.shared.f64 %0, [%1];" : "=d"(a) : "r"(addr));
 }
 
-// 2^-y for y = z 2^-F, 2^-21 <= y < 1021, to about one unit in the last place:
+// 2^-y for y = z 2^-F, 2^-21 <= |y| < 1021, to about one unit in the last place:
 // y = n + (i + phi) / 2048, 2^-y = 2^-n T[i] (1 - P), P = 1 - 2^(-phi / 2048)
 // (the table-driven scheme of P. T. P. Tang, ACM TOMS 15 (1989), in integers).
 // FP64 instructions issue at 1/32 of the integer rate here (2 against 64 per
@@ -133,7 +134,8 @@ __device__ __forceinline__ ExpFrame exp_frame(int F, uint32_t tab)
 __device__ __forceinline__ double exp2_neg(uint64_t z, const ExpFrame &E)
 {
   const uint32_t hi = (uint32_t)(z >> 32), lo = (uint32_t)z;
-  const uint32_t v = hi >> E.s, f = __funnelshift_r(lo, hi, E.s);          // n 2048 + i, phi's upper 32 bits
+  const int v = (int)hi >> E.s;
+  const uint32_t f = __funnelshift_r(lo, hi, E.s);    // v = n 2048 + i, phi's upper 32 bits
   uint64_t t;
   asm("ld.shared.u64 %0, [%1];" : "=l"(t) : "r"(E.tab + (v & (ETAB - 1)) * 8));
   const uint64_t lin = madw(lo & E.mask, E.mul, madw(f, 2977044472u, 0));
@@ -142,7 +144,56 @@ __device__ __forceinline__ double exp2_neg(uint64_t z, const ExpFrame &E)
   const uint32_t th = (uint32_t)(t >> 32), tl = (uint32_t)t, ph = (uint32_t)(p >> 32), pl = (uint32_t)p;
   const uint64_t s = madw(th, ph, 0) + mulhi(th, pl) + mulhi(tl, ph);      // T P
   const uint64_t m = (t - s) >> 11;                                        // [2^52, 2^53], units of 2^-53
-  return __hiloint2double((int)((uint32_t)(m >> 32) + (1021u << 20) - (v >> 11) * (1u << 20)), (int)(uint32_t)m);
+  return __hiloint2double((int)((uint32_t)(m >> 32) + (1021u << 20)) - (v >> 11) * (1 << 20), (int)(uint32_t)m);
+}
+
+// High 64 bits of a 64 x 64 bit product, less at most 2 units (three of the four
+// partial products).
+__device__ __forceinline__ uint64_t mulhi64(uint64_t a, uint64_t b)
+{
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+  return madw(ah, bh, 0) + mulhi(ah, bl) + mulhi(al, bh);
+}
+
+// d^-(P / 2) for d = D 2^-F, D >= 2^32, as 2^-y, y = (P / 2) log2 d, in integers:
+// D = m 2^lz', m in [1, 2) 2^63; j = 2048 log2 m to the nearest integer from the
+// SFU's logarithm; r = m T[j] - 1 (T of exp2_neg: a power of two of j / 2048, so
+// its logarithm needs no table), |r| < 2^-12.4; log2 d = E + j / 2048 + log2(1 +
+// r), ln(1 + r) = r - r^2 (1/2 - r / 3 + r^2 / 4).
+// (The general pow, or binary powering with its division, takes 16 to 20 FP64
+// instructions, 8 to 10 SM cycles a value; this about 35 integer ones and
+// exp2_neg.)  The error of y is about Q 2^-55, Q = P log2(e) / 2, to be compared
+// with the distance's own: P / 2 times its rounding, 2^-53 (|x|^2 + |y|^2) / d2.
+struct PowFrame {
+  int p8;                 // P 2^8: y's part from E + j / 2048, in units of 2^-52
+  uint32_t qh, ql;        // Q 2^56 (P <= 128: qh below 2^31)
+  int pad;
+};
+// E: exp_frame52.  ok: y in (-1000, 1000).
+__device__ __forceinline__ double pow_neg_half(uint64_t D, int F, const PowFrame &Q, const ExpFrame &E, bool &ok)
+{
+  const int lz = __clz((int)(D >> 32));
+  const uint64_t m = D << lz;
+  const uint32_t mh = (uint32_t)(m >> 32);
+  float l;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(__uint_as_float(0x3f800000u | ((mh >> 8) & 0x7fffffu))));
+  const int j = __float_as_int(fmaf(l, 2048.0f, 12582912.0f)) - 0x4B400000;       // 0 .. 2048
+  const int J = (63 - F - lz) * 2048 + j;
+  uint64_t t;
+  asm("ld.shared.u64 %0, [%1];" : "=l"(t) : "r"(E.tab + (j & (ETAB - 1)) * 8));
+  t = (j & (ETAB - 1)) ? t - (EXP_BIAS + 170) : t;   // (170: the mean of r2's floor)
+  // j = 2048: T[0] / 2, m just below 2
+  const uint64_t pr = mulhi64(m, j == ETAB ? t >> 1 : t);                         // (1 + r) 2^63
+  const long long r = (long long)(pr ^ 0x8000000000000000ull);
+  const int rs = (int)(r >> 20);                                                  // units of 2^-43
+  const uint32_t r2 = (uint32_t)(madws(rs, rs, 0) >> 32);                         // 2^-54
+  const uint32_t c = (uint32_t)(madws(rs, -349525, (long long)1 << 62) >> 32) + (r2 >> 25);   // 1/2 - r / 3 + r^2 / 4, 2^-31
+  const long long u = r - (long long)(madw(r2, c, 0) >> 22);
+  const long long qu = madws((int)(u >> 32), (int)Q.qh, (long long)mulhi((uint32_t)u, Q.qh)) +
+                       (madws((int)(u >> 32), (int)(Q.ql >> 1), 0) >> 31);        // Q u, units of 2^-55
+  const long long y = (qu >> 3) + ((long long)((uint64_t)(uint32_t)(J * Q.p8) << 32));   // 2^-52
+  ok = (uint32_t)((int)(y >> 32) + (1000 << 20)) < (2000u << 20);
+  return exp2_neg((uint64_t)y, E);
 }
 
 // 2^-y outside exp2_neg's range (y negative, beyond 1021, or no number).
@@ -161,6 +212,33 @@ __device__ __forceinline__ double exp2_neg64(double y53, uint32_t tab)
   }
   return exp2_neg((uint64_t)z, ExpFrame{10, 1023u, 2907270u, tab});
 }
+
+// exp2_neg for y up to 1088 (hi: z's high word, lim: that of 1021): beyond 1021
+// the value is formed 2^512 too large and rounded into the subnormal range by
+// one multiplication.
+__device__ __forceinline__ double exp2_neg_deep(uint64_t z, int hi, int lim, const ExpFrame &E)
+{
+  const bool deep = hi >= lim;
+  double v = exp2_neg(deep ? z - ((uint64_t)512 << (E.s + 43)) : z, E);
+  if (deep) v *= 0x1p-512;
+  return v;
+}
+
+// 2^-y for y = D 2^-F h_i h_j with the (positive) factors as 64-bit mantissas (Mi,
+// Mj, leading bit set) and the sum ex of their exponents (value = M 2^(ex - 63)):
+// D normalised, two products, one shift.  zh: the high word of y 2^52, saturated
+// (the value holds for zh in [1, 1088 2^20)).
+__device__ __forceinline__ double exp2_neg_scaled(uint64_t D, int F, uint64_t Mi, uint64_t Mj, int ex, const ExpFrame &E52,
+                                                  int &zh)
+{
+  const int lz = __clzll((long long)D);
+  const uint64_t t = mulhi64(mulhi64(D << lz, Mi), Mj);   // in [2^61, 2^64)
+  const int s = F + lz - ex - 54;                          // y 2^52 = t 2^-s
+  const uint64_t z = s < 0 ? t << 1 : t >> min(s, 63);     // (s < 0: y at least 1024)
+  zh = s < -1 || (s < 0 && (t >> 62)) ? 0x7fffffff : (int)min((uint32_t)(z >> 32), 0x7fffffffu);
+  return exp2_neg_deep(z, zh, 1021 << 20, E52);
+}
+__device__ __forceinline__ ExpFrame exp_frame52(uint32_t tab) { return ExpFrame{9, 511u, 5814540u, tab}; }
 
 }  // namespace sliced
 }  // namespace gsks
