@@ -124,12 +124,11 @@ struct TaskGeo {
   int a0, m, b0, n;
 };
 
-// One block's share of the scan: largest |coordinate| (as ordered bits), the
-// norms' range, whether anything is not finite.
+// One block's share of the scan, by high words (one reduction instruction each;
+// small calls wait for this code to be fetched): the largest |coordinate|, the
+// least and the largest norm (all ones: a value the form does not take).
 struct ScanPart {
-  unsigned long long maxabs;
-  double nmin, nmax;
-  int bad, pad;
+  uint32_t maxabs, nmin, nmax, pad;
 };
 constexpr int SCAN_MAX = 256;
 // Coordinates up to which every block of slice_kernel scans all points itself
@@ -207,23 +206,17 @@ cudaError_t launch_after(void (*kernel)(A...), int grid, int block, size_t smem,
 __device__ __forceinline__ ScanPart scan_fold(ScanPart r)
 {
   __shared__ ScanPart part[8];
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    r.maxabs = max(r.maxabs, __shfl_xor_sync(0xffffffffu, r.maxabs, o));
-    r.nmin = fmin(r.nmin, __shfl_xor_sync(0xffffffffu, r.nmin, o));
-    r.nmax = fmax(r.nmax, __shfl_xor_sync(0xffffffffu, r.nmax, o));
-  }
-  r.bad = __any_sync(0xffffffffu, r.bad);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = r;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  r.maxabs = __reduce_max_sync(full, r.maxabs);
+  r.nmin = __reduce_min_sync(full, r.nmin);
+  r.nmax = __reduce_max_sync(full, r.nmax);
+  if (lane == 0) part[threadIdx.x >> 5] = r;
   __syncthreads();
-  r = part[0];
-#pragma unroll
-  for (int q = 1; q < 8; q++) {
-    r.maxabs = max(r.maxabs, part[q].maxabs);
-    r.nmin = fmin(r.nmin, part[q].nmin);
-    r.nmax = fmax(r.nmax, part[q].nmax);
-    r.bad |= part[q].bad;
-  }
+  r = part[lane & 7];
+  r.maxabs = __reduce_max_sync(full, r.maxabs);
+  r.nmin = __reduce_min_sync(full, r.nmin);
+  r.nmax = __reduce_max_sync(full, r.nmax);
   return r;
 }
 
@@ -235,25 +228,24 @@ __device__ __forceinline__ ScanPart scan_fold(ScanPart r)
 __device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int m, int b0, int n, const double *hi,
                                                 const double *hj, int first, int step)
 {
-  ScanPart r{0, 1e300, -1e300, 0, 0};
+  ScanPart r{0, ~0u, 0, 0};
   const int lanes = min(a.k, 256), per = 256 / lanes, c0 = threadIdx.x % lanes, sub = threadIdx.x / lanes;
   if (sub < per) {
-#pragma unroll 4
+#pragma unroll 2
     for (int i = first * per + sub; i < m + n; i += step * per) {
       const bool A = i < m;
       const int p = A ? pool_index(a.amap, a0 + i, a.nxa, a.err) : pool_index(a.bmap, b0 + i - m, a.nxb, a.err);
       const double *x = (A ? a.XA : a.XB) + (size_t)p * a.k;
       for (int c = c0; c < a.k; c += lanes)
-        r.maxabs = max(r.maxabs, (unsigned long long)__double_as_longlong(x[c]) & 0x7fffffffffffffffull);
+        r.maxabs = max(r.maxabs, (uint32_t)__double2hiint(x[c]) & 0x7fffffffu);
       if (c0 == 0) {
-        const double nn = A ? a.XA2[p] : a.XB2[p];
-        r.bad |= !(nn >= 0.0 && nn < 1e300);
-        if (hi) {            // bandwidth factors: positive and far from the ends of the range
-          const double h = A ? hi[p] : hj[p];
-          r.bad |= !(h > 0x1p-300 && h < 0x1p300);
+        uint32_t nn = (uint32_t)__double2hiint(A ? a.XA2[p] : a.XB2[p]);
+        if (hi) {            // bandwidth factors: within 2^-300 .. 2^300
+          const uint32_t h = (uint32_t)__double2hiint(A ? hi[p] : hj[p]);
+          if (h - (723u << 20) >= 600u << 20) nn = ~0u;
         }
-        r.nmin = fmin(r.nmin, nn);
-        r.nmax = fmax(r.nmax, nn);
+        r.nmin = min(r.nmin, nn);
+        r.nmax = max(r.nmax, nn);
       }
     }
   }
@@ -297,16 +289,19 @@ __device__ CallParam call_param(const ScanPart &s, CallParam c, int kt, int kpad
 {
   auto pow2 = [](int e) { return __hiloint2double((1023 + e) << 20, 0); };
   c.fixed = 0;
-  const double mx = __longlong_as_double((long long)s.maxabs) * c.alpha;
-  if (c.alpha == 0.0 || s.bad || !(mx < 0x1p30)) return c;
+  // (upper bounds of the largest values, a lower one of the least norm)
+  if (c.alpha == 0.0 || s.maxabs >= 0x7fe00000u || s.nmax >= 0x7fe00000u) return c;
+  const double mx = __hiloint2double((int)s.maxabs + 1, 0) * c.alpha;
+  if (!(mx < 0x1p30)) return c;
   // e as low as the points allow (mx < 2^e), F = 51 + g - 2 e at most 62
   const int g = guard_bits(kpad);
   c.e = max((g - 11 + 1) / 2, (__double2hiint(mx) >> 20) - 1022);
   c.F = 51 + g - 2 * c.e;
   if (c.F < 33) return c;
-  if (s.nmax * c.ah > (double)kpad * pow2(2 * c.e)) return c;
+  const double nmin = __hiloint2double((int)s.nmin, 0), nmax = __hiloint2double((int)s.nmax + 1, 0);
+  if (nmax * c.ah > (double)kpad * pow2(2 * c.e)) return c;
   const bool relative = kt != KS_GAUSSIAN || c.F < 52;
-  if (relative && s.nmin * c.ah < pow2(45 - c.F)) return c;
+  if (relative && nmin * c.ah < pow2(45 - c.F)) return c;
   c.small = relative ? 1 << 19 : 0;
   if (kt != KS_GAUSSIAN && c.F < 43) return c;
   c.pre = max(0, 43 - c.F);
@@ -398,7 +393,7 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
   } else if (a.nscan >= 0) {
     // every block folds the scan's partials (at most one per thread) or, for
     // few points, scans them all itself
-    ScanPart r{0, 1e300, -1e300, 0, 0};
+    ScanPart r{0, ~0u, 0, 0};
     if (a.nscan == 0) r = scan_points(a, 0, a.m, 0, a.n, a.hi, a.hj, 0, 1);
     else if ((int)threadIdx.x < a.nscan) r = a.scan[threadIdx.x];
     r = scan_fold(r);
@@ -821,22 +816,27 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp,
       }
       return;
     }
-    // the common columns one by one (values of 1088 and more are 0, times w)
+    // the columns in the range (values of 1088 and more are 0, times w)
     const int yend = cp.end;
 #pragma unroll
-    for (int c = 0; c < COLS; c++) {
-      const int yh = (int)(W[c] >> 32);
-      if (yh <= 0 || (mask >> c & 1u)) {
-        mask |= 1u << c;
-      } else {
-        const double kv = yh < yend ? exp2_neg_deep((uint64_t)W[c] << cp.pre, yh, lim, E) : 0.0;
+    for (int c = 0; c < COLS; c += 2) {
+      double kv[2];
+      bool good[2];
 #pragma unroll
-        for (int r = 0; r < NR; r++) {
-          if (r > 0 && r >= a.nrhs) continue;
-          double w0;
-          lds1(wS + (r * BN + c) * 8, w0);
-          sum[r] = fma(kv, w0, sum[r]);
-        }
+      for (int s = 0; s < 2; s++) {
+        const int yh = (int)(W[c + s] >> 32);
+        good[s] = yh > 0 && !(mask >> (c + s) & 1u);
+        kv[s] = exp2_neg_deep((uint64_t)W[c + s] << cp.pre, yh, lim, E);
+        kv[s] = yh < yend ? kv[s] : 0.0;
+        mask = good[s] ? mask : mask | (1u << (c + s));
+      }
+#pragma unroll
+      for (int r = 0; r < NR; r++) {
+        if (r > 0 && r >= a.nrhs) continue;
+        double w0, w1;
+        lds2(wS + (r * BN + c) * 8, w0, w1);
+        if (good[0]) sum[r] = fma(kv[0], w0, sum[r]);
+        if (good[1]) sum[r] = fma(kv[1], w1, sum[r]);
       }
     }
   } else {
@@ -937,9 +937,11 @@ constexpr bool uses_table(int kt) { return has_frame(kt) || kt == KS_LIST; }
 template <int NR>
 __device__ __forceinline__ void row_done(const TileArgs &a, int i, int parts)
 {
-  __threadfence();
-  if (atomicAdd(&a.row_n[i], 1) != parts - 1) return;
-  __threadfence();
+  if (parts > 1) {
+    __threadfence();
+    if (atomicAdd(&a.row_n[i], 1) != parts - 1) return;
+    __threadfence();
+  }
   const size_t q = (size_t)(a.umap ? a.umap[i] : i) * (NR > 1 ? a.nrhs : 1);
 #pragma unroll
   for (int r = 0; r < NR; r++) {
