@@ -89,6 +89,8 @@ Ctx::~Ctx()
   for (DevBuf *b : {&partial, &err, &dA, &dA2, &dB, &dB2, &dw, &du, &dhi, &dhj, &dwork, &rmaps, &serr, &stats})
     b->release();
   for (PinBuf *b : {&hA, &hA2, &hB, &hB2, &hw, &hu, &hhi, &hhj}) b->release();
+  // (memory still in use by enqueued calls outlives the pool's handle)
+  if (pool) cudaMemPoolDestroy(pool);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -111,6 +113,28 @@ Ctx *get_ctx()
   cudaMemset(c->err.p, 0, sizeof(int));
   tl_ctx = std::move(c);
   return tl_ctx.get();
+}
+
+constexpr unsigned long long POOL_KEEP = 512ull << 20;
+
+cudaError_t stream_alloc(Ctx *c, void **p, size_t bytes, cudaStream_t s)
+{
+  if (!c->pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = c->device;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    unsigned long long keep = POOL_KEEP;
+    if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return e;
+    }
+    c->pool = pool;
+  }
+  return cudaMallocFromPoolAsync(p, bytes, c->pool, s);
 }
 
 int effective_precision()
@@ -422,8 +446,8 @@ int enqueue_fused(Ctx *c, const ks_t *ker, int m, int n, int k,
   const size_t pbytes = p.partial_elems * sizeof(double) * (size_t)std::max(nrhs, 1);
   double *partial = nullptr;
   if (stream_ordered_alloc) {
-    cudaError_t e = cudaMallocAsync((void **)&partial, pbytes, s);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMallocAsync");
+    cudaError_t e = stream_alloc(c, (void **)&partial, pbytes, s);
+    if (e != cudaSuccess) return cuda_status(e, "workspace");
   } else {
     if (!c->partial.ensure(pbytes)) return GSKS_ERR_ALLOC;
     partial = (double *)c->partial.p;
@@ -478,7 +502,7 @@ int enqueue_rhs(Ctx *c, const ks_t *ker, int m, int n, int k, int nrhs, double *
   const size_t bytes = ((size_t)m + n) * sizeof(int);
   int *maps = nullptr;
   if (stream_ordered_alloc) {
-    const cudaError_t e = cudaMallocAsync((void **)&maps, bytes, s);
+    const cudaError_t e = stream_alloc(c, (void **)&maps, bytes, s);
     if (e != cudaSuccess) return cuda_status(e, "rhs maps");
   } else {
     if (!c->rmaps.ensure(bytes)) return GSKS_ERR_ALLOC;

@@ -42,6 +42,7 @@ struct Ctx {
   DevBuf dA, dA2, dB, dB2, dw, du, dhi, dhj, dwork;
   DevBuf rmaps;                // per-rhs u and w maps of the multi-rhs calls
   DevBuf serr;                 // synchronous calls: [0] device error flags, [1] sgsks map-check flag
+  cudaMemPool_t pool = nullptr;   // workspaces of the stream-ordered calls (stream_alloc)
   DevBuf stats;                // the last split-precision call: rechecked pairs (u64), rescued rows (int)
   int *cur_err = nullptr;      // the error word kernels write (nullptr: err, the asynchronous calls')
   int host_direct = -1;        // the GPU reads pageable host memory (the host calls' gather), -1: not asked yet
@@ -74,6 +75,12 @@ struct Staged {
 };
 
 Ctx *get_ctx();
+// Workspace of one asynchronous call on stream s, released by cudaFreeAsync on s.
+// It comes from the thread's own pool, which keeps up to POOL_KEEP bytes between
+// calls (the device's default pool gives its memory back at every
+// synchronisation: 200 us and more to map it again for the next call) and goes
+// with the thread's context.
+cudaError_t stream_alloc(Ctx *c, void **p, size_t bytes, cudaStream_t s);
 int set_status(int s, const char *where);
 int cuda_status(cudaError_t e, const char *where);
 void note_launches(int n);

@@ -1375,7 +1375,7 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   const size_t total = o_p + al((size_t)nrhs * nparts * ldp * 8);
   uint8_t *ws = nullptr;
   if (stream_ordered_alloc) {
-    const cudaError_t e = cudaMallocAsync((void **)&ws, total, s);
+    const cudaError_t e = stream_alloc(c, (void **)&ws, total, s);
     if (e != cudaSuccess) return cuda_status(e, "sliced workspace");
   } else {
     if (!c->dwork.ensure(total)) return GSKS_ERR_ALLOC;

@@ -2696,7 +2696,7 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
   const size_t total = o_rowc + (anch ? al((size_t)m * 8) : 0);
   uint8_t *ws = nullptr;
   if (stream_ordered_alloc) {
-    cudaError_t e = cudaMallocAsync((void **)&ws, total, s);
+    cudaError_t e = stream_alloc(c, (void **)&ws, total, s);
     if (e != cudaSuccess) return cuda_status(e, "split workspace");
   } else {
     if (!c->dwork.ensure(total)) return GSKS_ERR_ALLOC;
