@@ -177,6 +177,12 @@ __device__ __forceinline__ int pool_index(const int *map, int pos, int npool, in
   return p;
 }
 
+__device__ __forceinline__ int pool_clamp(const int *map, int pos, int npool)
+{
+  const int p = map ? map[pos] : pos;
+  return npool >= 0 && (uint32_t)p >= (uint32_t)npool ? 0 : p;
+}
+
 // Programmatic dependent launch: a kernel launched with launch_after may start
 // when every block of the one before it has called launch_dependents, and
 // calls wait_primary before it touches anything that one reads or writes.  It
@@ -224,28 +230,42 @@ __device__ __forceinline__ ScanPart scan_fold(ScanPart r)
 // of amap from a0) followed by a source list (n of bmap from b0), with the
 // bandwidth factors hi, hj of the variable-bandwidth kernel: the block's
 // threads take one coordinate of every (256 / k)-th point (a point at a time for
-// long rows).
+// long rows), U of them in flight.
+// (Map entries out of range read point 0, as in slice_kernel, which flags them: a
+// flag here would keep the loads from being issued together.)
+template <int U>
 __device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int m, int b0, int n, const double *hi,
                                                 const double *hj, int first, int step)
 {
   ScanPart r{0, ~0u, 0, 0};
   const int lanes = min(a.k, 256), per = 256 / lanes, c0 = threadIdx.x % lanes, sub = threadIdx.x / lanes;
   if (sub < per) {
-#pragma unroll 2
-    for (int i = first * per + sub; i < m + n; i += step * per) {
-      const bool A = i < m;
-      const int p = A ? pool_index(a.amap, a0 + i, a.nxa, a.err) : pool_index(a.bmap, b0 + i - m, a.nxb, a.err);
-      const double *x = (A ? a.XA : a.XB) + (size_t)p * a.k;
-      for (int c = c0; c < a.k; c += lanes)
-        r.maxabs = max(r.maxabs, (uint32_t)__double2hiint(x[c]) & 0x7fffffffu);
-      if (c0 == 0) {
-        uint32_t nn = (uint32_t)__double2hiint(A ? a.XA2[p] : a.XB2[p]);
-        if (hi) {            // bandwidth factors: within 2^-300 .. 2^300
-          const uint32_t h = (uint32_t)__double2hiint(A ? hi[p] : hj[p]);
-          if (h - (723u << 20) >= 600u << 20) nn = ~0u;
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+      const int cnt = side ? n : m, npool = side ? a.nxb : a.nxa;
+      const int *__restrict__ map = side ? a.bmap : a.amap;
+      const int at = side ? b0 : a0;
+      const double *__restrict__ X = side ? a.XB : a.XA, *__restrict__ X2 = side ? a.XB2 : a.XA2;
+      const double *__restrict__ h = side ? hj : hi;
+      for (int i0 = first * per + sub; i0 < cnt; i0 += U * step * per) {
+        uint32_t xh[U], nh[U];
+#pragma unroll
+        for (int e = 0; e < U; e++) {       // (past the end: the last point again)
+          const int p = pool_clamp(map, at + min(i0 + e * step * per, cnt - 1), npool);
+          xh[e] = (uint32_t)__double2hiint(X[(size_t)p * a.k + c0]) & 0x7fffffffu;
+          for (int c = c0 + lanes; c < a.k; c += lanes)
+            xh[e] = max(xh[e], (uint32_t)__double2hiint(X[(size_t)p * a.k + c]) & 0x7fffffffu);
+          nh[e] = (uint32_t)__double2hiint(X2[p]);
+          if (h) {            // bandwidth factors: within 2^-300 .. 2^300
+            if ((uint32_t)__double2hiint(h[p]) - (723u << 20) >= 600u << 20) nh[e] = ~0u;
+          }
         }
-        r.nmin = min(r.nmin, nn);
-        r.nmax = max(r.nmax, nn);
+#pragma unroll
+        for (int e = 0; e < U; e++) {
+          r.maxabs = max(r.maxabs, xh[e]);
+          r.nmin = min(r.nmin, nh[e]);
+          r.nmax = max(r.nmax, nh[e]);
+        }
       }
     }
   }
@@ -257,7 +277,7 @@ __device__ __forceinline__ ScanPart scan_points(const SliceArgs &a, int a0, int 
 __global__ void __launch_bounds__(256) scan_kernel(SliceArgs a, ScanPart *__restrict__ part)
 {
   launch_dependents();
-  const ScanPart r = scan_fold(scan_points(a, 0, a.m, 0, a.n, a.hi, a.hj, blockIdx.x, gridDim.x));
+  const ScanPart r = scan_fold(scan_points<4>(a, 0, a.m, 0, a.n, a.hi, a.hj, blockIdx.x, gridDim.x));
   if (threadIdx.x == 0) part[blockIdx.x] = r;
 }
 
@@ -274,7 +294,7 @@ __global__ void __launch_bounds__(256) list_scan_kernel(SliceArgs a, int ntask, 
   const TaskGeo G = tg[t];
   const KParams &kp = tp[t].kp;
   const bool vb = kp.type == KS_GAUSSIAN_VAR_BANDWIDTH;
-  const ScanPart r = scan_fold(scan_points(a, G.a0, G.m, G.b0, G.n, vb ? kp.hi : nullptr, kp.hj, 0, 1));
+  const ScanPart r = scan_fold(scan_points<8>(a, G.a0, G.m, G.b0, G.n, vb ? kp.hi : nullptr, kp.hj, 0, 1));
   if (threadIdx.x == 0) tp[t].cp = call_param(r, tp[t].cp, tp[t].kp.type, a.kpad);
 }
 
@@ -374,8 +394,8 @@ __device__ __forceinline__ void slice8(const double (&v)[8], int e, bool live, u
   }
 }
 
-// One block per 32 points: lane = point, warp = group of eight coordinates
-// (then every eighth group).  Reads 64 bytes a thread, writes 16-byte row
+// One block per 32 points: lane = point, each warp a group of eight coordinates
+// (then every eighth one; the list form's blocks have no more warps than groups).  Reads 64 bytes a thread, writes 16-byte row
 // segments, consecutive points side by side (512 contiguous bytes a warp).
 __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
 {
@@ -394,7 +414,7 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     // every block folds the scan's partials (at most one per thread) or, for
     // few points, scans them all itself
     ScanPart r{0, ~0u, 0, 0};
-    if (a.nscan == 0) r = scan_points(a, 0, a.m, 0, a.n, a.hi, a.hj, 0, 1);
+    if (a.nscan == 0) r = scan_points<2>(a, 0, a.m, 0, a.n, a.hi, a.hj, 0, 1);
     else if ((int)threadIdx.x < a.nscan) r = a.scan[threadIdx.x];
     r = scan_fold(r);
     if (threadIdx.x == 0) {
@@ -450,7 +470,8 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
 
   double v[8];
   uint32_t mh = 0;
-  for (int kg = wp; kg < kgs; kg += 8) {
+  const int nw = blockDim.x >> 5;
+  for (int kg = wp; kg < kgs; kg += nw) {
     load8(kg, v);
     if (!fixed) {
 #pragma unroll
@@ -464,7 +485,8 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     s_max[wp][lane] = mh;
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 8; q++) mh = max(mh, s_max[q][lane]);
+    for (int q = 0; q < 8; q++)
+      if (q < nw) mh = max(mh, s_max[q][lane]);
     if (mh) {
       const int fld = (int)(mh >> 20);
       e = fld - 1022;                     // |x_p| < 2^e
@@ -473,8 +495,8 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     }
   }
   uint8_t *base = side ? a.imgB + (size_t)tile * btile_bytes(a.kpad, a.nr) : a.imgA + (size_t)tile * op_bytes(BM, a.kpad);
-  const bool once = kgs <= 8;             // each thread's only group is still in registers
-  for (int kg = wp; kg < kgs; kg += 8) {
+  const bool once = kgs <= nw;             // each thread's only group is still in registers
+  for (int kg = wp; kg < kgs; kg += nw) {
     if (!once) load8(kg, v);
     if (fixed) {
 #pragma unroll
@@ -1564,7 +1586,7 @@ int sliced_list_run(const SlicedListPlan &Pl, Ctx *c, const double *XA, const do
   p.nta = Pl.n_ta;
   // (also clears the work counter)
   list_scan_kernel<<<Pl.any_frame ? Pl.ntask : 1, 256, 0, s>>>(p, Pl.ntask, (const TaskGeo *)(ws + Pl.o_tg), tp);
-  cudaError_t e = launch_after(slice_kernel, Pl.n_ta * (BM / 32) + Pl.n_tb * (BN / 32), 256, 0, s, p);
+  cudaError_t e = launch_after(slice_kernel, Pl.n_ta * (BM / 32) + Pl.n_tb * (BN / 32), 32 * std::min(8, Pl.kpad / 8), 0, s, p);
   TileArgs a{};
   a.k = Pl.k; a.kpad = Pl.kpad; a.nrhs = 1; a.ntm = 1;
   a.imgA = p.imgA; a.imgB = p.imgB;

@@ -304,13 +304,21 @@ __device__ __forceinline__ int pool_index(const int *map, int pos, int npool, in
   return p;
 }
 
+// The same without the flag, for passes that pack_kernel follows (it flags every
+// entry): an atomic in a loop keeps its loads from being issued together.
+__device__ __forceinline__ int pool_clamp(const int *map, int pos, int npool)
+{
+  const int p = map ? map[pos] : pos;
+  return npool >= 0 && (uint32_t)p >= (uint32_t)npool ? 0 : p;
+}
+
 // Per-dimension min / max over the gathered targets and sources.  Every thread
 // keeps one dimension (the grid-wide thread count is rounded down to a
 // multiple of k; at least k threads are launched) and folds its points in
 // registers; one shared and one global atomic per thread and bound.
 __global__ void bbox_kernel(int m, int n, int k, const double *__restrict__ XA, const int *__restrict__ amap,
                             int nxa, const double *__restrict__ XB, const int *__restrict__ bmap, int nxb,
-                            int *err, long long *bbox)
+                            long long *bbox)
 {
   extern __shared__ long long sb[];
   for (int p = threadIdx.x; p < k; p += blockDim.x) {
@@ -327,8 +335,8 @@ __global__ void bbox_kernel(int m, int n, int k, const double *__restrict__ XA, 
 #pragma unroll 4
     for (long long pt = tid / k; pt < (long long)m + n; pt += per) {
       double v;
-      if (pt < m) v = XA[(size_t)pool_index(amap, (int)pt, nxa, err) * k + p];
-      else v = XB[(size_t)pool_index(bmap, (int)(pt - m), nxb, err) * k + p];
+      if (pt < m) v = XA[(size_t)pool_clamp(amap, (int)pt, nxa) * k + p];
+      else v = XB[(size_t)pool_clamp(bmap, (int)(pt - m), nxb) * k + p];
       const long long key = dkey(v);
       lo = min(lo, key);
       hi = max(hi, key);
@@ -456,6 +464,15 @@ __global__ void params_kernel(int k, int kt, double scal, double cons, double po
 
 }
 
+// Threads of params_kernel: a power of two at least k (its fixed-order sums are
+// then the same as with more threads, whose terms are zero).
+static int params_threads(int k)
+{
+  int t = 32;
+  while (t < k && t < 1024) t *= 2;
+  return t;
+}
+
 // Per task of the list form, the per-dimension min and max (ordered keys)
 // over its targets (XA through a_idx) and sources (XB through b_idx):
 // tbox[t][0][p], tbox[t][1][p]; each task's box is also folded into the
@@ -464,7 +481,7 @@ __global__ void params_kernel(int k, int kt, double scal, double cons, double po
 __global__ void __launch_bounds__(256) list_box_kernel(int ntask, int k, const SplitTaskGeo *__restrict__ tg,
                                                        const double *__restrict__ XA, const int *__restrict__ a_idx,
                                                        int nxa, const double *__restrict__ XB,
-                                                       const int *__restrict__ b_idx, int nxb, int *err,
+                                                       const int *__restrict__ b_idx, int nxb,
                                                        long long *__restrict__ tbox, long long *__restrict__ bbox)
 {
   __shared__ long long slo[256], shi[256];
@@ -479,12 +496,23 @@ __global__ void __launch_bounds__(256) list_box_kernel(int ntask, int k, const S
     long long lo = 0x7FFFFFFFFFFFFFFFLL, hi = (long long)0x8000000000000000ULL;
     if (grp < sub) {
       const int p = p0 + c;
-      for (int q = grp; q < npts; q += sub) {
-        const double v = q < G.m ? XA[(size_t)pool_index(a_idx, G.a0 + q, nxa, err) * k + p]
-                                 : XB[(size_t)pool_index(b_idx, G.b0 + q - G.m, nxb, err) * k + p];
-        const long long key = dkey(v);
-        lo = min(lo, key);
-        hi = max(hi, key);
+      // (a loop per side, without branches: eight points' loads go out together,
+      // or the largest task's block takes a load's latency per point)
+#pragma unroll
+      for (int side = 0; side < 2; side++) {
+        const int cnt = side ? G.n : G.m, npool = side ? nxb : nxa;
+        const int *__restrict__ idx = side ? b_idx + G.b0 : a_idx + G.a0;
+        const double *__restrict__ X = (side ? XB : XA) + p;
+        for (int q0 = grp; q0 < cnt; q0 += 8 * sub) {
+          long long key[8];
+#pragma unroll
+          for (int e = 0; e < 8; e++) {     // (past the end: the last point again)
+            const int q = min(q0 + e * sub, cnt - 1);
+            key[e] = dkey(X[(size_t)pool_clamp(idx, q, npool) * k]);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; e++) { lo = min(lo, key[e]); hi = max(hi, key[e]); }
+        }
       }
     }
     slo[tid] = lo;
@@ -613,7 +641,7 @@ __global__ void pool_split(long long n, int k, const double *__restrict__ X, con
 // over equal strided groups of sources, the groups then added in order.
 // sh: blockDim.x doubles of shared memory.
 __device__ void block_source_sums(int j0, int j1, int k, const double *__restrict__ X,
-                                  const int *__restrict__ map, int npool, int *err,
+                                  const int *__restrict__ map, int npool,
                                   const double *__restrict__ w, const int *__restrict__ wmap, double inv_n,
                                   double *ysum, double *wsum, double *sh)
 {
@@ -625,8 +653,18 @@ __device__ void block_source_sums(int j0, int j1, int k, const double *__restric
     double s = 0.0;
     if (grp < sub) {
       const int p = p0 + c;
-      for (int j = j0 + grp; j < j1; j += sub)
-        s += p < k ? X[(size_t)pool_index(map, j, npool, err) * k + p] : w[wmap ? wmap[j] : j];
+      // eight terms' loads at a time, added in the order of one by one
+      for (int q0 = j0 + grp; q0 < j1; q0 += 8 * sub) {
+        double v[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+          const int j = min(q0 + e * sub, j1 - 1);
+          v[e] = p < k ? X[(size_t)pool_clamp(map, j, npool) * k + p] : w[wmap ? wmap[j] : j];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+          if (q0 + e * sub < j1) s += v[e];
+      }
     }
     sh[t] = s;
     __syncthreads();
@@ -655,7 +693,7 @@ constexpr int ANCHOR_WPER = 4096;   // weights per block of the weight sum
 // cpart[(sb * 2 + 0) * k + p]: sum of coordinate p over sample block sb;
 // cpart[(sb * 2 + 1) * k + p]: the sum of its squares.
 __global__ void __launch_bounds__(256) anchor_coords(int n, int k, const double *__restrict__ XB,
-                                                     const int *__restrict__ bmap, int nxb, int *err,
+                                                     const int *__restrict__ bmap, int nxb,
                                                      double *__restrict__ cpart)
 {
   __shared__ double sh[2][256];
@@ -668,7 +706,7 @@ __global__ void __launch_bounds__(256) anchor_coords(int n, int k, const double 
   if (p < k) {
 #pragma unroll 8
     for (int q = q0 + wp; q < q1; q += 8) {
-      const double y = XB[(size_t)pool_index(bmap, q * stride, nxb, err) * k + p];
+      const double y = XB[(size_t)pool_clamp(bmap, q * stride, nxb) * k + p];
       s += y;
       s2 = fma(y, y, s2);
     }
@@ -733,79 +771,136 @@ __global__ void anchor_final(int n, int k, int nwb, int nrhs, const double *__re
 // anchored, or empty, are skipped): ybar[t * k ..] and wsum[t].
 __global__ void list_anchor(int ntask, int k, const TaskParam *__restrict__ tp, const SplitTaskGeo *__restrict__ tg,
                             const double *__restrict__ XB, const int *__restrict__ b_idx, int nxb,
-                            const double *__restrict__ w, const int *__restrict__ w_idx, int *err,
+                            const double *__restrict__ w, const int *__restrict__ w_idx,
                             double *__restrict__ ybar, double *__restrict__ wsum)
 {
   extern __shared__ double sh_sum[];
   const int t = blockIdx.x;
   if (t >= ntask || !tp[t].anch || tg[t].n <= 0 || tg[t].m <= 0) return;
   const SplitTaskGeo G = tg[t];
-  block_source_sums(G.b0, G.b0 + G.n, k, XB, b_idx, nxb, err, w, w_idx, 1.0 / (double)G.n,
+  block_source_sums(G.b0, G.b0 + G.n, k, XB, b_idx, nxb, w, w_idx, 1.0 / (double)G.n,
                     ybar + (size_t)t * k, wsum + t, sh_sum);
 }
 
+// 1 / p of a power of two (normal, and so is its reciprocal).
+__device__ __forceinline__ double rcp_pow2(double p) { return __hiloint2double((2046 << 20) - __double2hiint(p), 0); }
+
+// Threads of a pack_kernel block: a warp per group of 8 coordinates, at most 8.
+static int pack_threads(int kpad) { return 32 * std::min(8, kpad / 8); }
+
+// One side of pack_kernel: the points, their map, and (list form) the tiles, tile t
+// packing positions tiles[t].x .. tiles[t].x + tiles[t].y - 1 of the CSR list
+// `map` for task tile_task[t].
+struct PackSide {
+  int npts, ntile;
+  const double *X; const int *map; int npool;
+  const double *hvec;
+  uint8_t *img;
+  const int2 *tiles; const int *tile_task;
+};
+struct PackArgs {
+  PackSide a, b;
+  int k, kpad, kt, nrhs;
+  const double *w; const int *wmap;
+  const double *centre;
+  const Params *P;
+  const TaskParam *tp;
+  const double *ybar, *ybsq;
+  double *rowc;
+  int *err;
+};
+
 // Tile images: per tile, NBLK slice blocks in the no-swizzle K-major core-matrix
 // layout (element (r, p) at (p/8)*rows*16 + r*16 + (p%8)*2 bytes), then the
-// point metadata.  One thread per point.
-// List form (tiles != nullptr): tile t packs positions tiles[t].x ..
-// tiles[t].x + tiles[t].y - 1 of the CSR list `map`, for task tile_task[t].
-__global__ void pack_kernel(int side, int npts, int k, int kpad, const double *__restrict__ X,
-                            const int *__restrict__ map, int npool, int *err, const double *__restrict__ w,
-                            const int *__restrict__ wmap, const double *__restrict__ hvec, int kt,
-                            const double *__restrict__ centre, const Params *__restrict__ P,
-                            uint8_t *__restrict__ img, const int2 *__restrict__ tiles,
-                            const int *__restrict__ tile_task, const TaskParam *__restrict__ tp,
-                            const double *__restrict__ ybar, double *__restrict__ rowc, int nrhs = 1,
-                            const double *__restrict__ ybsq = nullptr)
+// point metadata.  A block takes 32 points of either side: lane = point, each warp a
+// group of 8 coordinates (then every eighth one), so that a point's coordinates are sliced
+// side by side and 32 points' 16-byte segments are stored together; the norms'
+// integer sums are added over the warps (exactly), the metadata left to warp 0.
+// (One thread per point took 70 us a side for 65536 points at k = 64 and, in the
+// batched workload at k = 16, 1.9 ms of 4000 tasks' 7.9.)  Bound by the FP64
+// pipe: two instructions and a conversion per coordinate.
+__global__ void __launch_bounds__(256) pack_kernel(PackArgs g)
 {
+  __shared__ long long s_na[8][32], s_nb[8][32];
+  __shared__ int s_ni[8][32];
   // nrhs > 1 (sources of several right-hand sides): w holds nrhs interleaved
   // columns and the tiles carry RMAX weights per point (SrcMetaX)
-  const int tile = blockIdx.x, r = threadIdx.x;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  constexpr int PER = BM / 32;
+  const int side = (int)blockIdx.x >= g.a.ntile * PER;
+  const PackSide &S = side ? g.b : g.a;
+  const int blk = side ? blockIdx.x - g.a.ntile * PER : blockIdx.x;
+  const int tile = blk / PER, r = (blk - tile * PER) * 32 + lane;
+  const int k = g.k, kpad = g.kpad, nrhs = g.nrhs;
+  const Params *__restrict__ P = g.P;
+  int kt = g.kt;
+  const double *hvec = S.hvec;
   int pt = tile * BM + r;
-  bool valid = pt < npts;
+  bool valid = pt < S.npts;
   bool centred = P->centred != 0;
-  if (tiles) {
-    const int2 tl = tiles[tile];
-    const TaskParam &T = tp[tile_task[tile]];
+  const TaskParam *TT = nullptr;   // the list task
+  const double *cen = g.centre;    // the centre: the call's, or the task's own (centre + task k)
+  if (S.tiles) {
+    const int2 tl = S.tiles[tile];
+    const int task = S.tile_task[tile];
+    TT = g.tp + task;
     pt = tl.x + r;
     valid = r < tl.y;
-    centred = T.centred != 0;
-    kt = T.kp.type;
-    hvec = side == 0 ? T.kp.hi : T.kp.hj;
+    centred = TT->centred != 0;
+    kt = TT->kp.type;
+    hvec = side == 0 ? TT->kp.hi : TT->kp.hj;
+    cen += (size_t)task * k;
   }
-  const int pidx = valid ? pool_index(map, pt, npool, err) : 0;
-  const double *x = X + (size_t)pidx * k;
-  // the centre: the call's, or (list form) the task's own (centre + task k)
-  const double *cen = tiles ? centre + (size_t)tile_task[tile] * k : centre;
+  const int pidx = valid ? pool_index(S.map, pt, S.npool, g.err) : 0;
+  const double *x = S.X + (size_t)pidx * k;
   // coordinate -> slice units: the call's scale, or the list task's
-  const TaskParam *TT = tiles ? &tp[tile_task[tile]] : nullptr;
   const double sc = TT ? TT->sc : P->alpha * P->inv_sigma * 128.0;
-  const double sig2 = TT ? TT->sig2 : P->sigma * P->sigma;
-  const bool gfast = TT ? TT->gfast != 0 : P->gfast != 0;
-  uint8_t *base = img + (size_t)tile * tile_bytes(BM, kpad, side == 1 ? smeta_pt(nrhs > 1 ? RMAX : 1) : sizeof(PtMeta));
+  uint8_t *base = S.img + (size_t)tile * tile_bytes(BM, kpad, side == 1 ? smeta_pt(nrhs > 1 ? RMAX : 1) : sizeof(PtMeta));
   const size_t bb = blk_bytes(BM, kpad);
+  const bool wide = (k & 1) == 0 && ((uintptr_t)S.X & 15) == 0;   // 16-byte loads
   // The norm of the represented point restricted to the products the tensor
   // cores form (a1a1 + 2a1a2 + a2a2 + 2a1a3), so that the assembled d2 of
   // identical points is 0 up to the FP32 accumulations.  Every term is an
   // integer multiple of 2^-48 (halves are multiples of 2^-24): summed exactly
-  // in integers, a1a1 at scale 1, 2a1(a2 + a3) at 2^24, a2a2 at 2^48.  FP64
-  // instructions issue slowly here; the slicing uses six per coordinate.
+  // in integers, a1a1 at scale 1, 2a1(a2 + a3) at 2^24, a2a2 at 2^48.
   int n_i = 0;
   long long n_a = 0, n_b = 0;
-  for (int kg = 0; kg < kpad / 8; kg++) {
+  const int nw = blockDim.x >> 5;
+  for (int kg = wp; kg < kpad / 8; kg += nw) {
+    double v[8];
+    const int c0 = kg * 8;
+    if (valid && wide && c0 + 8 <= k) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const double2 d = __ldg((const double2 *)(x + c0) + q);
+        v[2 * q] = d.x; v[2 * q + 1] = d.y;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = (valid && c0 + q < k) ? __ldg(x + c0 + q) : 0.0;
+    }
     __align__(16) __half s1[8], s2[8], s3[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) {
-      const int p = kg * 8 + e;
+      const int p = c0 + e;
       float a1 = 0.0f;
       __half h2 = __float2half_rn(0.0f), h3 = __float2half_rn(0.0f);
       if (valid && p < k) {
-        const double t = (centred ? x[p] - cen[p] : x[p]) * sc;   // the difference is exact near the centre
-        a1 = rintf((float)t);                          // |a1| <= 128
-        const float r1 = (float)(t - (double)a1);      // |r1| <= 1/2 (+ a rounding at ties)
+        const double t = (centred ? v[e] - __ldg(cen + p) : v[e]) * sc;   // the difference is exact near the centre
+        const float f = (float)t;
+        a1 = rintf(f);                                 // |a1| <= 128
+        // r1 = t - a1 rounded to FP32, |r1| <= 1/2 (+ a rounding at ties): below
+        // 1/2 f itself, else from t in units of 2^-53 as an integer (an FP64
+        // conversion and subtraction would be two more of the scarce instructions)
+        const long long tb = __double_as_longlong(t);
+        const int sh = (int)(tb >> 52 & 0x7ff) - 1022;                    // 0 .. 8 where |t| >= 1/2
+        long long T = ((tb & 0xfffffffffffffll) | 0x10000000000000ll) << (sh & 15);
+        T = tb < 0 ? -T : T;
+        const int ia = (int)a1;
+        const long long R = T - ((long long)ia << 53);
+        const float r1 = sh < 0 ? f : __ll2float_rn(R) * 0x1p-53f;
         h2 = __float2half_rn(r1);
         h3 = __float2half_rn(r1 - __half2float(h2));   // the difference is exact in FP32
-        const int ia = (int)a1;
         const int F2 = (int)(__half2float(h2) * 16777216.0f), F3 = (int)(__half2float(h3) * 16777216.0f);
         n_i += ia * ia;
         n_a += (long long)(2 * ia) * (F2 + F3);
@@ -819,30 +914,39 @@ __global__ void pack_kernel(int side, int npts, int k, int kpad, const double *_
     *(uint4 *)(base + img_off(1, kg, r, kpad)) = *(const uint4 *)s2;
     *(uint4 *)(base + img_off(2, kg, r, kpad)) = *(const uint4 *)s3;
   }
+  s_ni[wp][lane] = n_i;
+  s_na[wp][lane] = n_a;
+  s_nb[wp][lane] = n_b;
+  __syncthreads();
+  if (wp != 0) return;
+  for (int q = 1; q < nw; q++) { n_i += s_ni[q][lane]; n_a += s_na[q][lane]; n_b += s_nb[q][lane]; }
+  const double sig2 = TT ? TT->sig2 : P->sigma * P->sigma;
+  const bool gfast = TT ? TT->gfast != 0 : P->gfast != 0;
   const double nrm = ((double)n_i + (double)n_a * 0x1p-24 + (double)n_b * 0x1p-48) * (1.0 / 16384.0);
-  (void)bb;
   // The norm in units of the accumulators: nu = |x''|^2 / g with
   // g = 2 sigma^2 2^-14, so that d2 = g (nu_i + nu_j - H - L).  nu is split on
   // the grid q / g (a power of two): its high parts and H add exactly.
-  const double g = TT ? TT->g : P->g;
-  const double nu = nrm * sig2 / g;
-  const double qg = (TT ? TT->q : P->q) / g;
-  const double nh = rint(nu / qg) * qg;
+  const double gu = TT ? TT->g : P->g;
+  // (q, g and their ratio are powers of two: exact reciprocals, no divisions)
+  const double rg = rcp_pow2(gu);
+  const double nu = nrm * sig2 * rg;
+  const double qg = (TT ? TT->q : P->q) * rg;
+  const double nh = rint(nu * rcp_pow2(qg)) * qg;
   const double nl = nu - nh;
   PtMeta mt;
   mt.n_hi = (float)nh;
   mt.n_lo = (float)nl;
   mt.w = 0.0f;
   mt.h = 0.0f;
-  const size_t wi = valid ? (size_t)(wmap ? wmap[pt] : pt) * (nrhs > 1 ? nrhs : 1) : 0;   // weight column 0
+  const size_t wi = valid ? (size_t)(g.wmap ? g.wmap[pt] : pt) * (nrhs > 1 ? nrhs : 1) : 0;   // weight column 0
   double wf = 1.0;                 // the Gaussian fast path's source factor
-  if (side == 1 && valid) mt.w = (float)w[wi];
+  if (side == 1 && valid) mt.w = (float)g.w[wi];
   if (gfast) {
     // Gaussian: 2^-(g nl) is a per-point factor; fold it into w for sources
     // and into a row factor for targets (applied to the row sum)
-    const double f = exp2(-g * nl);
+    const double f = exp2(-gu * nl);
     mt.n_lo = 0.0f;
-    if (side == 1) { mt.w = valid ? (float)(w[wi] * f) : 0.0f; wf = f; }
+    if (side == 1) { mt.w = valid ? (float)(g.w[wi] * f) : 0.0f; wf = f; }
     else mt.h = (float)f;
   }
   mt.pos = valid ? pt : -1;
@@ -872,8 +976,8 @@ __global__ void pack_kernel(int side, int npts, int k, int kpad, const double *_
       if (valid) {
         double d0 = 0.0;
         for (int p = 0; p < k; p++) {
-          const double dx = x[p] - ybar[p];
-          d0 = fma(dx, dx, d0) + (ybsq[p] - ybar[p] * ybar[p]);
+          const double dx = x[p] - g.ybar[p];
+          d0 = fma(dx, dx, d0) + (g.ybsq[p] - g.ybar[p] * g.ybar[p]);
         }
         const double c = 1.0 - d0;
         double K0;
@@ -883,16 +987,16 @@ __global__ void pack_kernel(int side, int npts, int k, int kpad, const double *_
         mt.w = (float)d0;
         mt.h = (float)K0;
         mt.pad[0] = __float_as_int((float)c);
-        rowc[pt] = K0;
+        g.rowc[pt] = K0;
       }
     } else {
     mt.n_hi = mt.n_lo = mt.w = mt.h = 0.0f;
     if (valid) {
-      const double *yb = ybar + (TT ? (size_t)tile_task[tile] * k : 0);
+      const double *yb = g.ybar + (TT ? (size_t)S.tile_task[tile] * k : 0);
       double A = 0.0;
       for (int p = 0; p < k; p++) A = fma(x[p], yb[p], A);
-      const double G = 0.5 * g;
-      const double H0 = fmin(fmax(rint(A / G), -0x1p24), 0x1p24);
+      const double G = 0.5 * gu;
+      const double H0 = fmin(fmax(rint(A * rcp_pow2(G)), -0x1p24), 0x1p24);
       const double scal = TT ? TT->kp.scal : P->pscal, cons = TT ? TT->kp.cons : P->pcons;
       const int pw = TT ? TT->kp.pint : P->pw;
       const double v0 = fma(scal * G, H0, cons);
@@ -906,7 +1010,7 @@ __global__ void pack_kernel(int side, int npts, int k, int kpad, const double *_
       mt.n_lo = (float)c1;
       mt.w = (float)c2;
       mt.h = (float)c3;
-      rowc[pt] = vp;
+      g.rowc[pt] = vp;
     }
     }
   }
@@ -922,7 +1026,7 @@ __global__ void pack_kernel(int side, int npts, int k, int kpad, const double *_
   if (nrhs > 1) {
     SrcMetaX *sx = (SrcMetaX *)sm;
     for (int c = 1; c < RMAX; c++) {
-      const float wc = (valid && c < nrhs) ? (float)(w[wi + c] * wf) : 0.0f;
+      const float wc = (valid && c < nrhs) ? (float)(g.w[wi + c] * wf) : 0.0f;
       sx->wx[c - 1][r] = wc;
       wa += fabsf(wc);
     }
@@ -2715,23 +2819,25 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
     const long long tot = (long long)(m + n) * k;
     const int blocks = (int)std::max<long long>((k + 255) / 256,
                                                 std::min<long long>(8LL * sms, std::max<long long>(1, (tot + 255) / 256)));
-    bbox_kernel<<<blocks, 256, 2 * k * sizeof(long long), s>>>(m, n, k, XA, amap, nxa, XB, bmap, nxb,
-                                                               err_word(c), bbox);
+    bbox_kernel<<<blocks, 256, 2 * k * sizeof(long long), s>>>(m, n, k, XA, amap, nxa, XB, bmap, nxb, bbox);
   }
-  params_kernel<<<1, 1024, 0, s>>>(k, ker->type, ker->scal, ker->cons, ker->powe, tau, bbox, centre, P);
+  params_kernel<<<1, params_threads(k), 0, s>>>(k, ker->type, ker->scal, ker->cons, ker->powe, tau, bbox, centre, P);
   double *ybar = anch ? (double *)(ws + o_anc) : nullptr;
   double *ybsq = anch ? ybar + k + RMAX + (size_t)nwb * nrhs : nullptr;   // after the weight-sum partials
   double *rowc = anch ? (double *)(ws + o_rowc) : nullptr;
   if (anch) {
     double *wpart = ybar + k + RMAX, *cpart = ybsq + k;
-    anchor_coords<<<dim3((k + 31) / 32, ANCHOR_SB), 256, 0, s>>>(n, k, XB, bmap, nxb, err_word(c), cpart);
+    anchor_coords<<<dim3((k + 31) / 32, ANCHOR_SB), 256, 0, s>>>(n, k, XB, bmap, nxb, cpart);
     anchor_weights<<<nwb, 256, 0, s>>>(n, w, wmap, nrhs, wpart);
     anchor_final<<<1, 256, 0, s>>>(n, k, nwb, nrhs, cpart, wpart, ybar, ybsq, ybar + k);
   }
-  pack_kernel<<<ntm, BM, 0, s>>>(0, m, k, kpad, XA, amap, nxa, err_word(c), nullptr, nullptr, hi, ker->type,
-                                 centre, P, ws + o_a, nullptr, nullptr, nullptr, ybar, rowc, 1, ybsq);
-  pack_kernel<<<ntn, BN, 0, s>>>(1, n, k, kpad, XB, bmap, nxb, err_word(c), w, wmap, hj, ker->type, centre,
-                                 P, ws + o_b, nullptr, nullptr, nullptr, nullptr, nullptr, nrhs);
+  PackArgs pk{};
+  pk.a.npts = m; pk.a.ntile = ntm; pk.a.X = XA; pk.a.map = amap; pk.a.npool = nxa; pk.a.hvec = hi; pk.a.img = ws + o_a;
+  pk.b.npts = n; pk.b.ntile = ntn; pk.b.X = XB; pk.b.map = bmap; pk.b.npool = nxb; pk.b.hvec = hj; pk.b.img = ws + o_b;
+  pk.k = k; pk.kpad = kpad; pk.kt = ker->type; pk.nrhs = nrhs;
+  pk.w = w; pk.wmap = wmap; pk.centre = centre; pk.P = P;
+  pk.ybar = ybar; pk.ybsq = ybsq; pk.rowc = rowc; pk.err = err_word(c);
+  pack_kernel<<<(ntm + ntn) * (BM / 32), pack_threads(kpad), 0, s>>>(pk);
 
   TileArgs a{};
   a.m = m; a.n = n; a.k = k; a.kpad = kpad; a.kt = ker->type;
@@ -2790,7 +2896,7 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
     e = launch_rescue(a, std::max(1, std::min(2 * sms, (m + 7) / 8)), rlist, rcount, u, umap, s, NRK);
   if (stream_ordered_alloc) cudaFreeAsync(ws, s);
   if (e != cudaSuccess) return cuda_status(e, "split launch");
-  note_launches((defer ? 8 : 7) + ff_launches + (anch ? 3 : 0));
+  note_launches((defer ? 7 : 6) + ff_launches + (anch ? 3 : 0));
   return GSKS_OK;
 }
 
@@ -3051,21 +3157,24 @@ int split_list_run(const SplitListPlan &Pl, Ctx *c, const double *XA, const int 
   double *tcen = (double *)(ws + Pl.o_tcen);
   bbox_init<<<1, 256, 0, s>>>(k, bbox);
   // every task's box (its targets and sources), folded into the global box
-  list_box_kernel<<<ntask, 256, 0, s>>>(ntask, k, tg, XA, a_idx, nxa, XB, b_idx, nxb, err, tbox, bbox);
-  params_kernel<<<1, 1024, 0, s>>>(k, KS_LIST, 0.0, 0.0, 0.0, tau, bbox, centre, P);
+  list_box_kernel<<<ntask, 256, 0, s>>>(ntask, k, tg, XA, a_idx, nxa, XB, b_idx, nxb, tbox, bbox);
+  params_kernel<<<1, params_threads(k), 0, s>>>(k, KS_LIST, 0.0, 0.0, 0.0, tau, bbox, centre, P);
   task_params_kernel<<<(ntask + 127) / 128, 128, 0, s>>>(ntask, (const KParams *)(ws + Pl.o_kps), P, tau, tp, tbox,
                                                           tcen);
   double *ybar = Pl.any_anch ? (double *)(ws + Pl.o_ybar) : nullptr;
   double *wsum = Pl.any_anch ? (double *)(ws + Pl.o_wsum) : nullptr;
   double *rowc = Pl.any_anch ? (double *)(ws + Pl.o_rowc) : nullptr;
   if (Pl.any_anch)
-    list_anchor<<<ntask, 256, 256 * sizeof(double), s>>>(ntask, k, tp, tg, XB, b_idx, nxb, w, w_idx, err, ybar, wsum);
-  pack_kernel<<<Pl.n_ta, BM, 0, s>>>(0, 0, k, kpad, XA, a_idx, nxa, err, nullptr, nullptr, nullptr, KS_LIST,
-                                     tcen, P, ws + Pl.o_a, (const int2 *)(ws + Pl.o_ta),
-                                     (const int *)(ws + Pl.o_tat), tp, ybar, rowc);
-  pack_kernel<<<Pl.n_tb, BN, 0, s>>>(1, 0, k, kpad, XB, b_idx, nxb, err, w, w_idx, nullptr, KS_LIST,
-                                     tcen, P, ws + Pl.o_b, (const int2 *)(ws + Pl.o_tb),
-                                     (const int *)(ws + Pl.o_tbt), tp, nullptr, nullptr);
+    list_anchor<<<ntask, 256, 256 * sizeof(double), s>>>(ntask, k, tp, tg, XB, b_idx, nxb, w, w_idx, ybar, wsum);
+  PackArgs pk{};
+  pk.a.ntile = Pl.n_ta; pk.a.X = XA; pk.a.map = a_idx; pk.a.npool = nxa; pk.a.img = ws + Pl.o_a;
+  pk.a.tiles = (const int2 *)(ws + Pl.o_ta); pk.a.tile_task = (const int *)(ws + Pl.o_tat);
+  pk.b.ntile = Pl.n_tb; pk.b.X = XB; pk.b.map = b_idx; pk.b.npool = nxb; pk.b.img = ws + Pl.o_b;
+  pk.b.tiles = (const int2 *)(ws + Pl.o_tb); pk.b.tile_task = (const int *)(ws + Pl.o_tbt);
+  pk.k = k; pk.kpad = kpad; pk.kt = KS_LIST; pk.nrhs = 1;
+  pk.w = w; pk.wmap = w_idx; pk.centre = tcen; pk.P = P; pk.tp = tp;
+  pk.ybar = ybar; pk.rowc = rowc; pk.err = err;
+  pack_kernel<<<(Pl.n_ta + Pl.n_tb) * (BM / 32), pack_threads(kpad), 0, s>>>(pk);
   float2 *xaf = (float2 *)(ws + Pl.o_xaf), *xbf = Pl.same_pool ? xaf : (float2 *)(ws + Pl.o_xbf);
   {
     const long long na_c = (long long)nxa * k, nb_c = (long long)nxb * k;
@@ -3107,7 +3216,7 @@ int split_list_run(const SplitListPlan &Pl, Ctx *c, const double *XA, const int 
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) return cuda_status(e, "split list launch");
-  *launches += (Pl.same_pool ? 10 : 11) + (Pl.any_anch ? 2 : 0);
+  *launches += (Pl.same_pool ? 9 : 10) + (Pl.any_anch ? 2 : 0);
   return GSKS_OK;
 }
 
