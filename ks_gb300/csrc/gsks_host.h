@@ -122,6 +122,7 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k,
 struct SlicedListPlan {
   int ntask = 0, k = 0, kpad = 0, n_ta = 0, n_tb = 0, n_items = 0;
   bool any_frame = false;
+  int first[9] = {};           // the items of kernel type t: first[t] .. first[t + 1]
   DevBuf ws;
   size_t o_next = 0, o_ta = 0, o_tat = 0, o_tb = 0, o_tbt = 0, o_items = 0, o_tg = 0, o_tp = 0;
   size_t o_aa = 0, o_hi = 0, o_e = 0, o_a = 0, o_b = 0;

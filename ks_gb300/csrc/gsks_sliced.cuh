@@ -240,5 +240,40 @@ __device__ __forceinline__ double exp2_neg_scaled(uint64_t D, int F, uint64_t Mi
 }
 __device__ __forceinline__ ExpFrame exp_frame52(uint32_t tab) { return ExpFrame{9, 511u, 5814540u, tab}; }
 
+// (double)w: the conversion instruction issues to the FP64 pipe (2 per SM cycle),
+// these about a dozen integer ones take a third of its time.  Rounds to nearest,
+// ties away.
+__device__ __forceinline__ double to_double(long long w)
+{
+  const uint64_t a = (uint64_t)(w < 0 ? -w : w);
+  const int lz = __clzll((long long)a);
+  const uint64_t m = ((a << (lz & 63)) >> 1) + 512u;        // [2^62, 2^63] + half of 2^-52
+  const uint32_t hi = (uint32_t)(m >> 42) + ((1085u - (uint32_t)lz) << 20);
+  const uint32_t sg = (uint32_t)(w >> 32) & 0x80000000u;
+  return a ? __hiloint2double((int)(hi + sg), (int)(uint32_t)(m >> 10)) : 0.0;
+}
+
+// v^p, p = 2, 3 or 4, by 64-bit products of mantissas (an FP64 product issues at 2
+// per SM cycle; these three take about 14 to 20 integer instructions), to about
+// half a unit more than correct rounding.  ok: v^p lies well inside the normal
+// range (else the value does not hold).
+template <int P>
+__device__ __forceinline__ double pow_int(double v, bool &ok)
+{
+  const uint64_t b = (uint64_t)__double_as_longlong(v);
+  const int e = (int)(b >> 52 & 0x7ff) - 1023;
+  ok = (uint32_t)(e + 200) < 400u;
+  const uint64_t m = (b | 0x10000000000000ull) << 11;       // [1, 2) 2^63
+  uint64_t q = mulhi64(m, m);                               // [1, 4) 2^62
+  int up = 1;                                               // q = value 2^(63 - up)
+  if (P == 3) { q = mulhi64(q, m); up = 2; }
+  if (P == 4) { q = mulhi64(q, q); up = 3; }
+  const int lz = __clz((int)(q >> 32));                     // 0 .. up
+  const uint64_t r = ((q << lz) >> 1) + 512u;
+  const uint32_t hi = (uint32_t)(r >> 42) + (uint32_t)(P * e + up - lz + 1022) * (1u << 20);
+  const uint32_t sg = P == 3 ? (uint32_t)(b >> 32) & 0x80000000u : 0u;
+  return __hiloint2double((int)(hi + sg), (int)(uint32_t)(r >> 10));
+}
+
 }  // namespace sliced
 }  // namespace gsks
