@@ -182,29 +182,6 @@ __device__ __forceinline__ int pool_clamp(const int *map, int pos, int npool)
   return npool >= 0 && (uint32_t)p >= (uint32_t)npool ? 0 : p;
 }
 
-// Programmatic dependent launch: a kernel launched with launch_after may start
-// when every block of the one before it has called launch_dependents, and
-// calls wait_primary before it touches anything that one reads or writes.  It
-// overlaps launch and set-up (tensor memory, barriers, the table) with the
-// preparation: calls of a few tens of microseconds gain.
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_primary() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <typename... A>
-cudaError_t launch_after(void (*kernel)(A...), int grid, int block, size_t smem, cudaStream_t s, A... args)
-{
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3(grid);
-  c.blockDim = dim3(block);
-  c.dynamicSmemBytes = smem;
-  c.stream = s;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, args...);
-}
-
 // ---------------------------------------------------------------------------
 // A block's fold of its threads' scan values (256 threads, every thread calls;
 // the result in every thread).

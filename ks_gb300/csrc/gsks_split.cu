@@ -287,8 +287,16 @@ __device__ __forceinline__ double dval(long long k)
   return __longlong_as_double(k >= 0 ? k : k ^ 0x7FFFFFFFFFFFFFFFLL);
 }
 
-__global__ void bbox_init(int k, long long *bbox)
+// The bounds to be folded and, in a single call, the words that its kernels count in.
+__global__ void bbox_init(int k, long long *bbox, int *next_item, int *rcount, unsigned long long *stats)
 {
+  launch_dependents();
+  if (threadIdx.x == 0 && next_item) {
+    *next_item = 0;
+    *rcount = 0;
+    stats[0] = 0;
+    stats[1] = 0;
+  }
   for (int p = threadIdx.x + blockIdx.x * blockDim.x; p < k; p += blockDim.x * gridDim.x) {
     bbox[p] = 0x7FFFFFFFFFFFFFFFLL;
     bbox[k + p] = (long long)0x8000000000000000ULL;
@@ -316,9 +324,9 @@ __device__ __forceinline__ int pool_clamp(const int *map, int pos, int npool)
 // keeps one dimension (the grid-wide thread count is rounded down to a
 // multiple of k; at least k threads are launched) and folds its points in
 // registers; one shared and one global atomic per thread and bound.
-__global__ void bbox_kernel(int m, int n, int k, const double *__restrict__ XA, const int *__restrict__ amap,
-                            int nxa, const double *__restrict__ XB, const int *__restrict__ bmap, int nxb,
-                            long long *bbox)
+__device__ __forceinline__ void box_block(int blk, int nblk, int m, int n, int k, const double *__restrict__ XA,
+                                          const int *__restrict__ amap, int nxa, const double *__restrict__ XB,
+                                          const int *__restrict__ bmap, int nxb, long long *bbox)
 {
   extern __shared__ long long sb[];
   for (int p = threadIdx.x; p < k; p += blockDim.x) {
@@ -326,8 +334,8 @@ __global__ void bbox_kernel(int m, int n, int k, const double *__restrict__ XA, 
     sb[k + p] = (long long)0x8000000000000000ULL;
   }
   __syncthreads();
-  const long long nthr = (long long)blockDim.x * gridDim.x;
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long nthr = (long long)blockDim.x * nblk;
+  const long long tid = (long long)blk * blockDim.x + threadIdx.x;
   const long long per = nthr / k;                      // points advanced per step
   if (tid < per * k) {
     const int p = (int)(tid % k);
@@ -345,10 +353,141 @@ __global__ void bbox_kernel(int m, int n, int k, const double *__restrict__ XA, 
     atomicMax(&sb[k + p], hi);
   }
   __syncthreads();
+  wait_primary();   // the points are the caller's: only the bounds wait for bbox_init
   for (int p = threadIdx.x; p < k; p += blockDim.x) {
     atomicMin(&bbox[p], sb[p]);
     atomicMax(&bbox[k + p], sb[k + p]);
   }
+}
+
+// Anchor point of a single call's polynomial, tanh and compact / multiquadratic
+// kernels (the sources' mean and mean squares per coordinate) and the sum of
+// all weights.  Any point inside the sources' hull keeps each row's anchor
+// value within the range of that row's values, so the mean of a strided
+// sample of at most ANCHOR_SAMPLE sources serves: anchor_coords blocks (cb,
+// sb) take 32 coordinates of ANCHOR_SB-th of the sample each.  The weight sum
+// covers every source (anchor_weights: contiguous ranges, fixed-order tree).
+// anchor_final adds the partials in order.  All of it deterministic.  None of
+// it needs the bounding box: survey_kernel's blocks do both, and the two folds
+// are two blocks of params_kernel.
+constexpr int ANCHOR_SAMPLE = 2048;
+constexpr int ANCHOR_SB = 16;       // sample blocks of anchor_coords
+constexpr int ANCHOR_WPER = 4096;   // weights per block of the weight sum
+
+// cpart[(sb * 2 + 0) * k + p]: sum of coordinate p over sample block sb;
+// cpart[(sb * 2 + 1) * k + p]: the sum of its squares.
+__device__ __forceinline__ void anchor_coords(int cb, int sb, int n, int k, const double *__restrict__ XB,
+                                              const int *__restrict__ bmap, int nxb, double *__restrict__ cpart)
+{
+  __shared__ double sh[2][256];
+  const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+  const int S = min(n, ANCHOR_SAMPLE), stride = n / S;
+  const int per = (S + ANCHOR_SB - 1) / ANCHOR_SB;
+  const int q0 = sb * per, q1 = min(S, q0 + per);
+  const int p = cb * 32 + lane;
+  double s = 0.0, s2 = 0.0;
+  if (p < k) {
+#pragma unroll 16
+    for (int q = q0 + wp; q < q1; q += 8) {
+      const double y = XB[(size_t)pool_clamp(bmap, q * stride, nxb) * k + p];
+      s += y;
+      s2 = fma(y, y, s2);
+    }
+  }
+  sh[0][t] = s;
+  sh[1][t] = s2;
+  __syncthreads();
+  if (wp == 0 && p < k) {
+    double r = 0.0, r2 = 0.0;
+    for (int q = 0; q < 8; q++) { r += sh[0][q * 32 + lane]; r2 += sh[1][q * 32 + lane]; }
+    cpart[((size_t)sb * 2 + 0) * k + p] = r;
+    cpart[((size_t)sb * 2 + 1) * k + p] = r2;
+  }
+}
+
+// wpart[b * nrhs + r]: the sum of weight column r over sources b ANCHOR_WPER ..
+__device__ __forceinline__ void anchor_weights(int b, int n, const double *__restrict__ w,
+                                               const int *__restrict__ wmap, int nrhs, double *__restrict__ wpart)
+{
+  __shared__ double sh[256];
+  const int t = threadIdx.x;
+  const int j0 = b * ANCHOR_WPER, j1 = min(n, j0 + ANCHOR_WPER);
+  for (int r = 0; r < nrhs; r++) {
+    double s = 0.0;
+    #pragma unroll 16
+    for (int j = j0 + t; j < j1; j += 256) s += w[(size_t)(wmap ? wmap[j] : j) * nrhs + r];
+    sh[t] = s;
+    __syncthreads();
+    for (int h = 128; h > 0; h >>= 1) {
+      if (t < h) sh[t] += sh[t + h];
+      __syncthreads();
+    }
+    if (t == 0) wpart[(size_t)b * nrhs + r] = sh[0];
+    __syncthreads();
+  }
+}
+
+// ybar[p], ybsq[p]: the sample's mean and mean square of coordinate p;
+// wsum[r]: the sum of weight column r.
+struct AnchorSums {
+  int n, nwb, nrhs;
+  const double *cpart, *wpart;
+  double *ybar, *ybsq, *wsum;
+};
+__device__ __forceinline__ void anchor_final(const AnchorSums &a, int k)
+{
+  const double inv = 1.0 / (double)min(a.n, ANCHOR_SAMPLE);
+  for (int p = threadIdx.x; p < k; p += blockDim.x) {
+    double s = 0.0, q = 0.0;
+#pragma unroll
+    for (int sb = 0; sb < ANCHOR_SB; sb++) {
+      s += a.cpart[((size_t)sb * 2 + 0) * k + p];
+      q += a.cpart[((size_t)sb * 2 + 1) * k + p];
+    }
+    a.ybar[p] = s * inv;
+    a.ybsq[p] = q * inv;
+  }
+  for (int r = threadIdx.x; r < a.nrhs; r += blockDim.x) {
+    double s = 0.0;
+    for (int b = 0; b < a.nwb; b++) s += a.wpart[(size_t)b * a.nrhs + r];
+    a.wsum[r] = s;
+  }
+}
+
+// A single call's passes over its points that nothing comes before: blocks of
+// the bounding box, then (anchored kernels) of the anchor's coordinates, then
+// of the weight sum.  As three launches of 6, 11 and 5 us one after the other
+// they were a third of a call of 3000 x 2000 points.
+struct SurveyArgs {
+  int m, n, k, nbox, ncoord;   // blocks of the first two kinds
+  const double *XA, *XB; const int *amap, *bmap; int nxa, nxb;
+  const double *w; const int *wmap; int nrhs;
+  long long *bbox;
+  double *cpart, *wpart;
+};
+__global__ void __launch_bounds__(256) survey_kernel(SurveyArgs a)
+{
+  launch_dependents();
+  const int b = blockIdx.x;
+  if (b < a.nbox) {
+    box_block(b, a.nbox, a.m, a.n, a.k, a.XA, a.amap, a.nxa, a.XB, a.bmap, a.nxb, a.bbox);
+    return;
+  }
+  if (b < a.nbox + a.ncoord)
+    anchor_coords((b - a.nbox) / ANCHOR_SB, (b - a.nbox) % ANCHOR_SB, a.n, a.k, a.XB, a.bmap, a.nxb, a.cpart);
+  else
+    anchor_weights(b - a.nbox - a.ncoord, a.n, a.w, a.wmap, a.nrhs, a.wpart);
+  wait_primary();   // (so that this grid's end is bbox_init's too)
+}
+
+// The smallest power of two at or above x > 0, from its bits (its logarithm
+// and the power back are some 60 dependent FP64 instructions).
+__device__ __forceinline__ double pow2_above(double x)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long e = b >> 52, f = b & 0xfffffffffffffULL;
+  if (e == 0 || e >= 0x7ff) return exp2(ceil(log2(x)));   // subnormal, infinite, not a number
+  return __longlong_as_double((long long)((e + (f != 0)) << 52));
 }
 
 __device__ LapParam lap_param(double scal, double powe)
@@ -372,10 +511,14 @@ __device__ LapParam lap_param(double scal, double powe)
 // kt = KS_LIST: the list form, whose tasks mix centred (distance) and
 // uncentred (inner-product) kernels: the centre is the box's, the scale covers
 // the uncentred coordinates too, and the thresholds are set per task later.
+// A second block, if there is one, folds the anchor's partial sums.
 __global__ void params_kernel(int k, int kt, double scal, double cons, double powe, float tau, const long long *bbox,
-                              double *centre, Params *P)
+                              double *centre, Params *P, AnchorSums an)
 {
   __shared__ double s_sq[1024], s_mx[1024], s_sqc[1024], s_mxc[1024];
+  launch_dependents();
+  wait_primary();
+  if (blockIdx.x == 1) { anchor_final(an, k); return; }
   const bool dist = kt_uses_norms(kt);
   double sq = 0.0, mx = 0.0, sqc = 0.0, mxc = 0.0;
   for (int p = threadIdx.x; p < k; p += blockDim.x) {
@@ -412,10 +555,10 @@ __global__ void params_kernel(int k, int kt, double scal, double cons, double po
     const double log2e = 1.4426950408889634;
     const double alpha = (kt == KS_GAUSSIAN) ? sqrt(-scal * log2e) : 1.0;
     const double maxabs = alpha * s_mx[0];
-    double sigma = maxabs > 0.0 ? exp2(ceil(log2(maxabs))) : 1.0;
+    double sigma = maxabs > 0.0 ? pow2_above(maxabs) : 1.0;
     if (sigma < maxabs) sigma *= 2.0;
     const double nbound = alpha * alpha * s_sq[0];        // >= any |x''|^2
-    const double q = exp2(ceil(log2(2.0 * nbound + 1e-300)) - 23.0);
+    const double q = pow2_above(2.0 * nbound + 1e-300) * 0x1p-23;
     P->alpha = alpha; P->sigma = sigma; P->inv_sigma = 1.0 / sigma; P->q = q;
     P->g = 2.0 * sigma * sigma * 0x1p-14;
     P->rc = (float)(-P->g);
@@ -567,10 +710,10 @@ __global__ void task_params_kernel(int ntask, const KParams *__restrict__ kps, c
     }
   }
   const double maxabs = alpha * (centred ? mx_c : mx_u);
-  double sigma = maxabs > 0.0 ? exp2(ceil(log2(maxabs))) : 1.0;
+  double sigma = maxabs > 0.0 ? pow2_above(maxabs) : 1.0;
   if (sigma < maxabs) sigma *= 2.0;
   const double nbound = alpha * alpha * (centred ? sq_c : sq_u);
-  const double q = exp2(ceil(log2(2.0 * nbound + 1e-300)) - 23.0);
+  const double q = pow2_above(2.0 * nbound + 1e-300) * 0x1p-23;
   const double g = 2.0 * sigma * sigma * 0x1p-14;
   const int k = P->k;
   const double delta = 2.0 * (sigma * sigma * (double)k * 0x1p-31) +
@@ -620,6 +763,8 @@ __global__ void task_params_kernel(int ntask, const KParams *__restrict__ kps, c
 __global__ void pool_split(long long n, int k, const double *__restrict__ X, const int *__restrict__ map, int npool,
                            float2 *__restrict__ Xf, const Params *P)
 {
+  launch_dependents();
+  wait_primary();
   if (P && !P->any_flag) return;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)blockDim.x * gridDim.x) {
     size_t src = (size_t)i;
@@ -675,95 +820,6 @@ __device__ void block_source_sums(int j0, int j1, int k, const double *__restric
       else *wsum = r;
     }
     __syncthreads();
-  }
-}
-
-// Anchor point of a single call's polynomial, tanh and compact / multiquadratic
-// kernels (the sources' mean and mean squares per coordinate) and the sum of
-// all weights.  Any point inside the sources' hull keeps each row's anchor
-// value within the range of that row's values, so the mean of a strided
-// sample of at most ANCHOR_SAMPLE sources serves: anchor_coords blocks (cb,
-// sb) take 32 coordinates of ANCHOR_SB-th of the sample each.  The weight sum
-// covers every source (anchor_weights: contiguous ranges, fixed-order tree).
-// anchor_final adds the partials in order.  All of it deterministic.
-constexpr int ANCHOR_SAMPLE = 2048;
-constexpr int ANCHOR_SB = 16;       // sample blocks of anchor_coords
-constexpr int ANCHOR_WPER = 4096;   // weights per block of the weight sum
-
-// cpart[(sb * 2 + 0) * k + p]: sum of coordinate p over sample block sb;
-// cpart[(sb * 2 + 1) * k + p]: the sum of its squares.
-__global__ void __launch_bounds__(256) anchor_coords(int n, int k, const double *__restrict__ XB,
-                                                     const int *__restrict__ bmap, int nxb,
-                                                     double *__restrict__ cpart)
-{
-  __shared__ double sh[2][256];
-  const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
-  const int S = min(n, ANCHOR_SAMPLE), stride = n / S;
-  const int per = (S + ANCHOR_SB - 1) / ANCHOR_SB;
-  const int q0 = blockIdx.y * per, q1 = min(S, q0 + per);
-  const int p = blockIdx.x * 32 + lane;
-  double s = 0.0, s2 = 0.0;
-  if (p < k) {
-#pragma unroll 8
-    for (int q = q0 + wp; q < q1; q += 8) {
-      const double y = XB[(size_t)pool_clamp(bmap, q * stride, nxb) * k + p];
-      s += y;
-      s2 = fma(y, y, s2);
-    }
-  }
-  sh[0][t] = s;
-  sh[1][t] = s2;
-  __syncthreads();
-  if (wp == 0 && p < k) {
-    double r = 0.0, r2 = 0.0;
-    for (int q = 0; q < 8; q++) { r += sh[0][q * 32 + lane]; r2 += sh[1][q * 32 + lane]; }
-    cpart[((size_t)blockIdx.y * 2 + 0) * k + p] = r;
-    cpart[((size_t)blockIdx.y * 2 + 1) * k + p] = r2;
-  }
-}
-
-// wpart[b * nrhs + r]: the sum of weight column r over sources b ANCHOR_WPER ..
-__global__ void __launch_bounds__(256) anchor_weights(int n, const double *__restrict__ w,
-                                                      const int *__restrict__ wmap, int nrhs,
-                                                      double *__restrict__ wpart)
-{
-  __shared__ double sh[256];
-  const int t = threadIdx.x, b = blockIdx.x;
-  const int j0 = b * ANCHOR_WPER, j1 = min(n, j0 + ANCHOR_WPER);
-  for (int r = 0; r < nrhs; r++) {
-    double s = 0.0;
-    for (int j = j0 + t; j < j1; j += 256) s += w[(size_t)(wmap ? wmap[j] : j) * nrhs + r];
-    sh[t] = s;
-    __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-      if (t < h) sh[t] += sh[t + h];
-      __syncthreads();
-    }
-    if (t == 0) wpart[(size_t)b * nrhs + r] = sh[0];
-    __syncthreads();
-  }
-}
-
-// ybar[p], ybsq[p]: the sample's mean and mean square of coordinate p;
-// wsum[r]: the sum of weight column r.
-__global__ void anchor_final(int n, int k, int nwb, int nrhs, const double *__restrict__ cpart,
-                             const double *__restrict__ wpart, double *__restrict__ ybar,
-                             double *__restrict__ ybsq, double *__restrict__ wsum)
-{
-  const double inv = 1.0 / (double)min(n, ANCHOR_SAMPLE);
-  for (int p = threadIdx.x; p < k; p += blockDim.x) {
-    double a = 0.0, b = 0.0;
-    for (int sb = 0; sb < ANCHOR_SB; sb++) {
-      a += cpart[((size_t)sb * 2 + 0) * k + p];
-      b += cpart[((size_t)sb * 2 + 1) * k + p];
-    }
-    ybar[p] = a * inv;
-    ybsq[p] = b * inv;
-  }
-  for (int r = threadIdx.x; r < nrhs; r += blockDim.x) {
-    double a = 0.0;
-    for (int b = 0; b < nwb; b++) a += wpart[(size_t)b * nrhs + r];
-    wsum[r] = a;
   }
 }
 
@@ -823,6 +879,12 @@ __global__ void __launch_bounds__(256) pack_kernel(PackArgs g)
 {
   __shared__ long long s_na[8][32], s_nb[8][32];
   __shared__ int s_ni[8][32];
+  launch_dependents();
+  wait_primary();
+  g.P = after_wait(g.P);
+  g.centre = after_wait(g.centre);
+  g.ybar = after_wait(g.ybar);
+  g.ybsq = after_wait(g.ybsq);
   // nrhs > 1 (sources of several right-hand sides): w holds nrhs interleaved
   // columns and the tiles carry RMAX weights per point (SrcMetaX)
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -2270,6 +2332,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) split_tiles(TileArgs a)
     fence_mbar_init();
   }
   if (warp == 0) { tmem_alloc(&S->tmem_base, TMEM_COLS); tmem_relinquish(); }
+  wait_primary();   // every thread, before any wait of limited length
   float4 *tab_base = (float4 *)((uint8_t *)S + ((sizeof(SplitSmem) + 15) & ~(size_t)15));
   if constexpr (KT == KS_LAPLACE || KT == KS_LIST) laplace_table(tab_base, L.tab_sh, KT == KS_LAPLACE ? &a.P->lap : nullptr);
 
@@ -2566,6 +2629,12 @@ __global__ void split_reduce(int m, int nsc, int ldp, const double *__restrict__
                              int *__restrict__ rlist, int *__restrict__ rcount, const double *__restrict__ rowc,
                              const double *__restrict__ wsum, int nrhs)
 {
+  launch_dependents();
+  wait_primary();
+  partial = after_wait(partial);
+  pskip = after_wait(pskip);
+  rowc = after_wait(rowc);
+  wsum = after_wait(wsum);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   if constexpr (NR == 1) {
@@ -2613,9 +2682,12 @@ __global__ void split_reduce(int m, int nsc, int ldp, const double *__restrict__
 template <int KT, int NR>
 __global__ void __launch_bounds__(256) split_rescue(TileArgs a, const int *__restrict__ rlist,
                                                     const int *__restrict__ rcount, double *__restrict__ u,
-                                                    const int *__restrict__ umap)
+                                                    const int *__restrict__ umap, unsigned long long *nrescued)
 {
   __shared__ float4 tab[LTAB];
+  wait_primary();
+  rlist = after_wait(rlist);
+  rcount = after_wait(rcount);
   if constexpr (KT == KS_LAPLACE) laplace_table(tab, 0);
   __syncthreads();
   const LTab ltab{tab, 0};
@@ -2629,6 +2701,7 @@ __global__ void __launch_bounds__(256) split_rescue(TileArgs a, const int *__res
     T.kcoin = KT == KS_LAPLACE ? lap_coincident(a.kp) : 0.0;
   }
   const int nr = *rcount, lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *nrescued = nr;   // diagnostics (gsks_split_stats)
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < nr; e += nw) {
     const int i = rlist[e];
@@ -2653,22 +2726,24 @@ __global__ void __launch_bounds__(256) split_rescue(TileArgs a, const int *__res
 
 template <int NR>
 cudaError_t launch_rescue_t(const TileArgs &a, int grid, const int *rlist, const int *rcount, double *u,
-                            const int *umap, cudaStream_t s)
+                            const int *umap, unsigned long long *nrescued, cudaStream_t s)
 {
   switch (a.kt) {
-    case KS_GAUSSIAN: split_rescue<KS_GAUSSIAN, NR><<<grid, 256, 0, s>>>(a, rlist, rcount, u, umap); break;
+    case KS_GAUSSIAN:
+      return launch_after(split_rescue<KS_GAUSSIAN, NR>, grid, 256, 0, s, a, rlist, rcount, u, umap, nrescued);
     case KS_GAUSSIAN_VAR_BANDWIDTH:
-      split_rescue<KS_GAUSSIAN_VAR_BANDWIDTH, NR><<<grid, 256, 0, s>>>(a, rlist, rcount, u, umap); break;
-    case KS_LAPLACE: split_rescue<KS_LAPLACE, NR><<<grid, 256, 0, s>>>(a, rlist, rcount, u, umap); break;
+      return launch_after(split_rescue<KS_GAUSSIAN_VAR_BANDWIDTH, NR>, grid, 256, 0, s, a, rlist, rcount, u, umap,
+                          nrescued);
+    case KS_LAPLACE:
+      return launch_after(split_rescue<KS_LAPLACE, NR>, grid, 256, 0, s, a, rlist, rcount, u, umap, nrescued);
     default: return cudaSuccess;
   }
-  return cudaGetLastError();
 }
 cudaError_t launch_rescue(const TileArgs &a, int grid, const int *rlist, const int *rcount, double *u,
-                          const int *umap, cudaStream_t s, int nr)
+                          const int *umap, unsigned long long *nrescued, cudaStream_t s, int nr)
 {
-  return nr > 1 ? launch_rescue_t<RMAX>(a, grid, rlist, rcount, u, umap, s)
-                : launch_rescue_t<1>(a, grid, rlist, rcount, u, umap, s);
+  return nr > 1 ? launch_rescue_t<RMAX>(a, grid, rlist, rcount, u, umap, nrescued, s)
+                : launch_rescue_t<1>(a, grid, rlist, rcount, u, umap, nrescued, s);
 }
 
 template <int KT, int NR>
@@ -2683,8 +2758,11 @@ cudaError_t launch_tiles_t(const TileArgs &a, int grid, size_t smem, cudaStream_
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) attr_bytes[dev] = (int)smem;
   }
-  split_tiles<KT, NR><<<grid, NTHREADS, smem, s>>>(a);
-  return cudaGetLastError();
+  if (a.tab) {   // the list form: it follows fills of memory, not a kernel
+    split_tiles<KT, NR><<<grid, NTHREADS, smem, s>>>(a);
+    return cudaGetLastError();
+  }
+  return launch_after(split_tiles<KT, NR>, grid, NTHREADS, smem, s, a);
 }
 
 template <int NR>
@@ -2784,7 +2862,7 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
   const size_t o_ps = o_p + al(nparts * 8);
   const size_t o_rl = o_ps + (defer ? al(nskips * 4) : 0);
   const size_t o_rc = o_rl + (defer ? al((size_t)m * 4) : 0);
-  const size_t o_ni = o_rc + (defer ? al(4) : 0);   // work counter
+  const size_t o_ni = o_rc + al(4);   // work counter
   const size_t o_xaf = o_ni + al(4);
   const size_t o_xbf = o_xaf + (ff ? al((size_t)ffa * k * sizeof(float2)) : 0);
   // anchored polynomial: source mean and weight sum (ybar | wsum | block
@@ -2814,22 +2892,42 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
   // recomputed in FP64; random per-pair errors of this size keep the summed
   // result well inside 1e-6.
   const float tau = 5e-7f;
-  bbox_init<<<1, 256, 0, s>>>(k, bbox);
-  {
-    const long long tot = (long long)(m + n) * k;
-    const int blocks = (int)std::max<long long>((k + 255) / 256,
-                                                std::min<long long>(8LL * sms, std::max<long long>(1, (tot + 255) / 256)));
-    bbox_kernel<<<blocks, 256, 2 * k * sizeof(long long), s>>>(m, n, k, XA, amap, nxa, XB, bmap, nxb, bbox);
+  // diagnostics of this call (gsks_split_stats): rechecked pairs, rescued rows
+  if (!c->stats.ensure(16)) {
+    if (stream_ordered_alloc) cudaFreeAsync(ws, s);
+    return GSKS_ERR_ALLOC;
   }
-  params_kernel<<<1, params_threads(k), 0, s>>>(k, ker->type, ker->scal, ker->cons, ker->powe, tau, bbox, centre, P);
+  unsigned long long *stats = (unsigned long long *)c->stats.p;
+  int *rlist = defer ? (int *)(ws + o_rl) : nullptr, *rcount = (int *)(ws + o_rc);
+  int *next_item = (int *)(ws + o_ni);
   double *ybar = anch ? (double *)(ws + o_anc) : nullptr;
   double *ybsq = anch ? ybar + k + RMAX + (size_t)nwb * nrhs : nullptr;   // after the weight-sum partials
   double *rowc = anch ? (double *)(ws + o_rowc) : nullptr;
-  if (anch) {
-    double *wpart = ybar + k + RMAX, *cpart = ybsq + k;
-    anchor_coords<<<dim3((k + 31) / 32, ANCHOR_SB), 256, 0, s>>>(n, k, XB, bmap, nxb, cpart);
-    anchor_weights<<<nwb, 256, 0, s>>>(n, w, wmap, nrhs, wpart);
-    anchor_final<<<1, 256, 0, s>>>(n, k, nwb, nrhs, cpart, wpart, ybar, ybsq, ybar + k);
+  bbox_init<<<1, 256, 0, s>>>(k, bbox, next_item, rcount, stats);
+  cudaError_t e = cudaGetLastError();
+  {
+    const long long tot = (long long)(m + n) * k;
+    SurveyArgs v{};
+    v.m = m; v.n = n; v.k = k;
+    v.nbox = (int)std::max<long long>((k + 255) / 256,
+                                      std::min<long long>(8LL * sms, std::max<long long>(1, (tot + 255) / 256)));
+    v.ncoord = anch ? (k + 31) / 32 * ANCHOR_SB : 0;
+    v.XA = XA; v.XB = XB; v.amap = amap; v.bmap = bmap; v.nxa = nxa; v.nxb = nxb;
+    v.w = w; v.wmap = wmap; v.nrhs = nrhs;
+    v.bbox = bbox;
+    AnchorSums an{};
+    if (anch) {
+      v.wpart = ybar + k + RMAX;
+      v.cpart = ybsq + k;
+      an.n = n; an.nwb = nwb; an.nrhs = nrhs;
+      an.cpart = v.cpart; an.wpart = v.wpart;
+      an.ybar = ybar; an.ybsq = ybsq; an.wsum = ybar + k;
+    }
+    if (e == cudaSuccess)
+      e = launch_after(survey_kernel, v.nbox + v.ncoord + (anch ? nwb : 0), 256, 2 * k * sizeof(long long), s, v);
+    if (e == cudaSuccess)
+      e = launch_after(params_kernel, anch ? 2 : 1, params_threads(k), 0, s, k, ker->type, ker->scal, ker->cons,
+                       ker->powe, tau, bbox, centre, P, an);
   }
   PackArgs pk{};
   pk.a.npts = m; pk.a.ntile = ntm; pk.a.X = XA; pk.a.map = amap; pk.a.npool = nxa; pk.a.hvec = hi; pk.a.img = ws + o_a;
@@ -2837,7 +2935,7 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
   pk.k = k; pk.kpad = kpad; pk.kt = ker->type; pk.nrhs = nrhs;
   pk.w = w; pk.wmap = wmap; pk.centre = centre; pk.P = P;
   pk.ybar = ybar; pk.ybsq = ybsq; pk.rowc = rowc; pk.err = err_word(c);
-  pack_kernel<<<(ntm + ntn) * (BM / 32), pack_threads(kpad), 0, s>>>(pk);
+  if (e == cudaSuccess) e = launch_after(pack_kernel, (ntm + ntn) * (BM / 32), pack_threads(kpad), 0, s, pk);
 
   TileArgs a{};
   a.m = m; a.n = n; a.k = k; a.kpad = kpad; a.kt = ker->type;
@@ -2852,9 +2950,14 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
     const long long na_c = ffa * k, nb_c = ffb * k;
     const int ga = (int)std::min<long long>(8LL * sms, (na_c + 255) / 256 + 1);
     const int gb = (int)std::min<long long>(8LL * sms, (nb_c + 255) / 256 + 1);
-    pool_split<<<ga, 256, 0, s>>>(na_c, k, XA, ffpos ? amap : nullptr, nxa, xaf, P);
+    if (e == cudaSuccess)
+      e = launch_after(pool_split, ga, 256, 0, s, na_c, k, XA, ffpos ? amap : nullptr, nxa, xaf, P);
     ff_launches = 1;
-    if (ffb) { pool_split<<<gb, 256, 0, s>>>(nb_c, k, XB, ffpos ? bmap : nullptr, nxb, xbf, P); ff_launches = 2; }
+    if (ffb) {
+      if (e == cudaSuccess)
+        e = launch_after(pool_split, gb, 256, 0, s, nb_c, k, XB, ffpos ? bmap : nullptr, nxb, xbf, P);
+      ff_launches = 2;
+    }
     a.XAf = xaf; a.XBf = xbf;
     a.ffpos = ffpos ? 1 : 0;
   }
@@ -2863,40 +2966,29 @@ int enqueue_split(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, const
   a.P = P;
   a.partial = (double *)(ws + o_p);
   a.pskip = defer ? (float *)(ws + o_ps) : nullptr;
-  a.next_item = (int *)(ws + o_ni);
+  a.next_item = next_item;
   a.ldp = ldp;
   a.err = err_word(c);
   a.wait_limit = tl_split_wait > 0 ? tl_split_wait : WAIT_LIMIT;
   a.stall = tl_split_stall;
   a.nrhs = nrhs;
   const int grid = std::min(ntm * nsc, sms);
-  int *rlist = defer ? (int *)(ws + o_rl) : nullptr, *rcount = defer ? (int *)(ws + o_rc) : nullptr;
-  // diagnostics of this call (gsks_split_stats): rechecked pairs, rescued rows
-  if (!c->stats.ensure(16)) {
-    if (stream_ordered_alloc) cudaFreeAsync(ws, s);
-    return GSKS_ERR_ALLOC;
-  }
-  a.nrecheck = (unsigned long long *)c->stats.p;
-  cudaError_t e = cudaMemsetAsync(c->stats.p, 0, 16, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(a.next_item, 0, sizeof(int), s);
-  if (e == cudaSuccess && defer) e = cudaMemsetAsync(rcount, 0, sizeof(int), s);
+  a.nrecheck = stats;
   if (e == cudaSuccess) e = launch_tiles(a, grid, smem_bytes(kpad, a.kt, NRK), s, NRK);
   if (e == cudaSuccess) {
+    const double *wsum = anch ? ybar + k : nullptr;
     if (NRK > 1)
-      split_reduce<RMAX><<<(m + 255) / 256, 256, 0, s>>>(m, nsc, ldp, a.partial, a.pskip, u, umap, rlist, rcount,
-                                                         rowc, anch ? ybar + k : nullptr, nrhs);
+      e = launch_after(split_reduce<RMAX>, (m + 255) / 256, 256, 0, s, m, nsc, ldp, a.partial, a.pskip, u, umap, rlist,
+                       rcount, rowc, wsum, nrhs);
     else
-      split_reduce<1><<<(m + 255) / 256, 256, 0, s>>>(m, nsc, ldp, a.partial, a.pskip, u, umap, rlist, rcount, rowc,
-                                                      anch ? ybar + k : nullptr, 1);
-    e = cudaGetLastError();
+      e = launch_after(split_reduce<1>, (m + 255) / 256, 256, 0, s, m, nsc, ldp, a.partial, a.pskip, u, umap, rlist,
+                       rcount, rowc, wsum, 1);
   }
   if (e == cudaSuccess && defer)
-    e = cudaMemcpyAsync((uint8_t *)c->stats.p + 8, rcount, sizeof(int), cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess && defer)
-    e = launch_rescue(a, std::max(1, std::min(2 * sms, (m + 7) / 8)), rlist, rcount, u, umap, s, NRK);
+    e = launch_rescue(a, std::max(1, std::min(2 * sms, (m + 7) / 8)), rlist, rcount, u, umap, stats + 1, s, NRK);
   if (stream_ordered_alloc) cudaFreeAsync(ws, s);
   if (e != cudaSuccess) return cuda_status(e, "split launch");
-  note_launches((defer ? 7 : 6) + ff_launches + (anch ? 3 : 0));
+  note_launches((defer ? 7 : 6) + ff_launches);
   return GSKS_OK;
 }
 
@@ -3155,10 +3247,10 @@ int split_list_run(const SplitListPlan &Pl, Ctx *c, const double *XA, const int 
   const SplitTaskGeo *tg = (const SplitTaskGeo *)(ws + Pl.o_tg);
   long long *tbox = (long long *)(ws + Pl.o_tbox);
   double *tcen = (double *)(ws + Pl.o_tcen);
-  bbox_init<<<1, 256, 0, s>>>(k, bbox);
+  bbox_init<<<1, 256, 0, s>>>(k, bbox, nullptr, nullptr, nullptr);
   // every task's box (its targets and sources), folded into the global box
   list_box_kernel<<<ntask, 256, 0, s>>>(ntask, k, tg, XA, a_idx, nxa, XB, b_idx, nxb, tbox, bbox);
-  params_kernel<<<1, params_threads(k), 0, s>>>(k, KS_LIST, 0.0, 0.0, 0.0, tau, bbox, centre, P);
+  params_kernel<<<1, params_threads(k), 0, s>>>(k, KS_LIST, 0.0, 0.0, 0.0, tau, bbox, centre, P, AnchorSums{});
   task_params_kernel<<<(ntask + 127) / 128, 128, 0, s>>>(ntask, (const KParams *)(ws + Pl.o_kps), P, tau, tp, tbox,
                                                           tcen);
   double *ybar = Pl.any_anch ? (double *)(ws + Pl.o_ybar) : nullptr;
