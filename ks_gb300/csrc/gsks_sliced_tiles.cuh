@@ -18,7 +18,8 @@
 //         rows of nothing but extreme digits);
 //   W = sum over l of acc_l 2^-9l as one 64-bit integer, formed with integer
 //         instructions.  What is left out (levels 6 and beyond) is of the size
-//         2^-54 of 2^(e_i + e_j), below the rounding of the norms' own sum.
+//         2^-54 of 2^(e_i + e_j), below the rounding of the norms' own sum; for
+//         few coordinates (K_SEVEN) level 6 is formed too.
 //
 // One conversion then gives x.y in FP64, and the kernel functions follow as in
 // gsks_fp64.cu.  The Gaussian kernel goes further: with the bandwidth folded
@@ -42,7 +43,7 @@
 //                4032 SM cycles of shared-memory bandwidth per 64 columns at
 //                k = 64 where these take 2816)
 //   warps 2..17  epilogue, in two halves of eight, each with an accumulator
-//                buffer (192 TMEM columns) of its own: a half turns its
+//                buffer (192 TMEM columns, 224 with level 6) of its own: a half turns its
 //                accumulators into integers W (bound by the float-to-integer
 //                conversions, 16 per SM cycle) while the other forms kernel
 //                values (bound by the FP64 pipe) and the tensor cores fill the
@@ -79,8 +80,13 @@ constexpr int HALF_WARPS = EPI_WARPS / HALVES;
 constexpr int NTHREADS = 32 * (2 + EPI_WARPS);
 constexpr int NMETA = 4;                         // source metadata slots
 constexpr int NSTAGE_RES = 4, NSTAGE_STR = 2;    // operand stages (resident, streaming)
-constexpr uint32_t TMEM_COLS = 512;              // two buffers of six accumulators (allocation: a power of two)
-constexpr uint32_t TBUF = NS * BN;               // columns of one buffer
+constexpr uint32_t TMEM_COLS = 512;              // two buffers of up to seven accumulators (allocation: a power of two)
+// Levels formed: one more for few coordinates, where the levels left out are the
+// largest part of the error (Gaussian of h = 0.5, k = 3, error of the sums against
+// 64-bit arithmetic: 7.2e-16 with six, 4.7e-16 with seven, DFMA 4.7e-16; from k =
+// 16 on six are as good as DFMA or better: 1.8e-15 against 2.6e-15).
+constexpr int K_SEVEN = 16;                      // below it: seven levels
+__host__ __device__ constexpr int levels(int g) { return g == 3 ? NS + 1 : NS; }
 constexpr size_t SMEM_MAX = 232448;
 constexpr long long WAIT_LIMIT = 1LL << 32;      // clock cycles (~2 s) per wait
 
@@ -160,12 +166,12 @@ __host__ __device__ inline int kchunk(int kpad) { return kpad <= KRES ? kpad : K
 __host__ __device__ inline size_t op_bytes(int rows, int kpad) { return (size_t)NS * rows * kpad * 2; }
 __host__ __device__ inline size_t btile_bytes(int kpad, int nr) { return op_bytes(BN, kpad) + colmeta_bytes(nr); }
 // Bits of W below 2^-52 of 2^(e_i + e_j): what 64 bits leave for k coordinates
-// (|x.y| <= k 2^(e_i + e_j), and sums of norms four times that; three at most,
-// for combine's multipliers).
-__host__ __device__ inline int guard_bits(int kpad)
+// (|x.y| < k 2^(e_i + e_j), and with a frame sums of norms four times that;
+// three at most, for combine's multipliers).
+__host__ __device__ inline int guard_bits(int kpad, bool framed)
 {
   int g = 3;
-  for (int k = 32; k < kpad; k *= 2) g--;
+  for (int k = framed ? 32 : 128; k < kpad; k *= 2) g--;
   return g;
 }
 
@@ -290,7 +296,7 @@ inline __device__ CallParam call_param(const ScanPart &s, CallParam c, int kt, i
   const double mx = __hiloint2double((int)s.maxabs + 1, 0) * c.alpha;
   if (!(mx < 0x1p30)) return c;
   // e as low as the points allow (mx < 2^e), F = 51 + g - 2 e at most 62
-  const int g = guard_bits(kpad);
+  const int g = guard_bits(kpad, true);
   c.e = max((g - 11 + 1) / 2, (__double2hiint(mx) >> 20) - 1022);
   c.F = 51 + g - 2 * c.e;
   if (c.F < 33) return c;
@@ -349,7 +355,10 @@ __device__ __forceinline__ void slice8(const double (&v)[8], int e, bool live, u
     const int fld = (int)(b >> 52) & 0x7ff;
     const int sh = e + 1022 - fld;
     uint64_t X = (b & 0xfffffffffffffull) | 0x10000000000000ull;
-    X = (live && fld != 0 && sh <= 54) ? (X + ((1ull << sh) >> 1)) >> sh : 0ull;
+    // to nearest, ties to even: points on a grid of 2^-54 (uniform generators)
+    // have a tie in every second coordinate, and rounding these up showed as a
+    // bias of x.y
+    X = (live && fld != 0 && sh <= 54) ? (X + ((1ull << sh) >> 1) - (sh > 0 ? ~(X >> sh) & 1ull : 0ull)) >> sh : 0ull;
     if ((long long)b < 0) X = 0ull - X;
     X += 0x1008040201ull << 8;     // 256 (1 + 2^9 + 2^18 + 2^27 + 2^36)
 #pragma unroll
@@ -618,17 +627,18 @@ static_assert(1024 + NSTAGE_STR * NS * (size_t)(BM + HALVES * BN) * KST * 2 + NM
 // The high word that takes the bias of combine's level 0 back out.
 template <int SIGN>
 __device__ __forceinline__ uint32_t combine_bias(int g) { return 0u - 0x4B400000u * (uint32_t)(SIGN * (1 << (4 + g))); }
-// w + SIGN W of one pair, from its six level sums, with g guard bits: four
+// w + SIGN W of one pair, from its level sums, with g guard bits: four
 // 32 x 32 + 64 bit multiply-adds and one into the high word.  Levels 4 and 5
 // join in FP32 (the sum of level 5 is not exact to begin with, and its last
 // bits lie below W's).  Level 0, at most 2^22 over 64 coordinates, becomes an
 // integer by adding 1.5 2^23 to it (w starts with combine_bias in its high
 // word); the others, up to 2^24, need the conversion instruction.
-template <int SIGN>
-__device__ __forceinline__ long long combine(const uint32_t (&r)[NS], int g, long long w)
+template <int SIGN, int LV>
+__device__ __forceinline__ long long combine(const uint32_t (&r)[LV], int g, long long w)
 {
   const float f4 = SIGN * __int_as_float((127 + g) << 23), f5 = SIGN * __int_as_float((118 + g) << 23);   // 2^g, 2^(g-9)
-  const float v = fmaf(__uint_as_float(r[5]), f5, __uint_as_float(r[4]) * f4);
+  float v = fmaf(__uint_as_float(r[5]), f5, __uint_as_float(r[4]) * f4);
+  if (LV > NS) v = fmaf(__uint_as_float(r[LV - 1]), SIGN * __int_as_float((109 + g) << 23), v);                // 2^(g-18)
   w = madws(__float2int_rn(v), 1, w);
   w = madws(__float2int_rn(__uint_as_float(r[3])), SIGN * (1 << (9 + g)), w);
   w = madws(__float2int_rn(__uint_as_float(r[2])), SIGN * (1 << (18 + g)), w);
@@ -931,7 +941,7 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
 
 constexpr bool uses_table(int kt) { return has_frame(kt); }
 
-// G: guard bits of the resident layouts (k <= 32: 3, k <= 64: 2), -1: streaming.
+// G: guard bits of the resident layouts (3; with a frame and k > 32: 2), -1: streaming.
 // A thread's partial sums of row i are stored; the last of the row's parts
 // (count in all) adds them in order into u.  (A reduction kernel of its own cost
 // a launch: 3 us of a 40 us call.)
@@ -956,6 +966,9 @@ __device__ __forceinline__ void row_done(const TileArgs &a, int i, int parts)
 template <int KT, int NR, int G, bool LISTED>
 __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
 {
+  constexpr int LV = levels(G);
+  const bool seven = LV > NS && a.k < K_SEVEN;
+  constexpr uint32_t TBUF = LV * BN;                // columns of one accumulator buffer
   constexpr bool STREAM = G < 0;
   constexpr bool TABLE = uses_table(KT);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1106,9 +1119,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
               for (int s = 0; s < KRES / 16; s++) {
                 if (s < nks) {
 #pragma unroll
-                  for (int i = 0; i < NS; i++)
+                  for (int i = 0; i < NS; i++) {
+                    // (level 6 starts in slice 1, whose first instruction adds to
+                    // levels 1 .. 5: its own first product goes before)
+                    int n = seven && i > 0 ? NS + 1 - i : NS - i;
+                    if (seven && i == 1 && s == 0 && first) {
+                      umma_f16(tmem + h * TBUF + NS * BN, dA + ablk, dB + (uint64_t)(NS - 1) * BN, idesc_f16_f32(BM, BN), 0u);
+                      n = NS - 1;
+                    }
                     umma_f16(tmem + h * TBUF + i * BN, dA + (uint64_t)s * astep + i * ablk, dB + (uint64_t)s * bstep,
-                             idesc_f16_f32(BM, BN * (NS - i)), (i > 0 || s > 0 || !first) ? 1u : 0u);
+                             idesc_f16_f32(BM, BN * n), (i > 0 || s > 0 || !first) ? 1u : 0u);
+                  }
                 }
               }
               if (last) umma_commit(&S->t_full[h]);
@@ -1131,8 +1152,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     const int grp = (warp - 2) >> 2, qd = warp & 3, half = grp >> 1;
     const int row = qd * 32 + lane, c0 = (grp & 1) * COLS;
     const uint32_t tT = tmem + ((uint32_t)(qd * 32) << 16) + half * TBUF + c0;
-    const int gb = G >= 0 ? G : guard_bits(a.kpad);
     constexpr bool FRAMED = has_frame(KT);
+    const int gb = G >= 0 ? G : guard_bits(a.kpad, FRAMED);
     constexpr int SIGN = FRAMED ? -1 : 1;           // W or -W
     const uint32_t bias = combine_bias<SIGN>(gb);
     const uint32_t tabS = smem_addr(sTab);
@@ -1172,9 +1193,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
           tc_fence_after();
 #pragma unroll
           for (int q = 0; q < COLS; q += 4) {
-            uint32_t r[4][NS];
+            uint32_t r[4][LV];
 #pragma unroll
             for (int l = 0; l < NS; l++) tmem_ld4(tT + l * BN + q, r[0][l], r[1][l], r[2][l], r[3][l]);
+            if constexpr (LV > NS) {
+              r[0][NS] = r[1][NS] = r[2][NS] = r[3][NS] = 0;
+              if (seven) tmem_ld4(tT + NS * BN + q, r[0][NS], r[1][NS], r[2][NS], r[3][NS]);
+            }
             const long long b0 = (long long)((uint64_t)bias << 32);
             long long w0[4] = {b0, b0, b0, b0};
             if (STREAM && c > 0) {
@@ -1188,7 +1213,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
             }
             tmem_ld_wait();
 #pragma unroll
-            for (int s = 0; s < 4; s++) W[q + s] = combine<SIGN>(r[s], gb, w0[s]);
+            for (int s = 0; s < 4; s++) W[q + s] = combine<SIGN, LV>(r[s], gb, w0[s]);
           }
           tc_fence_before();
           __syncwarp();
@@ -1281,7 +1306,8 @@ template <int KT, int NR, bool LISTED>
 cudaError_t launch_g(const TileArgs &a, int grid, cudaStream_t s)
 {
   if (a.kpad > KRES) return launch_t<KT, NR, -1, LISTED>(a, grid, s);
-  return a.kpad > 32 ? launch_t<KT, NR, 2, LISTED>(a, grid, s) : launch_t<KT, NR, 3, LISTED>(a, grid, s);
+  if constexpr (!has_frame(KT)) return launch_t<KT, NR, 3, LISTED>(a, grid, s);
+  else return a.kpad > 32 ? launch_t<KT, NR, 2, LISTED>(a, grid, s) : launch_t<KT, NR, 3, LISTED>(a, grid, s);
 }
 
 }  // namespace sliced

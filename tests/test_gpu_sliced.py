@@ -98,7 +98,7 @@ def _params(ktype, params, k):
     return p
 
 
-@pytest.mark.parametrize("k", [3, 16, 17, 64, 65, 200, 1024, 1025])
+@pytest.mark.parametrize("k", [3, 15, 16, 17, 64, 65, 200, 1024, 1025])
 @pytest.mark.parametrize("ktype,params", KINDS)
 def test_kernels_over_k(gpu, oracle_mod, ktype, params, k):
     from ks_gb300 import gsks
