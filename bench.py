@@ -296,8 +296,15 @@ def roofline_split(per, peaks, rates):
 # FP64 pipe: ncu reports sm__inst_executed_pipe_fp64.avg.peak_sustained = 1/16
 # warp instruction per SM cycle on GB300, i.e. 2 DFMA per SM per cycle; the
 # FP64 tensor-core MMA (DMMA) issues to the same pipe at 1.8 FMA per SM cycle
-# (profiles/fp64_pipe_peak.md).
+# (profiles/fp64_pipe_peak.md).  The FP64 form's inner products run on the f16
+# tensor cores instead (k <= 1024): 21 exact digit products per coordinate; its
+# kernel values run on integer instructions, which leaves the FP64 pipe the
+# weighted sum (and, for polynomials, scal x.y + cons).
 FP64_FMA_PER_SM_CYCLE = 2.0
+
+
+FP64_DIGIT_PRODUCTS = 21
+FP64_PIPE_PER_PAIR = {"gaussian": 1, "laplace": 1, "polynomial": 2}
 
 
 def fp64_peak(sms, sm_mhz):
@@ -305,19 +312,22 @@ def fp64_peak(sms, sm_mhz):
     return 2.0 * FP64_FMA_PER_SM_CYCLE * sms * sm_mhz * 1e6
 
 
-def roofline_fp64(per, peak):
-    """FP64 form per kernel: the reference's flop model (2k + f per pair,
-    test/test_dgsks.c:254-283; it counts more flops for pow/exp than binary
-    powering issues, so it can exceed 1) and the rank-k part alone (2k per
-    pair, every one a DFMA: a lower bound of the pipe's load)."""
+def roofline_fp64(per, peaks, peak):
+    """FP64 form per kernel: the executed digit products at the tensor peak, the
+    FP64 instructions per pair at that pipe's rate, and the time over the larger
+    of the two.  alg_tflops is the reference's flop model (2k + f per pair,
+    test/test_dgsks.c:254-283) over the time."""
     out = {}
+    tc_peak = peaks.get("bf16_tflops", 1900.0) * 1e12
     for name, kt, p, f in KERNELS:
         t = per[name] * 1e-3
-        flops = M_T * N_S * (2 * K_DIM + f)
-        rank_k = M_T * N_S * 2 * K_DIM
-        out[name] = {"ms": round(per[name], 3), "pairs_per_s": M_T * N_S / t,
-                     "achieved_tflops": round(flops / t / 1e12, 4), "frac": round(flops / t / peak, 4),
-                     "frac_rank_k": round(rank_k / t / peak, 4)}
+        pairs = M_T * N_S
+        execd = FP64_DIGIT_PRODUCTS * 2.0 * pairs * ((K_DIM + 15) // 16 * 16)
+        t_tc, t_fp64 = execd / tc_peak, 2.0 * FP64_PIPE_PER_PAIR[name] * pairs / peak
+        out[name] = {"ms": round(per[name], 3), "pairs_per_s": pairs / t,
+                     "alg_tflops": round(pairs * (2 * K_DIM + f) / t / 1e12, 4),
+                     "executed_tflops": round(execd / t / 1e12, 2), "frac_executed_tensor": round(t_tc / t, 4),
+                     "frac_fp64_pipe": round(t_fp64 / t, 4), "frac_of_binding": round(max(t_tc, t_fp64) / t, 4)}
     return out
 
 
@@ -385,7 +395,7 @@ def run_ours(args, ws, rank, local):
     p64 = fp64_peak(sms, sm_mhz)
     for form in forms:
         results[form]["per_kernel"] = (roofline_split(pers[form], peaks, rates) if form == "split"
-                                       else roofline_fp64(pers[form], p64))
+                                       else roofline_fp64(pers[form], peaks, p64))
     head = forms[0]
     H = results[head]
 
@@ -402,11 +412,12 @@ def run_ours(args, ws, rank, local):
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst; f16 runs at the bf16 rate)"
                 if "bf16_tflops" in peaks else "fallback 1.9 PFLOP/s bf16"}
     else:
-        roof = {"bound": "fp64", "kernel": f"fp64_tiles<{dom}>", "achieved": dk["achieved_tflops"],
-                "peak": round(p64 / 1e12, 4), "unit": "TFLOP/s", "frac": dk["frac"],
-                "traffic": read_traffic(f"fp64_tiles_{dom}_general_stride"),
-                "peak_source": "FP64 pipe issue rate (ncu peak_sustained: 2 DFMA per SM cycle) x SMs x the "
-                               "median SM clock sampled in the timed region"}
+        roof = {"bound": "tensor", "kernel": f"sliced_tiles<{dom}>", "achieved": dk["executed_tflops"],
+                "peak": round(peaks.get("bf16_tflops", 1900.0), 1), "unit": "TFLOP/s",
+                "frac": dk["frac_executed_tensor"], "traffic": read_traffic(f"sliced_tiles_{dom}_general_stride"),
+                "flops": "executed f16 digit products (21 per coordinate pair); frac_fp64_pipe beside it",
+                "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst; f16 runs at the bf16 rate)"
+                if "bf16_tflops" in peaks else "fallback 1.9 PFLOP/s bf16"}
     roof["fp64_peak_tflops"] = round(p64 / 1e12, 4)
     roof["fp64_peak_source"] = ("2 DFMA per SM cycle (ncu sm__inst_executed_pipe_fp64 peak_sustained) x "
                                 f"{sms} SMs x {sm_mhz:.0f} MHz (median sampled); live probes: DFMA chains "
@@ -910,7 +921,7 @@ def _config_data(torch, name, k, m, seed):
 def config_results(args, torch, gsks, O, cname, ks, clk, flush, steps, warmup):
     """One configuration at full size: per k and kernel, the split form over all
     m*n pairs (median of `steps` calls, L2 flushed before each), the FP64 form
-    on a block of target rows x all sources (about 0.3 s), and both forms'
+    on a block of target rows x all sources (15 to 90 ms), and both forms'
     errors on 256 sampled rows against the oracle.  Both forms are timed
     inside the clock sampler `clk`."""
     import numpy as np
@@ -956,8 +967,9 @@ def config_results(args, torch, gsks, O, cname, ks, clk, flush, steps, warmup):
             pairs = float(m) * m
             u_split = (u / steps).cpu().numpy()
             stats = gsks.split_stats()
-            # FP64 on a block of rows sized to about 0.3 s (at least 1024 rows: the
-            # plan splits the sources into chunks, so every SM stays busy)
+            # FP64 on a block of rows that the DFMA kernels took 0.3 s for (15 to 90 ms
+            # now; at least 1024 rows: the plan splits the sources into chunks, so every
+            # SM stays busy)
             est = 5.9e11 / (k + 12)
             mr = int(min(m, max(1024, est * 0.3 / m)))
             mr = (mr // 64) * 64
@@ -992,8 +1004,7 @@ def config_results(args, torch, gsks, O, cname, ks, clk, flush, steps, warmup):
             err = {"split": {kk: float("%.3g" % v) for kk, v in O.errors(u_split[sample], ref, cond=cond).items()},
                    "fp64": {kk: float("%.3g" % v) for kk, v in O.errors(ufh[sample], ref, cond=cond).items()}}
             alg = 2.0 * pairs * k
-            sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
-            p64 = fp64_peak(sms, clk.summary().get("sm_mhz") or 2070.0)
+            kp16 = (k + 15) // 16 * 16
             results.append({"k": k, "kernel": name, "pairs": pairs,
                             "split": {"value": pairs / t_split, "ms": round(t_split * 1e3, 3),
                                       "alg_tflops": round(alg / t_split / 1e12, 2),
@@ -1001,7 +1012,7 @@ def config_results(args, torch, gsks, O, cname, ks, clk, flush, steps, warmup):
                                       "rechecked_pairs": stats["rechecked_pairs"],
                                       "rescued_rows": stats["rescued_rows"]},
                             "fp64": {"value": fp64_rate, "rows_timed": mr, "ms": round(t_fp64 * 1e3, 2),
-                                     "frac_rank_k": round(2.0 * k * fp64_rate / p64, 4)},
+                                     "frac_executed_tensor": round(FP64_DIGIT_PRODUCTS * 2.0 * kp16 * fp64_rate / tc_peak, 4)},
                             "split_over_fp64": (pairs / t_split) / fp64_rate,
                             "error": err, "rows_checked": int(sample.size)})
             del u, uf

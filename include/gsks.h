@@ -6,7 +6,7 @@
  *   - status codes and gsks_last_error() (the reference prints and exits,
  *     frame/dgsks.c:465-467, frame/omp_dgsks_list.cpp:321-324,
  *     frame/ks_util.c:50-51);
- *   - a precision switch: plain FP64 or split-precision tensor-core form;
+ *   - a precision switch: FP64 or split-precision tensor-core form;
  *   - device-resident entry points taking device pointers and a CUDA stream;
  *   - dgsks_list, a flat C-ABI batched call over CSR task lists (the
  *     reference only has the C++ std::vector interface of
@@ -50,7 +50,9 @@ const char *gsks_error_string(int code);
 
 /* ---- precision --------------------------------------------------------- */
 enum {
-  GSKS_FP64 = 0,        /* FP64 rank-k, FP64 kernel function and sums        */
+  GSKS_FP64 = 0,        /* FP64: exact digit products on the tensor cores up
+                           to k = 1024 (DFMA beyond), kernel function in
+                           FP64 or 64-bit integers, FP64 sums               */
   GSKS_SPLIT_BF16X3 = 1 /* split-precision tensor-core form.  (The name is
                            kept for compatibility: each coordinate is split
                            into three 16-bit slices, an integer head exact in

@@ -1,4 +1,7 @@
-// gsks_fp64.cu -- plain FP64 form of the fused kernel summation (sm_103a).
+// gsks_fp64.cu -- DFMA kernels of the fused kernel summation (sm_103a): the FP64
+// form beyond k = 1024 and the allocation-free entry.  (Up to k = 1024 the digit
+// products of gsks_sliced.cu are 7 to 45 times as fast; beyond it a row's digits
+// no longer fit the sums' 64 bits.)
 //
 // A work item is (a tile of up to BM targets gathered through amap) x (a
 // chunk of sources gathered through bmap).  It forms the rank-k inner
@@ -11,7 +14,7 @@
 // Replaces the reference's BLIS loop nest and x86 micro-kernels:
 //   frame/dgsks.c:367-776 (jc/pc/ic loops, gather-packing :70-213),
 //   micro_kernel/x86_64/sandybridge/ks_*_int_d8x4.c (rank-k + kernel + sum).
-// The batched form (gsks_list.cu) runs the same item over a size-sorted queue
+// The batched form (gsks_list.cu), k > 1024, runs the same item over a size-sorted queue
 // of (task, target tile, source chunk) items in one persistent launch.
 //
 // GB300 note: FP64 issues at a small fraction of the FP32 rate on this part,

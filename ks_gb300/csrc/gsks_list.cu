@@ -1,11 +1,11 @@
-// gsks_list.cu -- dgsks_list: many kernel summations in one persistent launch.
+// gsks_list.cu -- dgsks_list: many kernel summations in one batched evaluation.
 //
 // The reference batches with OpenMP: a greedy cost-balanced assignment of
 // tasks to 68 worker queues, one dgsks call per task into a per-thread copy of
 // u, and a serial merge (frame/omp_dgsks_list.cpp:297-420).  Here the whole
 // list becomes one queue of work items (task, target tile, source chunk)
 // sorted by cost, largest first, which a persistent kernel drains through an
-// atomic counter (no waits).  Every item writes per-row partial sums; a merge
+// atomic counter (FP64 form up to k = 1024: one such kernel per kernel type).  Every item writes per-row partial sums; a merge
 // kernel then adds, for each distinct u entry, the contributions of all list
 // positions that name it in ascending position order -- the same order on
 // every run, so the result is deterministic without floating-point atomics.

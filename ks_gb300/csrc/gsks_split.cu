@@ -873,7 +873,7 @@ struct PackArgs {
 // side by side and 32 points' 16-byte segments are stored together; the norms'
 // integer sums are added over the warps (exactly), the metadata left to warp 0.
 // (One thread per point took 70 us a side for 65536 points at k = 64 and, in the
-// batched workload at k = 16, 1.9 ms of 4000 tasks' 7.9.)  Bound by the FP64
+// batched workload at k = 16, 1.9 ms of 4000 tasks' 7.9; now 1.2 ms.)  Bound by the FP64
 // pipe: two instructions and a conversion per coordinate.
 __global__ void __launch_bounds__(256) pack_kernel(PackArgs g)
 {
