@@ -23,3 +23,22 @@ def test_split_survey_edges(gpu, oracle_mod, m, n, k, ktype, params):
     perm = rng.permutation(N).astype(np.int32)
     e = _run(gpu, oracle_mod, ktype, params, X, rng.standard_normal(N), perm[:m], perm[m:], perm[:m], perm[m:])
     assert e["normwise"] <= TOL and e["cond_max"] <= TOL, e
+
+
+@pytest.mark.parametrize("k", [5, 64, 100])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e200])
+def test_split_non_finite_coordinate(gpu, k, bad):
+    """A coordinate that the operand slices cannot hold does not turn into a finite value."""
+    from ks_gb300 import gsks
+    rng = np.random.default_rng(k)
+    X = rng.random((300, k))
+    X[7, k // 2] = bad
+    t = lambda a: gpu.from_numpy(np.ascontiguousarray(a)).cuda()
+    i = t(np.arange(300, dtype=np.int32))
+    x, u = t(X), gpu.zeros(300, dtype=gpu.float64, device="cuda")
+    with np.errstate(over="ignore"):
+        x2 = t((X * X).sum(1))
+    gsks.dgsks_device(gsks.make_kernel(1, scal=0.05, cons=1.0, powe=2.0), 300, 300, k, u, i, x, x2, i, x, x2, i,
+                      t(rng.random(300)), i, precision=1, stream=gpu.cuda.current_stream(), nxa=300, nxb=300)
+    gpu.cuda.synchronize()
+    assert not np.isfinite(u.cpu().numpy()[7])
