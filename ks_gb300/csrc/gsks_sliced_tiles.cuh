@@ -86,7 +86,8 @@ constexpr uint32_t TMEM_COLS = 512;              // two buffers of up to seven a
 // 64-bit arithmetic: 7.2e-16 with six, 4.7e-16 with seven, DFMA 4.7e-16; from k =
 // 16 on six are as good as DFMA or better: 1.8e-15 against 2.6e-15).
 constexpr int K_SEVEN = 16;                      // below it: seven levels
-__host__ __device__ constexpr int levels(int g) { return g == 3 ? NS + 1 : NS; }
+// (A variant of its own: as a run-time choice it cost a batch at k = 16 5 %.)
+__host__ __device__ constexpr int levels(int g) { return g == 4 ? NS + 1 : NS; }
 constexpr size_t SMEM_MAX = 232448;
 constexpr long long WAIT_LIMIT = 1LL << 32;      // clock cycles (~2 s) per wait
 
@@ -941,7 +942,8 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
 
 constexpr bool uses_table(int kt) { return has_frame(kt); }
 
-// G: guard bits of the resident layouts (3; with a frame and k > 32: 2), -1: streaming.
+// G: guard bits of the resident layouts (3; with a frame and k > 32: 2),
+// 4: three with a seventh level, -1: streaming.
 // A thread's partial sums of row i are stored; the last of the row's parts
 // (count in all) adds them in order into u.  (A reduction kernel of its own cost
 // a launch: 3 us of a 40 us call.)
@@ -967,7 +969,7 @@ template <int KT, int NR, int G, bool LISTED>
 __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
 {
   constexpr int LV = levels(G);
-  const bool seven = LV > NS && a.k < K_SEVEN;
+  constexpr bool seven = LV > NS;
   constexpr uint32_t TBUF = LV * BN;                // columns of one accumulator buffer
   constexpr bool STREAM = G < 0;
   constexpr bool TABLE = uses_table(KT);
@@ -1153,7 +1155,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     const int row = qd * 32 + lane, c0 = (grp & 1) * COLS;
     const uint32_t tT = tmem + ((uint32_t)(qd * 32) << 16) + half * TBUF + c0;
     constexpr bool FRAMED = has_frame(KT);
-    const int gb = G >= 0 ? G : guard_bits(a.kpad, FRAMED);
+    const int gb = G >= 0 ? (G < 3 ? G : 3) : guard_bits(a.kpad, FRAMED);
     constexpr int SIGN = FRAMED ? -1 : 1;           // W or -W
     const uint32_t bias = combine_bias<SIGN>(gb);
     const uint32_t tabS = smem_addr(sTab);
@@ -1195,11 +1197,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
           for (int q = 0; q < COLS; q += 4) {
             uint32_t r[4][LV];
 #pragma unroll
-            for (int l = 0; l < NS; l++) tmem_ld4(tT + l * BN + q, r[0][l], r[1][l], r[2][l], r[3][l]);
-            if constexpr (LV > NS) {
-              r[0][NS] = r[1][NS] = r[2][NS] = r[3][NS] = 0;
-              if (seven) tmem_ld4(tT + NS * BN + q, r[0][NS], r[1][NS], r[2][NS], r[3][NS]);
-            }
+            for (int l = 0; l < LV; l++) tmem_ld4(tT + l * BN + q, r[0][l], r[1][l], r[2][l], r[3][l]);
             const long long b0 = (long long)((uint64_t)bias << 32);
             long long w0[4] = {b0, b0, b0, b0};
             if (STREAM && c > 0) {
@@ -1306,6 +1304,7 @@ template <int KT, int NR, bool LISTED>
 cudaError_t launch_g(const TileArgs &a, int grid, cudaStream_t s)
 {
   if (a.kpad > KRES) return launch_t<KT, NR, -1, LISTED>(a, grid, s);
+  if (a.k < K_SEVEN) return launch_t<KT, NR, 4, LISTED>(a, grid, s);
   if constexpr (!has_frame(KT)) return launch_t<KT, NR, 3, LISTED>(a, grid, s);
   else return a.kpad > 32 ? launch_t<KT, NR, 2, LISTED>(a, grid, s) : launch_t<KT, NR, 3, LISTED>(a, grid, s);
 }
