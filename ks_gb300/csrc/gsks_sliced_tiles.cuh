@@ -780,7 +780,7 @@ __device__ __noinline__ double rare_value(const TileArgs &a, const KParams &kp, 
       if (d2 < fmax(1e-15, kp.coinc * 2.0 * ((double)A * ldexp(1.0, -cp.F)))) d2 = 1.79e308;
       return pow_call(d2, kp);      // the row's sum is multiplied by scal
     } else {
-      const int pa = a.amap ? a.amap[i] : i, pb = a.bmap ? a.bmap[j] : j;
+      const int pa = pool_clamp(a.amap, i, a.nxa), pb = pool_clamp(a.bmap, j, a.nxb);   // flagged by slice_kernel
       return exp2_neg64(((d2 * (0.5 * 1.4426950408889634 * 0x1p53)) * kp.hi[pa]) * kp.hj[pb], tab);
     }
   }
