@@ -411,7 +411,10 @@ KParams make_kparams(const ks_t *ker, const double *hi, const double *hj)
 {
   KParams kp;
   kp.type = ker->type; kp.scal = ker->scal; kp.cons = ker->cons; kp.powe = ker->powe;
-  kp.hi = hi; kp.hj = hj;
+  // only the variable-bandwidth kernel has bandwidths: whatever else a descriptor of
+  // another type holds there (nothing sets it) reaches no kernel
+  const bool varbw = ker->type == KS_GAUSSIAN_VAR_BANDWIDTH;
+  kp.hi = varbw ? hi : nullptr; kp.hj = varbw ? hj : nullptr;
   kp.coinc = 0.0;
   kp.pmode = POW_GENERAL; kp.pint = 0;
   const double p = ker->powe;

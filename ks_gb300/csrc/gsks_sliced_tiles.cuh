@@ -277,7 +277,7 @@ static __global__ void __launch_bounds__(256) list_scan_kernel(SliceArgs a, int 
   const TaskGeo G = tg[t];
   const KParams &kp = tp[t].kp;
   const bool vb = kp.type == KS_GAUSSIAN_VAR_BANDWIDTH;
-  const ScanPart r = scan_fold(scan_points<8>(a, G.a0, G.m, G.b0, G.n, vb ? kp.hi : nullptr, kp.hj, 0, 1));
+  const ScanPart r = scan_fold(scan_points<8>(a, G.a0, G.m, G.b0, G.n, vb ? kp.hi : nullptr, vb ? kp.hj : nullptr, 0, 1));
   if (threadIdx.x == 0) tp[t].cp = call_param(r, tp[t].cp, tp[t].kp.type, a.kpad);
 }
 
