@@ -12,14 +12,13 @@
 //         six balanced digits |d| <= 256, stored as FP16 integers (the
 //         row's largest coordinate is held to its last bit, every other one to
 //         2^-54 of 2^e);
-//   the products of digits i and j, i + j = l <= 5, are integers; their sums
+//   the products of digits i and j, i + j = l <= 6, are integers; their sums
 //         over 64 coordinates stay within 2^24 and are exact in the FP32
-//         accumulator of level l (levels 4 and 5 may round their last bit on
-//         rows of nothing but extreme digits);
+//         accumulator of level l up to 3 (beyond, rows of nothing but extreme
+//         digits may round their last bit);
 //   W = sum over l of acc_l 2^-9l as one 64-bit integer, formed with integer
-//         instructions.  What is left out (levels 6 and beyond) is of the size
-//         2^-54 of 2^(e_i + e_j), below the rounding of the norms' own sum; for
-//         few coordinates (K_SEVEN) level 6 is formed too.
+//         instructions, one rounding per 64 coordinates.  What is left out
+//         (levels 7 and beyond) is at most k 2^-61 of 2^(e_i + e_j).
 //
 // One conversion then gives x.y in FP64, and the kernel functions follow as in
 // gsks_fp64.cu.  The Gaussian kernel goes further: with the bandwidth folded
@@ -36,14 +35,14 @@
 //                k = 64), source tiles through four stages; beyond k = 64 two
 //                source tiles and the targets in 32-wide chunks
 //   warp 1       MMA issue: the source slices lie stacked along N, so that
-//                target slice i times slices 0 .. 5 - i is one tcgen05.mma of
-//                N = 32 (6 - i) whose columns are the accumulators of levels
-//                i .. 5: six instructions per 16 coordinates, each target
+//                target slice i times slices 0 .. 6 - i (0 .. 5 for i = 0) is one
+//                tcgen05.mma of N = 32 (7 - i) whose columns are the accumulators of
+//                levels i .. 6: six instructions per 16 coordinates, each target
 //                slice read once (21 of N = 64 read it six times over and took
 //                4032 SM cycles of shared-memory bandwidth per 64 columns at
 //                k = 64 where these take 2816)
 //   warps 2..17  epilogue, in two halves of eight, each with an accumulator
-//                buffer (192 TMEM columns, 224 with level 6) of its own: a half turns its
+//                buffer (224 TMEM columns) of its own: a half turns its
 //                accumulators into integers W (bound by the float-to-integer
 //                conversions, 16 per SM cycle) while the other forms kernel
 //                values (bound by the FP64 pipe) and the tensor cores fill the
@@ -81,13 +80,14 @@ constexpr int NTHREADS = 32 * (2 + EPI_WARPS);
 constexpr int NMETA = 4;                         // source metadata slots
 constexpr int NSTAGE_RES = 4, NSTAGE_STR = 2;    // operand stages (resident, streaming)
 constexpr uint32_t TMEM_COLS = 512;              // two buffers of up to seven accumulators (allocation: a power of two)
-// Levels formed: one more for few coordinates, where the levels left out are the
-// largest part of the error (Gaussian of h = 0.5, k = 3, error of the sums against
-// 64-bit arithmetic: 7.2e-16 with six, 4.7e-16 with seven, DFMA 4.7e-16; from k =
-// 16 on six are as good as DFMA or better: 1.8e-15 against 2.6e-15).
-constexpr int K_SEVEN = 16;                      // below it: seven levels
-// (A variant of its own: as a run-time choice it cost a batch at k = 16 5 %.)
-__host__ __device__ constexpr int levels(int g) { return g == 4 ? NS + 1 : NS; }
+// Levels formed.  With six the products left out were the largest part of the error
+// wherever the points do not lie in one orthant far from the origin: the error's rms in
+// units of 2^-53 of the conditioned sum, six levels -> seven (DFMA): Laplace of normal
+// points, k = 16, 4.5 -> 0.5 (0.5); tanh of sparse rows, k = 33, 2.4 -> 0.7 (0.2);
+// polynomial of rows with one large coordinate, k = 1000, 4.5 -> 1.3 (1.3).  The seventh
+// costs 8 % where the streamed images bound the kernel (8192 x 12000, k = 1024: 4.30 ->
+// 4.65 ms), 1 to 3 % elsewhere (65536 x 65536, k = 64: 13.84 -> 14.01 ms).
+constexpr int LV = NS + 1;
 constexpr size_t SMEM_MAX = 232448;
 constexpr long long WAIT_LIMIT = 1LL << 32;      // clock cycles (~2 s) per wait
 
@@ -629,17 +629,17 @@ static_assert(1024 + NSTAGE_STR * NS * (size_t)(BM + HALVES * BN) * KST * 2 + NM
 template <int SIGN>
 __device__ __forceinline__ uint32_t combine_bias(int g) { return 0u - 0x4B400000u * (uint32_t)(SIGN * (1 << (4 + g))); }
 // w + SIGN W of one pair, from its level sums, with g guard bits: four
-// 32 x 32 + 64 bit multiply-adds and one into the high word.  Levels 4 and 5
-// join in FP32 (the sum of level 5 is not exact to begin with, and its last
-// bits lie below W's).  Level 0, at most 2^22 over 64 coordinates, becomes an
-// integer by adding 1.5 2^23 to it (w starts with combine_bias in its high
-// word); the others, up to 2^24, need the conversion instruction.
-template <int SIGN, int LV>
+// 32 x 32 + 64 bit multiply-adds and one into the high word.  Levels 4 to 6
+// join in FP32 (their last bits lie below W's or near its last one).  Level 0, at
+// most 2^22 over 64 coordinates, becomes an integer by adding 1.5 2^23 to it (w
+// starts with combine_bias in its high word); the others, up to 2^24, need the
+// conversion instruction.
+template <int SIGN>
 __device__ __forceinline__ long long combine(const uint32_t (&r)[LV], int g, long long w)
 {
   const float f4 = SIGN * __int_as_float((127 + g) << 23), f5 = SIGN * __int_as_float((118 + g) << 23);   // 2^g, 2^(g-9)
   float v = fmaf(__uint_as_float(r[5]), f5, __uint_as_float(r[4]) * f4);
-  if (LV > NS) v = fmaf(__uint_as_float(r[LV - 1]), SIGN * __int_as_float((109 + g) << 23), v);                // 2^(g-18)
+  v = fmaf(__uint_as_float(r[6]), SIGN * __int_as_float((109 + g) << 23), v);   // 2^(g-18)
   w = madws(__float2int_rn(v), 1, w);
   w = madws(__float2int_rn(__uint_as_float(r[3])), SIGN * (1 << (9 + g)), w);
   w = madws(__float2int_rn(__uint_as_float(r[2])), SIGN * (1 << (18 + g)), w);
@@ -942,8 +942,6 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
 
 constexpr bool uses_table(int kt) { return has_frame(kt); }
 
-// G: guard bits of the resident layouts (3; with a frame and k > 32: 2),
-// 4: three with a seventh level, -1: streaming.
 // A thread's partial sums of row i are stored; the last of the row's parts
 // (count in all) adds them in order into u.  (A reduction kernel of its own cost
 // a launch: 3 us of a 40 us call.)
@@ -965,11 +963,10 @@ __device__ __forceinline__ void row_done(const TileArgs &a, int i, int parts)
   }
 }
 
+// G: guard bits of the resident layouts (3; with a frame and k > 32: 2), -1: streaming.
 template <int KT, int NR, int G, bool LISTED>
 __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
 {
-  constexpr int LV = levels(G);
-  constexpr bool seven = LV > NS;
   constexpr uint32_t TBUF = LV * BN;                // columns of one accumulator buffer
   constexpr bool STREAM = G < 0;
   constexpr bool TABLE = uses_table(KT);
@@ -1124,8 +1121,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
                   for (int i = 0; i < NS; i++) {
                     // (level 6 starts in slice 1, whose first instruction adds to
                     // levels 1 .. 5: its own first product goes before)
-                    int n = seven && i > 0 ? NS + 1 - i : NS - i;
-                    if (seven && i == 1 && s == 0 && first) {
+                    int n = i > 0 ? NS + 1 - i : NS;
+                    if (i == 1 && s == 0 && first) {
                       umma_f16(tmem + h * TBUF + NS * BN, dA + ablk, dB + (uint64_t)(NS - 1) * BN, idesc_f16_f32(BM, BN), 0u);
                       n = NS - 1;
                     }
@@ -1155,7 +1152,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     const int row = qd * 32 + lane, c0 = (grp & 1) * COLS;
     const uint32_t tT = tmem + ((uint32_t)(qd * 32) << 16) + half * TBUF + c0;
     constexpr bool FRAMED = has_frame(KT);
-    const int gb = G >= 0 ? (G < 3 ? G : 3) : guard_bits(a.kpad, FRAMED);
+    const int gb = G >= 0 ? G : guard_bits(a.kpad, FRAMED);
     constexpr int SIGN = FRAMED ? -1 : 1;           // W or -W
     const uint32_t bias = combine_bias<SIGN>(gb);
     const uint32_t tabS = smem_addr(sTab);
@@ -1211,7 +1208,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
             }
             tmem_ld_wait();
 #pragma unroll
-            for (int s = 0; s < 4; s++) W[q + s] = combine<SIGN, LV>(r[s], gb, w0[s]);
+            for (int s = 0; s < 4; s++) W[q + s] = combine<SIGN>(r[s], gb, w0[s]);
           }
           tc_fence_before();
           __syncwarp();
@@ -1304,7 +1301,6 @@ template <int KT, int NR, bool LISTED>
 cudaError_t launch_g(const TileArgs &a, int grid, cudaStream_t s)
 {
   if (a.kpad > KRES) return launch_t<KT, NR, -1, LISTED>(a, grid, s);
-  if (a.k < K_SEVEN) return launch_t<KT, NR, 4, LISTED>(a, grid, s);
   if constexpr (!has_frame(KT)) return launch_t<KT, NR, 3, LISTED>(a, grid, s);
   else return a.kpad > 32 ? launch_t<KT, NR, 2, LISTED>(a, grid, s) : launch_t<KT, NR, 3, LISTED>(a, grid, s);
 }
