@@ -1152,9 +1152,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     const int row = qd * 32 + lane, c0 = (grp & 1) * COLS;
     const uint32_t tT = tmem + ((uint32_t)(qd * 32) << 16) + half * TBUF + c0;
     constexpr bool FRAMED = has_frame(KT);
-    const int gb = G >= 0 ? G : guard_bits(a.kpad, FRAMED);
     constexpr int SIGN = FRAMED ? -1 : 1;           // W or -W
-    const uint32_t bias = combine_bias<SIGN>(gb);
     const uint32_t tabS = smem_addr(sTab);
     int tbase = 0, tg = 0;                          // tiles before this item, accumulations taken
     for (int it = 0; !*abort; it++) {
@@ -1171,6 +1169,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
       const KParams &kp = LISTED ? S->tslot[it & 1].kp : a.kp;
       const CallParam &cp = LISTED ? S->tslot[it & 1].cp : *a.cp;
       const bool fixed = FRAMED && cp.fixed != 0;
+      // (without the frame's norms the sum of many coordinates leaves two bits more)
+      const int gb = G >= 0 ? G : guard_bits(a.kpad, fixed);
+      const uint32_t bias = combine_bias<SIGN>(gb);
       const ExpFrame E = KT == KS_GAUSSIAN ? exp_frame(max(fixed ? cp.F : 43, 43), tabS) : exp_frame52(tabS);
       const long long arow = __double_as_longlong(a.row_aa[i0]);
       const bool anyrow = __any_sync(0xffffffffu, a.row_e[i0] == EFLAG);

@@ -42,3 +42,39 @@ def test_every_level_that_reaches_the_rounding(gpu, k, listed):
     tol = runs * 2.0 ** -49 + 2 * k * 2.0 ** -59 + 8 * 2.0 ** -53 * float(exact)
     err = abs(Fraction(float(u.cpu()[0])) - exact)
     assert err <= tol, (float(err), tol)
+
+
+def test_guard_bits_without_a_frame(gpu):
+    """A kernel that has a fixed-point form, on points that leave it off (one near the
+    origin): x.y keeps the guard bits of a plain inner product.  Rows x = (3/4, s, .., s)
+    and y = (5/8, t, .., t) on the digits' grid, k = 1024: every run of 64 coordinates has
+    the same sum, so that its rounding to W's unit (2^-52; 2^-50 with the frame's guard
+    bits) adds up 16 times.  Bound on the exponent: 16 roundings of at most one unit, twice
+    for 2 x.y, the level left out (2^-50), the norms' and the value's own rounding."""
+    import math
+    from ks_gb300 import gsks
+    torch = gpu
+    k, rows = 1024, 400
+    rng = np.random.default_rng(1)
+    s = rng.integers(2 ** 47, 2 ** 48, rows)             # units of 2^-53: 2^-6 .. 2^-5
+    t = int(rng.integers(2 ** 47, 2 ** 48))
+    x = np.empty((rows + 2, k))
+    x[:rows] = (s.astype(float) * 2.0 ** -53)[:, None]
+    x[:rows, 0] = 0.75
+    x[rows] = t * 2.0 ** -53
+    x[rows, 0] = 0.625
+    x[rows + 1] = 2.0 ** -40                             # the point near the origin
+    n2 = lambda c0, c: Fraction(c0) ** 2 + (k - 1) * Fraction(int(c), 2 ** 53) ** 2
+    x2 = np.array([float(n2(0.75, c)) for c in s] + [float(n2(0.625, t)), k * 2.0 ** -80])
+    X, X2 = torch.from_numpy(x).cuda(), torch.from_numpy(x2).cuda()
+    w = torch.tensor([1.0, 0.0], dtype=torch.float64, device="cuda")
+    bm = torch.tensor([rows, rows + 1], dtype=torch.int32, device="cuda")
+    u = torch.zeros(rows, dtype=torch.float64, device="cuda")
+    wm = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    gsks.dgsks_device(gsks.make_kernel(0, scal=-1.0), rows, 2, k, u, None, X, X2, None, X, X2, bm, w, wm, nxa=rows + 2,
+                      nxb=rows + 2)
+    torch.cuda.synchronize()
+    d2 = [Fraction(1, 64) + (k - 1) * Fraction(int(c) - t, 2 ** 53) ** 2 for c in s]
+    err = max(abs(float(u.cpu()[i]) / math.exp(-float(d2[i])) - 1.0) for i in range(rows))
+    assert err <= 2.0 ** -47 + 2.0 ** -50 + 8 * 2.0 ** -53, err / 2.0 ** -53
