@@ -195,8 +195,8 @@ int gsks_split_stats(long long *rechecked_pairs, int *rescued_rows);
  * no CUDA context). */
 int gsks_host_gather_on_device(void);
 
-/* Test hook of the split-precision form (no counterpart in the reference).
- * Sets, for the calling thread's later split-precision calls (dgsks,
+/* Test hook of the tensor-core kernels (no counterpart in the reference).
+ * Sets, for the calling thread's later calls in either precision (dgsks,
  * dgsks_status, gsks_dgsks_device, dgsks_list, ...), the limit of the
  * kernel's bounded waits in clock cycles (wait_cycles <= 0: the library's
  * limit, about 2 s) and, with stall != 0, makes the bulk-copy role of every

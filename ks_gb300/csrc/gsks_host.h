@@ -133,6 +133,11 @@ int sliced_list_run(const SlicedListPlan &P, Ctx *c, const double *XA, const dou
                     const double *XB, const double *XB2, const int *b_idx, int nxb, const double *w, const int *w_idx,
                     double *partial, int *err, cudaStream_t s, int *launches);
 
+// Test hook (gsks_split_test_wait), per host thread: the wait limit in clock cycles (0: the
+// default) and the producers' stall of both tensor-core forms.
+extern thread_local long long tl_split_wait;
+extern thread_local int tl_split_stall;
+
 // Split-precision form (gsks_split.cu).  nrhs <= 4 interleaved columns of u
 // and w in one sweep; GSKS_ERR_TOO_LARGE when k or the shared memory of that
 // sweep does not fit (the caller then sweeps once per column).

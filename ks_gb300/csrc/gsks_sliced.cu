@@ -120,7 +120,8 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   a.ldp = ldp;
   a.err = p.err;
   a.next_item = p.next_item;
-  a.wait_limit = WAIT_LIMIT;
+  a.wait_limit = tl_split_wait > 0 ? tl_split_wait : WAIT_LIMIT;
+  a.stall = tl_split_stall;
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_tiles(a, std::min(ntm * nsc, sms), nr, s);
   if (stream_ordered_alloc) cudaFreeAsync(ws, s);

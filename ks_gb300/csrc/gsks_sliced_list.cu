@@ -168,7 +168,8 @@ int sliced_list_run(const SlicedListPlan &Pl, Ctx *c, const double *XA, const do
   a.partial = partial;
   a.err = err;
   a.next_item = p.next_item;
-  a.wait_limit = WAIT_LIMIT;
+  a.wait_limit = tl_split_wait > 0 ? tl_split_wait : WAIT_LIMIT;
+  a.stall = tl_split_stall;
   a.tp = tp;
   if (e == cudaSuccess) e = cudaGetLastError();
   int kernels = 0;

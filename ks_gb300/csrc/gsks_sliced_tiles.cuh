@@ -550,6 +550,7 @@ struct TileArgs {
   int ldp;
   int *err, *next_item;
   long long wait_limit;
+  int stall;                        // test hook: the producer issues nothing (the waits run out)
   // list form
   const Item *tab;
   int ntab;
@@ -1011,7 +1012,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
 
   if (warp == 0) {
     // ---------------- producer ----------------
-    if (lane == 0) {
+    if (lane == 0 && !a.stall) {
       int g = 0, tt = 0, a_issued = -1;
       int b_last[NSTAGE_RES], m_last[NMETA];
       for (int s = 0; s < NSTAGE_RES; s++) b_last[s] = -1;
@@ -1155,8 +1156,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
     constexpr int SIGN = FRAMED ? -1 : 1;           // W or -W
     const uint32_t tabS = smem_addr(sTab);
     int tbase = 0, tg = 0;                          // tiles before this item, accumulations taken
-    for (int it = 0; !*abort; it++) {
-      if (!mbar_wait(&S->a_full, it & 1, abort, a.wait_limit)) break;
+    // All lanes of a warp go on or none does: a lane that saw another role's abort
+    // while its neighbours' phase completed would leave them at the next vote or load
+    // of tensor memory.
+    auto wait = [&](uint64_t *bar, int parity) {
+      return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort, a.wait_limit)) != 0;
+    };
+    for (int it = 0;; it++) {
+      if (!wait(&S->a_full, it & 1)) break;
       const int item = ((volatile int *)S->islot)[it & 1];
       if (item < 0) break;
       __syncwarp();
@@ -1181,7 +1188,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
       bool ok = true;
       for (int tj = t0 + half; tj < t1; tj += HALVES) {
         const int tt = tbase + tj - t0, ms = tt % NMETA;
-        if (!mbar_wait(&S->m_full[ms], (tt / NMETA) & 1, abort, a.wait_limit)) { ok = false; break; }
+        if (!wait(&S->m_full[ms], (tt / NMETA) & 1)) { ok = false; break; }
         const ColMeta *cm = (const ColMeta *)(sMeta + ms * L.meta);
         const uint32_t cmS = smem_addr(cm) + c0 * 8;   // the group's first column
         // Accumulators -> W (the fixed form: y = A + B - W), four columns at a
@@ -1189,7 +1196,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
         long long W[COLS];
         const int ngr = STREAM ? a.kpad / KRES : 1;
         for (int c = 0; c < ngr; c++, tg++) {
-          if (!mbar_wait(&S->t_full[half], tg & 1, abort, a.wait_limit)) { ok = false; break; }
+          if (!wait(&S->t_full[half], tg & 1)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int q = 0; q < COLS; q += 4) {
@@ -1258,11 +1265,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
         // and arrives on r_empty
         const int rb = it & 1, ru = it >> 1;   // slot, and its earlier uses
         if (grp > 0) {
-          if (ru > 0 && !mbar_wait(&S->r_empty[rb], (ru - 1) & 1, abort, a.wait_limit)) break;
+          if (ru > 0 && !wait(&S->r_empty[rb], (ru - 1) & 1)) break;
           S->rsum[rb][grp - 1][row] = racc[0];
           mbar_arrive(&S->r_full[rb]);
         } else {
-          if (!mbar_wait(&S->r_full[rb], ru & 1, abort, a.wait_limit)) break;
+          if (!wait(&S->r_full[rb], ru & 1)) break;
           double s = racc[0];
           for (int q = 0; q < GROUPS - 1; q++) s += S->rsum[rb][q][row];
           mbar_arrive(&S->r_empty[rb]);

@@ -3345,7 +3345,7 @@ extern "C" int gsks_split_stats(long long *rechecked_pairs, int *rescued_rows)
 }
 
 // Test hook (gsks.h): the wait limit and the producer stall of this thread's
-// later split-precision calls.
+// later calls.
 extern "C" int gsks_split_test_wait(long long wait_cycles, int stall)
 {
   tl_split_wait = wait_cycles > 0 ? wait_cycles : 0;

@@ -135,7 +135,7 @@ def host_gather_on_device() -> bool:
 
 def split_test_wait(wait_cycles: int = 0, stall: bool = False) -> None:
     """Test hook: bounded-wait limit (clock cycles, 0 = default) and producer
-    stall of this thread's later split-precision calls (gsks.h)."""
+    stall of this thread's later calls on the tensor cores (gsks.h)."""
     load().gsks_split_test_wait(C.c_longlong(int(wait_cycles)), C.c_int(1 if stall else 0))
 
 
