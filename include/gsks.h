@@ -50,9 +50,13 @@ const char *gsks_error_string(int code);
 
 /* ---- precision --------------------------------------------------------- */
 enum {
-  GSKS_FP64 = 0,        /* FP64: exact digit products on the tensor cores up
-                           to k = 1024 (DFMA beyond), kernel function in
-                           FP64 or 64-bit integers, FP64 sums               */
+  GSKS_FP64 = 0,        /* FP64: digit products on the tensor cores up to
+                           k = 1024 (DFMA beyond), kernel function in FP64
+                           or 64-bit integers, FP64 sums.  x.y is off by a
+                           few units of 2^-53 sum |x_p y_p|, also where the
+                           coordinates of a point differ widely in size
+                           (such pairs are formed by DFMA), distances by a
+                           few units of 2^-53 (|x|^2 + |y|^2)               */
   GSKS_SPLIT_BF16X3 = 1 /* split-precision tensor-core form.  (The name is
                            kept for compatibility: each coordinate is split
                            into three 16-bit slices, an integer head exact in

@@ -17,13 +17,19 @@ constexpr int KRES = 64;             // largest padded k of the target-resident 
 constexpr int KST = 32;              // k-chunk of one streamed stage beyond it
 constexpr int KMAX = 1024;           // largest padded k
 constexpr int RMAX = 4;              // right-hand sides of one sweep
-constexpr int EFLAG = 1 << 20;       // exponent of a point whose inner products are formed directly
 constexpr int ELIM = 450;            // largest magnitude of a sliced point's exponent
+// A point's exponent word where x.y goes through FP64 (dot_cols): the exponent plus
+// EBIAS (twice of which leaves a double's high word unchanged), what the point's digits
+// do not promise for its inner products (held_bits), and the class of its length.
+constexpr int EBIAS = 2048;
+constexpr int NOT_COARSE = 1 << 20, NOT_LARGE = 1 << 21, NOT_DENSE = 1 << 22;
+constexpr int NOT_HELD = NOT_COARSE | NOT_LARGE | NOT_DENSE;   // also of a point without digits
+constexpr int ECLASS = 24;
 constexpr int ETAB = 2048;           // entries of the 2^-f table
 
 // Metadata of a source tile, one block of shared memory: the norms (FP64, or
-// the integers of the fixed-point Gaussian), bandwidths, exponents, whether the
-// tile holds a point with EFLAG, and the weight columns.
+// the integers of the fixed-point Gaussian), bandwidths, exponents,
+// what the digits of all its points do not promise (NOT_HELD's bits), and the weight columns.
 struct ColMeta {
   double bb[BN];
   uint64_t hj[BN];      // FP64 bits, or (fixed-point form) the mantissa

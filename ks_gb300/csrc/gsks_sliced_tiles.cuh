@@ -11,7 +11,7 @@
 //   x_p = 2^e (d0 2^-8 + d1 2^-17 + ... + d5 2^-53),  e the row's exponent,
 //         six balanced digits |d| <= 256, stored as FP16 integers (the
 //         row's largest coordinate is held to its last bit, every other one to
-//         2^-54 of 2^e);
+//         2^-54 of 2^e: held_bits says where that is not enough);
 //   the products of digits i and j, i + j = l <= 6, are integers; their sums
 //         over 64 coordinates stay within 2^24 and are exact in the FP32
 //         accumulator of level l up to 3 (beyond, rows of nothing but extreme
@@ -380,12 +380,55 @@ __device__ __forceinline__ void slice8(const double (&v)[8], int e, bool live, u
   }
 }
 
+// What decides how well a point's digits hold its inner products (x.y of the kernels
+// without norms).  With x_p = xi_p 2^e the error of W is about 2^-54 of 2^(e_i + e_j)
+// (|xi|^2 + |eta|^2)^1/2, rms: nothing beside sum |x_p y_p| of ordinary points, all of it
+// where the large coordinates of one point meet zeros or small ones of the other
+// ((1e20, 1) and (1e-20, 1)).  Sound without a look at W are pairs of
+//   coarse points: 26 bits below 2^e (three digits) hold every coordinate; W is exact;
+//   large ones (k up to 128: one or two roundings to W's unit): every coordinate that is
+//     not 0 is at least 2^-3, so that |xi_p eta_p| >= 2^-6 for each p that both have;
+//   dense ones: three quarters of the coordinates or more are at least 2^-5, so that half
+//     of them are in both points.
+// Of other pairs dot_cols forms those with a small W directly: |W| < 2^-4 2^c, c the larger
+// class, 2^c >= |xi| (and the share of W's own roundings in long rows).
+struct HeldStat {
+  int large3, large5;       // coordinates of at least 2^-3, 2^-5
+  int count;                // that are not 0
+  int sq;                   // |xi|^2 2^16, rounded down
+  int fine;                 // one needs more than 26 bits
+};
+__device__ __forceinline__ void held_stat(const double (&v)[8], int e, HeldStat &t)
+{
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const uint64_t b = (uint64_t)__double_as_longlong(v[q]) & 0x7fffffffffffffffull;
+    const uint64_t M = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+    const int sh = e + 1022 - (int)(b >> 52);          // 0 and more; xi = M 2^-(53 + sh)
+    const int top = sh < 8 ? (int)(M >> (45 + sh)) : 0;
+    t.large3 += sh < 3;
+    t.large5 += sh < 5;
+    t.count += b != 0;
+    t.sq += top * top;
+    t.fine |= b != 0 && (sh > 25 || (M & ((1ull << (27 + sh)) - 1)) != 0);
+  }
+}
+// The bits and class of a point's exponent word.
+__device__ __forceinline__ int held_bits(const HeldStat &t, int k, int kpad)
+{
+  int c = t.sq <= 1 << 16 ? 0 : (17 - __clz(t.sq - 1)) / 2;            // 4^c >= |xi|^2
+  c = max(c, kpad > 512 ? 3 : kpad > 256 ? 1 : 0);
+  return (t.fine ? NOT_COARSE : 0) | (t.large3 < t.count || kpad > 128 ? NOT_LARGE : 0) |
+         (4 * t.large5 < 3 * k ? NOT_DENSE : 0) | c << ECLASS;
+}
+
 // One block per 32 points: lane = point, each warp a group of eight coordinates
 // (then every eighth one; the list form's blocks have no more warps than groups).  Reads 64 bytes a thread, writes 16-byte row
 // segments, consecutive points side by side (512 contiguous bytes a warp).
 static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
 {
   __shared__ uint32_t s_max[8][32];
+  __shared__ HeldStat s_held[8][32];
   __shared__ CallParam s_cp;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int nbA = a.nta * (BM / 32);
@@ -482,12 +525,15 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
   }
   uint8_t *base = side ? a.imgB + (size_t)tile * btile_bytes(a.kpad, a.nr) : a.imgA + (size_t)tile * op_bytes(BM, a.kpad);
   const bool once = kgs <= nw;             // each thread's only group is still in registers
+  const bool dots = !kt_uses_norms(kt);
+  HeldStat held{};
   for (int kg = wp; kg < kgs; kg += nw) {
     if (!once) load8(kg, v);
     if (fixed) {
 #pragma unroll
       for (int q = 0; q < 8; q++) v[q] *= mul;
     }
+    if (dots) held_stat(v, e, held);
     uint4 out[NS];
     slice8(v, e, !flag, out);
     const int c = kg / gpc, kgc = kg - c * gpc;
@@ -498,8 +544,20 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     for (int s = 0; s < NS; s++) *(uint4 *)(dst + s * step) = out[s];
   }
 
+  if (dots) {
+    s_held[wp][lane] = held;
+    __syncthreads();
+  }
   if (wp == 0) {
-    const bool norms = kt_uses_norms(kt), varbw = kt == KS_GAUSSIAN_VAR_BANDWIDTH;
+    int bits = flag ? NOT_HELD : 0;
+    if (dots && !flag && mh) {                // (points of zeros only: W is exact)
+      for (int q = 1; q < nw; q++) {
+        const HeldStat &t = s_held[q][lane];
+        held.large3 += t.large3; held.large5 += t.large5; held.count += t.count; held.sq += t.sq; held.fine |= t.fine;
+      }
+      bits = held_bits(held, a.k, a.kpad);
+    }
+    const bool norms = !dots, varbw = kt == KS_GAUSSIAN_VAR_BANDWIDTH;
     double nn = (valid && norms) ? (side ? a.XB2[p] : a.XA2[p]) : 0.0;
     if (fixed) {
       const double y = fma(nn, s_cp.ah, nn * s_cp.al) * ldexp(1.0, s_cp.F);
@@ -518,15 +576,15 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     if (!side) {
       a.row_aa[slot] = nn;
       a.row_hi[slot] = hb;
-      a.row_e[slot] = flag ? EFLAG : e;
+      a.row_e[slot] = fixed ? e : (e + EBIAS) | bits;
       if (a.row_n) a.row_n[slot] = 0;
     } else {
       ColMeta *cm = (ColMeta *)(base + op_bytes(BN, a.kpad));
       cm->bb[r] = nn;
       cm->hj[r] = hb;
-      cm->e[r] = flag ? EFLAG : e;
-      const bool any = __any_sync(0xffffffffu, flag);
-      if (lane == 0) { cm->flag = any ? 1 : 0; cm->pad[0] = cm->pad[1] = cm->pad[2] = 0; }
+      cm->e[r] = fixed ? e : (e + EBIAS) | bits;
+      const int any = (int)__reduce_or_sync(0xffffffffu, (unsigned)bits) & NOT_HELD;
+      if (lane == 0) { cm->flag = any; cm->pad[0] = cm->pad[1] = cm->pad[2] = 0; }
       const size_t wi = valid ? (size_t)(a.wmap ? a.wmap[pt] : pt) * a.nrhs : 0;
       for (int q = 0; q < a.nr; q++) cm->w[q][r] = (valid && q < a.nrhs) ? a.w[wi + q] : 0.0;
     }
@@ -539,7 +597,7 @@ struct TileArgs {
   int ntm, ntn, nsc, chunk_tiles;   // items = ntm * nsc, chunk_tiles source tiles each
   const uint8_t *imgA, *imgB;
   const double *row_aa; const uint64_t *row_hi; const int *row_e;
-  const double *XA, *XB;            // pools and maps, for the points with EFLAG
+  const double *XA, *XB;            // pools and maps, for pairs formed directly
   const int *amap, *bmap;
   int nxa, nxb;
   KParams kp;
@@ -665,6 +723,37 @@ static __device__ __noinline__ double dot_direct(const double *__restrict__ x, c
   double s = 0.0;
   for (int p = 0; p < k; p++) s = fma(x[p], y[p], s);
   return s;
+}
+// x.y of a row with two others, in the order of the DFMA kernels, eight coordinates' loads at
+// a time (each lane has rows of its own: whole 32-byte sectors).
+static __device__ __noinline__ double2 dot_direct2(const double *__restrict__ x, const double *__restrict__ y0,
+                                                   const double *__restrict__ y1, int k)
+{
+  double s0 = 0.0, s1 = 0.0;
+  int p = 0;
+  if ((k & 1) == 0 && (((uintptr_t)x | (uintptr_t)y0 | (uintptr_t)y1) & 15) == 0) {
+    for (; p + 8 <= k; p += 8) {
+      double2 a[4], b[4], c[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        a[q] = __ldg((const double2 *)(x + p) + q);
+        b[q] = __ldg((const double2 *)(y0 + p) + q);
+        c[q] = __ldg((const double2 *)(y1 + p) + q);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        s0 = fma(a[q].y, b[q].y, fma(a[q].x, b[q].x, s0));
+        s1 = fma(a[q].y, c[q].y, fma(a[q].x, c[q].x, s1));
+      }
+    }
+  }
+#pragma unroll 4
+  for (; p < k; p++) {
+    const double v = __ldg(x + p);
+    s0 = fma(v, __ldg(y0 + p), s0);
+    s1 = fma(v, __ldg(y1 + p), s1);
+  }
+  return make_double2(s0, s1);
 }
 
 // |x_i - y_j|^2 from the pool coordinates.  For points that agree to about
@@ -910,26 +999,111 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp,
   }
 }
 
-// One thread's columns of a tile through x.y in FP64; W holds SIGN W.  slow: a
-// point of the row or of the tile has no digits (EFLAG).
+// A call's copy of kvalue, for the pairs formed directly.
+template <int KT>
+__device__ __noinline__ double kvalue_call(const TileArgs &a, const KParams &kp, double dot)
+{
+  return kvalue<KT>(a, kp, 0, dot, RowMeta{}, 0.0, 0.0, 0.0, 0);
+}
+
+// The columns that dot_cols left (a bit each; the whole warp calls).  Few pairs among the
+// lanes: four at a time, each by eight lanes, since a lane on its own waits for its loads at
+// every eighth coordinate (one point of a 65536-point tile row held its warp, and with it
+// the tile, for 20 000 cycles a tile).  Many: each lane its own, two at a time.
+template <int KT, int NR>
+__device__ __noinline__ void direct_cols(const TileArgs &a, const KParams &kp, int i, const ColMeta *cm, int c0,
+                                         int j0, uint32_t direct, double (&sum)[NR])
+{
+  const unsigned full = 0xffffffffu;
+  const int total = (int)__reduce_add_sync(full, __popc(direct));
+  if (total == 0) return;
+  const int trips = ((int)__reduce_max_sync(full, __popc(direct)) + 1) / 2;
+  const double *x = a.XA + (direct ? (size_t)pool_clamp(a.amap, i, a.nxa) * a.k : 0);
+  if (total > trips * min(32, 4 + a.k / 4)) {
+    while (direct) {
+      const int ca = __ffs(direct) - 1;
+      direct &= direct - 1;
+      const int cb = direct ? __ffs(direct) - 1 : -1;
+      direct &= direct - 1;
+      const double *y0 = a.XB + (size_t)pool_clamp(a.bmap, j0 + ca, a.nxb) * a.k;
+      const double *y1 = cb < 0 ? y0 : a.XB + (size_t)pool_clamp(a.bmap, j0 + cb, a.nxb) * a.k;
+      const double2 dot = dot_direct2(x, y0, y1, a.k);
+      const double ka = kvalue_call<KT>(a, kp, dot.x), kb = cb < 0 ? 0.0 : kvalue_call<KT>(a, kp, dot.y);
+#pragma unroll
+      for (int r = 0; r < NR; r++) {
+        if (r > 0 && r >= a.nrhs) continue;
+        sum[r] = fma(ka, cm->w[r][c0 + ca], sum[r]);
+        if (cb >= 0) sum[r] = fma(kb, cm->w[r][c0 + cb], sum[r]);
+      }
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  for (int left = total; left > 0; left -= 4) {
+    int src = 0, col = 0, mine[4];               // my group's pair; my own pairs, by group
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const unsigned b = __ballot_sync(full, direct != 0);
+      const int l = b ? __ffs(b) - 1 : 0, c = __shfl_sync(full, __ffs(direct) - 1, l);
+      mine[g] = b && lane == l ? c : -1;
+      if (b && lane == l) direct &= direct - 1;
+      if (g == lane >> 3) { src = l; col = b ? c : -1; }
+    }
+    const double *xs = (const double *)__shfl_sync(full, (unsigned long long)x, src);
+    double s = 0.0;
+    if (col >= 0) {
+      const double *y = a.XB + (size_t)pool_clamp(a.bmap, j0 + col, a.nxb) * a.k;
+#pragma unroll 8
+      for (int p = sub; p < a.k; p += 8) s = fma(__ldg(xs + p), __ldg(y + p), s);
+    }
+#pragma unroll
+    for (int d = 4; d; d >>= 1) s += __shfl_xor_sync(full, s, d);
+    const double kv = kvalue_call<KT>(a, kp, s);
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const double kg = __shfl_sync(full, kv, 8 * g);
+      if (mine[g] < 0) continue;
+#pragma unroll
+      for (int r = 0; r < NR; r++)
+        if (r == 0 || r < a.nrhs) sum[r] = fma(kg, cm->w[r][c0 + mine[g]], sum[r]);
+    }
+  }
+}
+
+// One thread's columns of a tile through x.y in FP64; W holds SIGN W.  slow: the digits
+// of the rows and of the tile's points do not promise every x.y (NOT_HELD).  A pair of a
+// point without digits is formed directly; for the kernels without norms, pairs whose W is
+// too small for their digits are left to direct_cols.
 template <int KT, int NR, int SIGN>
 __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, const long long (&W)[COLS],
                                          const RowMeta &am, const ColMeta *cm, int c0, const Place &P, int gb, bool slow,
                                          uint32_t tab, double (&sum)[NR])
 {
+  constexpr bool DOTS = !kt_uses_norms(KT);
   double cfold = 0.0;
   if (KT == KS_GAUSSIAN) cfold = -kp.scal * (1.4426950408889634 * 0x1p53);
   if (KT == KS_GAUSSIAN_VAR_BANDWIDTH) cfold = am.hi * (0.5 * 1.4426950408889634 * 0x1p53);
+  uint32_t direct = 0;
+  if (DOTS && slow && am.i >= 0) {
+#pragma unroll
+    for (int c = 0; c < COLS; c++) {
+      const int ej = cm->e[c0 + c];
+      // (a point without digits: W = 0)
+      const int lim = 1 << (16 + gb + (max(am.e, ej) >> ECLASS));          // 2^-4 2^class, high word
+      if (c < P.nv && ((am.e | ej) & NOT_HELD) == NOT_HELD &&
+          (uint32_t)((int)(W[c] >> 32) + lim) < 2u * (uint32_t)lim)
+        direct |= 1u << c;
+    }
+  }
 #pragma unroll
   for (int c = 0; c < COLS; c++) {
-    if (c < P.nv) {
+    if (c < P.nv && (!DOTS || !(direct >> c & 1u))) {
       const int ej = cm->e[c0 + c], j = P.j0 + c;
       double dot = to_double(SIGN * W[c]);
-      dot = __hiloint2double(__double2hiint(dot) + (W[c] != 0 ? (am.e + ej - 52 - gb) << 20 : 0), __double2loint(dot));
-      if (slow && (am.e == EFLAG || ej == EFLAG) && am.i >= 0) {
-        int pa = a.amap ? a.amap[am.i] : am.i, pb = a.bmap ? a.bmap[j] : j;
-        if (a.nxa >= 0 && (pa < 0 || pa >= a.nxa)) pa = 0;   // flagged by slice_kernel
-        if (a.nxb >= 0 && (pb < 0 || pb >= a.nxb)) pb = 0;
+      dot = __hiloint2double(__double2hiint(dot) + (W[c] != 0 ? (int)((uint32_t)(am.e + ej - 52 - gb) << 20) : 0),
+                             __double2loint(dot));
+      if (!DOTS && slow && ((am.e | ej) & NOT_HELD) == NOT_HELD && am.i >= 0) {
+        const int pa = pool_clamp(a.amap, am.i, a.nxa), pb = pool_clamp(a.bmap, j, a.nxb);   // flagged by slice_kernel
         dot = dot_direct(a.XA + (size_t)pa * a.k, a.XB + (size_t)pb * a.k, a.k);
       }
       const double kv = kvalue<KT>(a, kp, j, dot, am, cm->bb[c0 + c],
@@ -938,6 +1112,14 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
       for (int r = 0; r < NR; r++)
         if (r == 0 || r < a.nrhs) sum[r] = fma(kv, cm->w[r][c0 + c], sum[r]);
     }
+  }
+  if (DOTS && slow) {
+    double t[NR];           // (of its own: sum stays in registers)
+#pragma unroll
+    for (int r = 0; r < NR; r++) t[r] = sum[r];
+    direct_cols<KT, NR>(a, kp, am.i, cm, c0, P.j0, direct, t);
+#pragma unroll
+    for (int r = 0; r < NR; r++) sum[r] = t[r];
   }
 }
 
@@ -1181,7 +1363,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
       const uint32_t bias = combine_bias<SIGN>(gb);
       const ExpFrame E = KT == KS_GAUSSIAN ? exp_frame(max(fixed ? cp.F : 43, 43), tabS) : exp_frame52(tabS);
       const long long arow = __double_as_longlong(a.row_aa[i0]);
-      const bool anyrow = __any_sync(0xffffffffu, a.row_e[i0] == EFLAG);
+      const int unheld = (int)__reduce_or_sync(0xffffffffu, (unsigned)a.row_e[i0]);
       double racc[NR];
 #pragma unroll
       for (int r = 0; r < NR; r++) racc[r] = 0.0;
@@ -1234,7 +1416,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
         } else {
           const Place P = place_of<LISTED>(a, item, row, tj, c0);
           const RowMeta am{__longlong_as_double(arow), __longlong_as_double((long long)a.row_hi[i0]), a.row_e[i0], P.i};
-          const bool slow = anyrow || cm->flag != 0;
+          const bool slow = ((unheld | cm->flag) & NOT_HELD) == NOT_HELD;
           dot_cols<KT, NR, SIGN>(a, kp, W, am, cm, c0, P, gb, slow, tabS, tsum);
         }
 #pragma unroll
