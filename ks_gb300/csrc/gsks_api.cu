@@ -91,6 +91,9 @@ Ctx::~Ctx()
   for (PinBuf *b : {&hA, &hA2, &hB, &hB2, &hw, &hu, &hhi, &hhj}) b->release();
   // (memory still in use by enqueued calls outlives the pool's handle)
   if (pool) cudaMemPoolDestroy(pool);
+  if (fork) cudaEventDestroy(fork);
+  if (join) cudaEventDestroy(join);
+  if (side) cudaStreamDestroy(side);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -104,7 +107,10 @@ Ctx *get_ctx()
   if (tl_ctx && tl_ctx->device == dev) return tl_ctx.get();
   std::unique_ptr<Ctx> c(new Ctx);
   c->device = dev;
-  if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) {
+  if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming)) != cudaSuccess) {
     cuda_status(e, "cudaStreamCreate");
     return nullptr;
   }

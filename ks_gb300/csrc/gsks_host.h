@@ -37,6 +37,8 @@ struct PinBuf {
 struct Ctx {
   int device = -1;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;             // a batched call's second branch,
+  cudaEvent_t fork = nullptr, join = nullptr;   // from and back to the call's stream
   int num_sms = 0;
   DevBuf partial, err;
   DevBuf dA, dA2, dB, dB2, dw, du, dhi, dhj, dwork;

@@ -11,17 +11,17 @@ namespace sliced {
 
 static_assert(KS_EPANECHNIKOV < NTYPES, "one work counter per kernel type");
 
-static cudaError_t launch_type(int type, const TileArgs &a, int grid, cudaStream_t s)
+static cudaError_t launch_type(int type, const TileArgs &a, int grid, cudaStream_t s, bool dependent)
 {
   switch (type) {
-    case KS_GAUSSIAN: return launch_g<KS_GAUSSIAN, 1, true>(a, grid, s);
-    case KS_GAUSSIAN_VAR_BANDWIDTH: return launch_g<KS_GAUSSIAN_VAR_BANDWIDTH, 1, true>(a, grid, s);
-    case KS_POLYNOMIAL: return launch_g<KS_POLYNOMIAL, 1, true>(a, grid, s);
-    case KS_LAPLACE: return launch_g<KS_LAPLACE, 1, true>(a, grid, s);
-    case KS_TANH: return launch_g<KS_TANH, 1, true>(a, grid, s);
-    case KS_QUARTIC: return launch_g<KS_QUARTIC, 1, true>(a, grid, s);
-    case KS_MULTIQUADRATIC: return launch_g<KS_MULTIQUADRATIC, 1, true>(a, grid, s);
-    default: return launch_g<KS_EPANECHNIKOV, 1, true>(a, grid, s);
+    case KS_GAUSSIAN: return launch_g<KS_GAUSSIAN, 1, true>(a, grid, s, dependent);
+    case KS_GAUSSIAN_VAR_BANDWIDTH: return launch_g<KS_GAUSSIAN_VAR_BANDWIDTH, 1, true>(a, grid, s, dependent);
+    case KS_POLYNOMIAL: return launch_g<KS_POLYNOMIAL, 1, true>(a, grid, s, dependent);
+    case KS_LAPLACE: return launch_g<KS_LAPLACE, 1, true>(a, grid, s, dependent);
+    case KS_TANH: return launch_g<KS_TANH, 1, true>(a, grid, s, dependent);
+    case KS_QUARTIC: return launch_g<KS_QUARTIC, 1, true>(a, grid, s, dependent);
+    case KS_MULTIQUADRATIC: return launch_g<KS_MULTIQUADRATIC, 1, true>(a, grid, s, dependent);
+    default: return launch_g<KS_EPANECHNIKOV, 1, true>(a, grid, s, dependent);
   }
 }
 
@@ -172,14 +172,26 @@ int sliced_list_run(const SlicedListPlan &Pl, Ctx *c, const double *XA, const do
   a.stall = tl_split_stall;
   a.tp = tp;
   if (e == cudaSuccess) e = cudaGetLastError();
-  int kernels = 0;
+  // Several types: every other one in the thread's second stream, which waits for
+  // slice_kernel by an event, so that each launch follows it in full.
+  int types = 0, kernels = 0;
+  for (int t = 0; t < NTYPES; t++) types += Pl.first[t + 1] > Pl.first[t];
+  const bool fork = types > 1 && e == cudaSuccess;
+  if (fork) {
+    e = cudaEventRecord(c->fork, s);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(c->side, c->fork, 0);
+    if (e != cudaSuccess) return cuda_status(e, "sliced list launch");
+  }
   for (int t = 0; t < NTYPES && e == cudaSuccess; t++) {
     a.ntab = Pl.first[t + 1] - Pl.first[t];
     if (!a.ntab) continue;
     a.tab = (const Item *)(ws + Pl.o_items) + Pl.first[t];
     a.next_item = p.next_item + t;
-    a.later = kernels++ > 0;
-    e = launch_type(t, a, std::min(a.ntab, std::max(1, c->num_sms)), s);
+    e = launch_type(t, a, std::min(a.ntab, std::max(1, c->num_sms)), kernels++ & 1 ? c->side : s, !fork);
+  }
+  if (fork) {   // (after a failed launch too: a capture of s must not end with side left in it)
+    const cudaError_t r = cudaEventRecord(c->join, c->side), w = cudaStreamWaitEvent(s, c->join, 0);
+    if (e == cudaSuccess) e = r != cudaSuccess ? r : w;
   }
   if (e != cudaSuccess) return cuda_status(e, "sliced list launch");
   *launches += 2 + kernels;

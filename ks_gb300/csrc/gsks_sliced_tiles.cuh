@@ -52,9 +52,10 @@
 // row's runs to arrive adds them in run order (deterministic).  Every wait is
 // bounded, as in gsks_split.cu; no wait is on another CTA.  The batched form
 // (LISTED) runs the same kernels over tables of tiles and items from many tasks,
-// each with its own descriptor and frame: one launch per kernel type, each let in
-// as the one before runs out of items.  (One kernel with every type's epilogue
-// spilled 800 bytes a thread and took 1.5 times as long.)
+// each with its own descriptor and frame: one launch per kernel type, in two streams
+// that start after slice_kernel, so that a type's blocks get in as the one's before it in
+// the other stream run out of items.  (One kernel with every type's epilogue spilled 800
+// bytes a thread and took 1.5 times as long.)
 #pragma once
 #include "gsks.h"
 #include "gsks_internal.cuh"
@@ -613,7 +614,6 @@ struct TileArgs {
   const Item *tab;
   int ntab;
   const TaskParam *tp;
-  int later;                        // another type's kernel was launched just before
 };
 
 // Geometry of a work item: target tile, source tiles, list positions of its
@@ -1181,12 +1181,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
   if (warp == 0) { tmem_alloc(&S->tmem_base, TMEM_COLS); tmem_relinquish(); }
   if constexpr (TABLE)
     for (int i = threadIdx.x; i < ETAB; i += NTHREADS) sTab[i] = g_exp_table.v[i];
-  // slice_kernel's results from here on.  The list form launches a kernel per
-  // kernel type, one after another: the later ones (a.later) need not wait for
-  // the earlier, which have waited for slice_kernel before they let them start;
-  // they only end after them.
-  if (!LISTED || !a.later) wait_primary();
-  if (LISTED) launch_dependents();
+  wait_primary();   // slice_kernel's results from here on
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1467,11 +1462,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
   __syncthreads();
   if (*abort && threadIdx.x == 0) atomicOr(a.err, DEVERR_TIMEOUT);
   if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
-  if (LISTED && a.later) wait_primary();
 }
 
+// dependent: slice_kernel is the launch just before this one on s.
 template <int KT, int NR, int G, bool LISTED>
-cudaError_t launch_t(const TileArgs &a, int grid, cudaStream_t s)
+cudaError_t launch_t(const TileArgs &a, int grid, cudaStream_t s, bool dependent)
 {
   const size_t smem = smem_bytes(smem_layout(a.kpad, NR, uses_table(KT)));
   // The attribute is per function and device; raised once to the most any launch takes.
@@ -1484,15 +1479,17 @@ cudaError_t launch_t(const TileArgs &a, int grid, cudaStream_t s)
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) raised[dev] = true;
   }
-  return launch_after(sliced_tiles<KT, NR, G, LISTED>, grid, NTHREADS, smem, s, a);
+  if (dependent) return launch_after(sliced_tiles<KT, NR, G, LISTED>, grid, NTHREADS, smem, s, a);
+  sliced_tiles<KT, NR, G, LISTED><<<grid, NTHREADS, smem, s>>>(a);
+  return cudaGetLastError();
 }
 
 template <int KT, int NR, bool LISTED>
-cudaError_t launch_g(const TileArgs &a, int grid, cudaStream_t s)
+cudaError_t launch_g(const TileArgs &a, int grid, cudaStream_t s, bool dependent = true)
 {
-  if (a.kpad > KRES) return launch_t<KT, NR, -1, LISTED>(a, grid, s);
-  if constexpr (!has_frame(KT)) return launch_t<KT, NR, 3, LISTED>(a, grid, s);
-  else return a.kpad > 32 ? launch_t<KT, NR, 2, LISTED>(a, grid, s) : launch_t<KT, NR, 3, LISTED>(a, grid, s);
+  if (a.kpad > KRES) return launch_t<KT, NR, -1, LISTED>(a, grid, s, dependent);
+  if constexpr (!has_frame(KT)) return launch_t<KT, NR, 3, LISTED>(a, grid, s, dependent);
+  else return a.kpad > 32 ? launch_t<KT, NR, 2, LISTED>(a, grid, s, dependent) : launch_t<KT, NR, 3, LISTED>(a, grid, s, dependent);
 }
 
 }  // namespace sliced
