@@ -65,7 +65,11 @@ bool DevBuf::ensure(size_t bytes)
   if (bytes <= cap) return true;
   if (p) { cudaFree(p); p = nullptr; cap = 0; }
   size_t want = std::max<size_t>(bytes + bytes / 4, 256);
-  if (cudaMalloc(&p, want) != cudaSuccess) { p = nullptr; return false; }
+  if (cudaMalloc(&p, want) != cudaSuccess && cudaMalloc(&p, want = bytes) != cudaSuccess) {
+    p = nullptr;
+    cudaGetLastError();   // the caller's to report, or to do without
+    return false;
+  }
   cap = want;
   return true;
 }
@@ -120,8 +124,6 @@ Ctx *get_ctx()
   tl_ctx = std::move(c);
   return tl_ctx.get();
 }
-
-constexpr unsigned long long POOL_KEEP = 512ull << 20;
 
 cudaError_t stream_alloc(Ctx *c, void **p, size_t bytes, cudaStream_t s)
 {
@@ -447,9 +449,12 @@ int enqueue_fused(Ctx *c, const ks_t *ker, int m, int n, int k,
     return enqueue_split(c, ker, m, n, k, u, umap, XA, XA2, amap, nxa, XB, XB2, bmap, nxb,
                          w, wmap, hi, hj, s, stream_ordered_alloc, std::max(nrhs, 1));
   if (precision != GSKS_FP64) return GSKS_ERR_PRECISION;
-  if (sliced_takes(k))
-    return enqueue_sliced(c, ker, m, n, k, u, umap, XA, XA2, amap, nxa, XB, XB2, bmap, nxb,
-                          w, wmap, hi, hj, s, stream_ordered_alloc, std::max(nrhs, 1));
+  if (sliced_takes(k)) {
+    const int st = enqueue_sliced(c, ker, m, n, k, u, umap, XA, XA2, amap, nxa, XB, XB2, bmap, nxb,
+                                  w, wmap, hi, hj, s, stream_ordered_alloc, std::max(nrhs, 1));
+    // (no room for the digits, 12 bytes a coordinate: the DFMA kernels need none)
+    if (st != GSKS_ERR_ALLOC) return st;
+  }
 
   Fp64Plan p = fp64_plan(m, n, k, c->num_sms);
   const size_t pbytes = p.partial_elems * sizeof(double) * (size_t)std::max(nrhs, 1);

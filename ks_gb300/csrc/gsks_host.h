@@ -77,11 +77,12 @@ struct Staged {
 };
 
 Ctx *get_ctx();
-// Workspace of one asynchronous call on stream s, released by cudaFreeAsync on s.
-// It comes from the thread's own pool, which keeps up to POOL_KEEP bytes between
-// calls (the device's default pool gives its memory back at every
-// synchronisation: 200 us and more to map it again for the next call) and goes
-// with the thread's context.
+// Workspace of one call on stream s, released by cudaFreeAsync on s.  It comes from
+// the thread's own pool, which keeps up to POOL_KEEP bytes between calls (the device's
+// default pool gives its memory back at every synchronisation: 200 us and more to map it
+// again for the next call) and goes with the thread's context.  Of a larger workspace the
+// rest is given back at the next synchronisation and mapped again by the next call.
+constexpr size_t POOL_KEEP = 512ull << 20;
 cudaError_t stream_alloc(Ctx *c, void **p, size_t bytes, cudaStream_t s);
 int set_status(int s, const char *where);
 int cuda_status(cudaError_t e, const char *where);
@@ -109,6 +110,7 @@ int enqueue_fused(Ctx *c, const ks_t *ker, int m, int n, int k,
 
 // FP64 form on the tensor cores (gsks_sliced.cu), for k up to 1024
 // (sliced_takes); nrhs <= 4 interleaved columns of u and w in one sweep.
+// GSKS_ERR_ALLOC, with nothing enqueued, where the workspace cannot be had.
 bool sliced_takes(int k);
 int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k,
                    double *u, const int *umap,
@@ -121,6 +123,7 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k,
 // (task t, target position r, source chunk sc) into partial[pbase[t] + sc * m_t
 // + r].  kps: ntask device-side descriptors; hoff_a / hoff_b: host offsets.
 // sliced_list_run takes device pointers and only launches kernels.
+// sliced_list_plan: GSKS_ERR_ALLOC, with P.ws empty, where the workspace cannot be had.
 struct SlicedListPlan {
   int ntask = 0, k = 0, kpad = 0, n_ta = 0, n_tb = 0, n_items = 0;
   bool any_frame = false;

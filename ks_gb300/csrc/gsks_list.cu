@@ -241,26 +241,29 @@ int list_plan_build(ListPlan &L, Ctx *c, ks_t *kernel, ks_t *kernels, int ntask,
     if (flags & DEVERR_MAP_RANGE) return GSKS_ERR_MAP_RANGE;
   }
 
-  // ---- work items, largest first ----------------------------------------
+  // ---- partial sums, work items -------------------------------------------
   std::vector<ListTask> tasks(ntask);
-  std::vector<ListItem> items;
   long long pbase = 0;
   for (int t = 0; t < ntask; t++) {
     const int m = hoff_a[t + 1] - hoff_a[t], n = hoff_b[t + 1] - hoff_b[t];
     const int nsc = (m > 0 && n > 0) ? (n + LIST_CHUNK - 1) / LIST_CHUNK : 0;
     tasks[t] = ListTask{pbase, m, nsc};
-    if (L.split || L.sliced) { pbase += (long long)nsc * m; continue; }   // these plan their own items
-    for (int sc = 0; sc < nsc; sc++)
-      for (int i0 = 0; i0 < m; i0 += fp64cfg::BM) {
-        ListItem it{};
-        it.task = t; it.a0 = hoff_a[t] + i0; it.rows = std::min(fp64cfg::BM, m - i0);
-        it.b0 = hoff_b[t] + sc * LIST_CHUNK; it.cols = std::min(LIST_CHUNK, n - sc * LIST_CHUNK);
-        it.out = pbase + (long long)sc * m + i0;
-        items.push_back(it);
-      }
     pbase += (long long)nsc * m;
   }
-  {
+  // The DFMA form's items, largest first (the other forms plan their own).
+  std::vector<ListItem> items;
+  auto dfma_items = [&] {
+    for (int t = 0; t < ntask; t++) {
+      const int m = tasks[t].m, n = hoff_b[t + 1] - hoff_b[t];
+      for (int sc = 0; sc < tasks[t].nsc; sc++)
+        for (int i0 = 0; i0 < m; i0 += fp64cfg::BM) {
+          ListItem it{};
+          it.task = t; it.a0 = hoff_a[t] + i0; it.rows = std::min(fp64cfg::BM, m - i0);
+          it.b0 = hoff_b[t] + sc * LIST_CHUNK; it.cols = std::min(LIST_CHUNK, n - sc * LIST_CHUNK);
+          it.out = tasks[t].pbase + (long long)sc * m + i0;
+          items.push_back(it);
+        }
+    }
     // largest rows x cols first, ties in build order: a counting sort (the
     // products are bounded by the tile height times the source chunk)
     int cmax = 0;
@@ -271,10 +274,12 @@ int list_plan_build(ListPlan &L, Ctx *c, ks_t *kernel, ks_t *kernels, int ntask,
     std::vector<ListItem> sorted(items.size());
     for (const ListItem &it : items) sorted[start[cmax - it.rows * it.cols]++] = it;
     items.swap(sorted);
-  }
+    L.nitems = (int)items.size();
+    return upload(L.items, items.data(), items.size(), s);
+  };
   L.pbase = pbase;
-  L.nitems = (int)items.size();
-  bool ok = (L.split || L.sliced || upload(L.items, items.data(), items.size(), s)) &&
+  L.nitems = 0;
+  bool ok = (L.split || L.sliced || dfma_items()) &&
             upload(L.tasks, tasks.data(), tasks.size(), s) && upload(L.kps, kps.data(), kps.size(), s) &&
             upload(L.a_off, hoff_a.data(), (size_t)ntask + 1, s) &&
             L.partial.ensure(std::max<long long>(pbase, 1) * sizeof(double)) && L.counter.ensure(2 * sizeof(int)) &&
@@ -293,10 +298,16 @@ int list_plan_build(ListPlan &L, Ctx *c, ks_t *kernel, ks_t *kernels, int ntask,
     std::vector<KParams> kpt(ntask);
     std::vector<long long> pb(ntask);
     for (int t = 0; t < ntask; t++) { kpt[t] = kps[kernels ? t : 0]; pb[t] = tasks[t].pbase; }
-    const int st = L.split ? split_list_plan(L.sp, kpt.data(), ntask, k, hoff_a.data(), hoff_b.data(), pb.data(),
-                                             LIST_CHUNK, nxa, nxb, same_pool, s)
-                           : sliced_list_plan(L.lp, kpt.data(), ntask, k, hoff_a.data(), hoff_b.data(), pb.data(),
-                                              LIST_CHUNK, s);
+    int st = L.split ? split_list_plan(L.sp, kpt.data(), ntask, k, hoff_a.data(), hoff_b.data(), pb.data(),
+                                       LIST_CHUNK, nxa, nxb, same_pool, s)
+                     : sliced_list_plan(L.lp, kpt.data(), ntask, k, hoff_a.data(), hoff_b.data(), pb.data(),
+                                        LIST_CHUNK, s);
+    if (st == GSKS_ERR_ALLOC && L.sliced) {
+      // (no room for the digits, 12 bytes a coordinate and list position: the DFMA
+      // kernels need none)
+      L.sliced = false;
+      st = dfma_items() ? GSKS_OK : GSKS_ERR_ALLOC;
+    }
     if (st) return st;
   }
   // the host vectors above die here: every copy from them must have left
@@ -431,6 +442,8 @@ extern "C" int dgsks_list(ks_t *kernel, ks_t *kernels, int ntask, int k,
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e, "dgsks_list copy back");
   }
+  // (kept for the next call, but no large one)
+  if (B.plan.lp.ws.cap > POOL_KEEP) B.plan.lp.ws.release();
   note_launches(launches);
   return set_status(GSKS_OK, nullptr);
 }

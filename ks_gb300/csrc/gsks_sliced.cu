@@ -73,8 +73,14 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   const int nparts = nr > 1 ? nsc * GROUPS : nsc;          // partials per row and column
   const size_t total = o_p + al((size_t)nrhs * nparts * ldp * 8);
   uint8_t *ws = nullptr;
-  if (stream_ordered_alloc) {
+  // (a synchronous call keeps its workspace for the next one, but no large one)
+  const bool from_pool = stream_ordered_alloc || total > POOL_KEEP;
+  if (from_pool) {
     const cudaError_t e = stream_alloc(c, (void **)&ws, total, s);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      return GSKS_ERR_ALLOC;
+    }
     if (e != cudaSuccess) return cuda_status(e, "sliced workspace");
   } else {
     if (!c->dwork.ensure(total)) return GSKS_ERR_ALLOC;
@@ -124,7 +130,7 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   a.stall = tl_split_stall;
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = launch_tiles(a, std::min(ntm * nsc, sms), nr, s);
-  if (stream_ordered_alloc) cudaFreeAsync(ws, s);
+  if (from_pool) cudaFreeAsync(ws, s);
   if (e != cudaSuccess) return cuda_status(e, "sliced launch");
   note_launches(scan ? 3 : 2);
   return GSKS_OK;
