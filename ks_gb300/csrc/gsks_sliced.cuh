@@ -42,10 +42,11 @@ __host__ __device__ constexpr size_t colmeta_bytes(int nr) { return offsetof(Col
 static_assert(colmeta_bytes(1) % 16 == 0 && sizeof(ColMeta) % 16 == 0, "ColMeta is copied by the bulk-copy engine");
 
 // ---------------------------------------------------------------------------
-// 2^-(i / ETAB) in units of 2^-64, i = 0 .. ETAB - 1 (the first one unit short
-// of 1), plus EXP_BIAS: half of 2^-53 for exp2_neg's last shift and the mean of its
-// floors.  Products of the eleven constants 2^(-2^b / ETAB) in 64-bit fixed point,
-// evaluated by the compiler.
+// 2^-(i / ETAB) in units of 2^-63, i = 0 .. ETAB - 1, plus EXP_BIAS: half of 2^-53 for
+// exp2_neg's last shift and the mean of its floors.  (In units of 2^-64 the first entry has
+// no room for the half: values just below 1, all of a wide Gaussian's, were 0.6 2^-53 too
+// small in the mean.)  Products of the eleven constants 2^(-2^b / ETAB) in 64-bit fixed
+// point, evaluated by the compiler.
 constexpr uint64_t mulhi64c(uint64_t a, uint64_t b)
 {
   const uint64_t al = a & 0xffffffffu, ah = a >> 32, bl = b & 0xffffffffu, bh = b >> 32;
@@ -53,7 +54,7 @@ constexpr uint64_t mulhi64c(uint64_t a, uint64_t b)
   const uint64_t n = al * bh + (m & 0xffffffffu);
   return ah * bh + (m >> 32) + (n >> 32);
 }
-constexpr uint64_t EXP_BIAS = 1300;
+constexpr uint64_t EXP_BIAS = 640;
 struct ExpTable {
   uint64_t v[ETAB];
   constexpr ExpTable() : v()
@@ -61,7 +62,7 @@ struct ExpTable {
     constexpr uint64_t c[11] = {0xffe9d2b2f7db2756, 0xffd3a751c0f7e10c, 0xffa756521c8daed2, 0xff4ecb59511ec8a5,
                                 0xfe9e115c7b8f884c, 0xfd3e0c0cf486c175, 0xfa83b2db722a033a, 0xf5257d152486cc2c,
                                 0xeac0c6e7dd24392f, 0xd744fccad69d6af4, 0xb504f333f9de6484};
-    v[0] = ~0ull;
+    v[0] = (1ull << 63) + EXP_BIAS;
     for (int i = 1; i < ETAB; i++) {
       uint64_t p = 0;
       bool first = true;
@@ -70,7 +71,7 @@ struct ExpTable {
           p = first ? c[b] : mulhi64c(p, c[b]);
           first = false;
         }
-      v[i] = p + EXP_BIAS;
+      v[i] = (p >> 1) + EXP_BIAS;
     }
   }
 };
@@ -109,7 +110,7 @@ __device__ __forceinline__ void lds1(uint32_t addr, double &a)
   asm volatile("ld.shared.f64 %0, [%1];" : "=d"(a) : "r"(addr));
 }
 
-// 2^-y for y = z 2^-F, 2^-21 <= |y| < 1021, to about one unit in the last place:
+// 2^-y for y = z 2^-F, |z| >= 2^32, |y| < 1021, to about one unit in the last place:
 // y = n + (i + phi) / 2048, 2^-y = 2^-n T[i] (1 - P), P = 1 - 2^(-phi / 2048)
 // (the table-driven scheme of P. T. P. Tang, ACM TOMS 15 (1989), in integers).
 // FP64 instructions issue at 1/32 of the integer rate here (2 against 64 per
@@ -119,13 +120,14 @@ __device__ __forceinline__ void lds1(uint32_t addr, double &a)
 //   ln2 2^32 rounded up (2977044472), less q in units of 2^-55: z^2/2 - z^3/6 +
 //   z^4/24, z = ln2 phi / 2048, and the excess of the first constant; the
 //   fourth power replaced by its best cubic on [0, 1] (error 2^-7 of 20 2^-55).
-// Against exp2l over y in [2^-21, 1000]: at most 1.6 2^-53 relative, rms 0.45
-// 2^-53 (correctly rounded: 1 and 0.43).  y = 0 gives 1 - 2^-53: callers treat
-// it apart.
+// Against 50 decimals (the integer steps run on the host, F = 43 .. 62, y up to 1000): at
+// most 1.4 2^-53 relative, rms 0.43 2^-53 (correctly rounded: 1 and 0.43); below 2^-11 rms
+// 0.30, mean 0.03 or less.  y = 0 gives 1.
 struct ExpFrame {
   int s;                  // F - 43, 0 .. 19
   uint32_t mask, mul;     // 2^s - 1, ln2 2^(32 - s) (flo in units of P)
   uint32_t tab;           // shared-memory address of the table
+  uint32_t half;          // half a unit of z, in units of P, where z was rounded down (else 0)
 };
 __device__ __forceinline__ ExpFrame exp_frame(int F, uint32_t tab)
 {
@@ -134,6 +136,7 @@ __device__ __forceinline__ ExpFrame exp_frame(int F, uint32_t tab)
   f.mask = (1u << f.s) - 1u;
   f.mul = (2977044472u >> f.s) + (f.s ? (2977044472u >> (f.s - 1)) & 1u : 0u);
   f.tab = tab;
+  f.half = 0;
   return f;
 }
 // (The table's contents never change, so its load may move freely.)
@@ -144,12 +147,12 @@ __device__ __forceinline__ double exp2_neg(uint64_t z, const ExpFrame &E)
   const uint32_t f = __funnelshift_r(lo, hi, E.s);    // v = n 2048 + i, phi's upper 32 bits
   uint64_t t;
   asm("ld.shared.u64 %0, [%1];" : "=l"(t) : "r"(E.tab + (v & (ETAB - 1)) * 8));
-  const uint64_t lin = madw(lo & E.mask, E.mul, madw(f, 2977044472u, 0));
+  const uint64_t lin = madw(lo & E.mask, E.mul, madw(f, 2977044472u, E.half));
   const uint32_t q = mulhi(f, mulhi(f, 2063529957u - mulhi(f, 232762u)) + 744u);
   const uint64_t p = (uint64_t)madws((int)q, -(1 << 20), (long long)lin) >> 11;   // P in units of 2^-64
   const uint32_t th = (uint32_t)(t >> 32), tl = (uint32_t)t, ph = (uint32_t)(p >> 32), pl = (uint32_t)p;
-  const uint64_t s = madw(th, ph, 0) + mulhi(th, pl) + mulhi(tl, ph);      // T P
-  const uint64_t m = (t - s) >> 11;                                        // [2^52, 2^53], units of 2^-53
+  const uint64_t s = madw(th, ph, 0) + mulhi(th, pl) + mulhi(tl, ph);      // T P, units of 2^-63
+  const uint64_t m = (t - s) >> 10;                                        // [2^52, 2^53], units of 2^-53
   return __hiloint2double((int)((uint32_t)(m >> 32) + (1021u << 20)) - (v >> 11) * (1 << 20), (int)(uint32_t)m);
 }
 
@@ -175,7 +178,7 @@ struct PowFrame {
   uint32_t qh, ql;        // Q 2^56 (P <= 128: qh below 2^31)
   int pad;
 };
-// E: exp_frame52.  ok: y in (-1000, 1000).
+// E: exp_frame_floor(52).  ok: y in (-1000, 1000).
 __device__ __forceinline__ double pow_neg_half(uint64_t D, int F, const PowFrame &Q, const ExpFrame &E, bool &ok)
 {
   const int lz = __clz((int)(D >> 32));
@@ -187,7 +190,7 @@ __device__ __forceinline__ double pow_neg_half(uint64_t D, int F, const PowFrame
   const int J = (63 - F - lz) * 2048 + j;
   uint64_t t;
   asm("ld.shared.u64 %0, [%1];" : "=l"(t) : "r"(E.tab + (j & (ETAB - 1)) * 8));
-  t = (j & (ETAB - 1)) ? t - (EXP_BIAS + 170) : t;   // (170: the mean of r2's floor)
+  t = (j & (ETAB - 1)) ? 2 * (t - EXP_BIAS) - 225 : ~0ull;   // units of 2^-64 (225: the mean of the floors of r)
   // j = 2048: T[0] / 2, m just below 2
   const uint64_t pr = mulhi64(m, j == ETAB ? t >> 1 : t);                         // (1 + r) 2^63
   const long long r = (long long)(pr ^ 0x8000000000000000ull);
@@ -216,15 +219,13 @@ __device__ __forceinline__ double exp2_neg64(double y53, uint32_t tab)
     if ((uint32_t)(__double2hiint(y53) - 0x43e10000) < 0x7ff00001u - 0x43e10000u) return 0.0;
     return exp2_neg_wide(y53 * 0x1p-53);
   }
-  return exp2_neg((uint64_t)z, ExpFrame{10, 1023u, 2907270u, tab});
+  return exp2_neg((uint64_t)z, ExpFrame{10, 1023u, 2907270u, tab, 0});
 }
 
-// exp2_neg for y up to 1088 (hi: z's high word, lim: that of 1021): beyond 1021
-// the value is formed 2^512 too large and rounded into the subnormal range by
-// one multiplication.
-__device__ __forceinline__ double exp2_neg_deep(uint64_t z, int hi, int lim, const ExpFrame &E)
+// exp2_neg for y up to 1088 (deep: y is 1021 or more): beyond 1021 the value is formed
+// 2^512 too large and rounded into the subnormal range by one multiplication.
+__device__ __forceinline__ double exp2_neg_deep(uint64_t z, bool deep, const ExpFrame &E)
 {
-  const bool deep = hi >= lim;
   double v = exp2_neg(deep ? z - ((uint64_t)512 << (E.s + 43)) : z, E);
   if (deep) v *= 0x1p-512;
   return v;
@@ -232,19 +233,24 @@ __device__ __forceinline__ double exp2_neg_deep(uint64_t z, int hi, int lim, con
 
 // 2^-y for y = D 2^-F h_i h_j with the (positive) factors as 64-bit mantissas (Mi,
 // Mj, leading bit set) and the sum ex of their exponents (value = M 2^(ex - 63)):
-// D normalised, two products, one shift.  zh: the high word of y 2^52, saturated
-// (the value holds for zh in [1, 1088 2^20)).
-__device__ __forceinline__ double exp2_neg_scaled(uint64_t D, int F, uint64_t Mi, uint64_t Mj, int ex, const ExpFrame &E52,
-                                                  int &zh)
+// D normalised, two products, one shift.  zh: the high word of y 2^53, saturated
+// (the value holds for zh in [1, 1088 2^21)).  E: exp_frame_floor(53).
+__device__ __forceinline__ double exp2_neg_scaled(uint64_t D, int F, uint64_t Mi, uint64_t Mj, int ex, const ExpFrame &E,
+                                                  uint32_t &zh)
 {
   const int lz = __clzll((long long)D);
   const uint64_t t = mulhi64(mulhi64(D << lz, Mi), Mj);   // in [2^61, 2^64)
-  const int s = F + lz - ex - 54;                          // y 2^52 = t 2^-s
-  const uint64_t z = s < 0 ? t << 1 : t >> min(s, 63);     // (s < 0: y at least 1024)
-  zh = s < -1 || (s < 0 && (t >> 62)) ? 0x7fffffff : (int)min((uint32_t)(z >> 32), 0x7fffffffu);
-  return exp2_neg_deep(z, zh, 1021 << 20, E52);
+  const int s = F + lz - ex - 55;                          // y 2^53 = t 2^-s
+  const uint64_t z = s < 0 ? t << 1 : t >> min(s, 63);     // (s < 0: y at least 512)
+  zh = s < -1 || (s < 0 && (t >> 63)) ? 0xffffffffu : (uint32_t)(z >> 32);
+  return exp2_neg_deep(z, zh >= 1021u << 21, E);
 }
-__device__ __forceinline__ ExpFrame exp_frame52(uint32_t tab) { return ExpFrame{9, 511u, 5814540u, tab}; }
+// Frames of a z rounded down (pow_neg_half 52, exp2_neg_scaled 53): its mean error, half a
+// unit, is taken out (values were 0.7 2^-53 too large in the mean).
+__device__ __forceinline__ ExpFrame exp_frame_floor(int F, uint32_t tab)
+{
+  return F == 52 ? ExpFrame{9, 511u, 5814540u, tab, 2907270u} : ExpFrame{10, 1023u, 2907270u, tab, 1453635u};
+}
 
 // (double)w: the conversion instruction issues to the FP64 pipe (2 per SM cycle),
 // these about a dozen integer ones take a third of its time.  Rounds to nearest,

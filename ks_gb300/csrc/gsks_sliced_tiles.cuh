@@ -862,7 +862,7 @@ __device__ __noinline__ double rare_value(const TileArgs &a, const KParams &kp, 
       y = __double2ll_rn(near_d2(a, i, j, 0.0) * cp.ah * ldexp(1.0, cp.F));
     if (y <= 0) return 1.0;
     if ((int)(y >> 32) >= cp.end) return 0.0;
-    return exp2_neg_deep((uint64_t)y << cp.pre, (int)(y >> 32), cp.lim, exp_frame(max(cp.F, 43), tab));
+    return exp2_neg_deep((uint64_t)y << cp.pre, (int)(y >> 32) >= cp.lim, exp_frame(max(cp.F, 43), tab));
   } else {
     double d2 = direct_d2(a, cp, y, A, i, j);
     if constexpr (KT == KS_LAPLACE) {
@@ -928,7 +928,7 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp,
       for (int s = 0; s < 2; s++) {
         const int yh = (int)(W[c + s] >> 32);
         good[s] = yh > 0 && !(mask >> (c + s) & 1u);
-        kv[s] = exp2_neg_deep((uint64_t)W[c + s] << cp.pre, yh, lim, E);
+        kv[s] = exp2_neg_deep((uint64_t)W[c + s] << cp.pre, yh >= lim, E);
         kv[s] = yh < yend ? kv[s] : 0.0;
         mask = good[s] ? mask : mask | (1u << (c + s));
       }
@@ -963,10 +963,10 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp,
           kv[s] = pow_neg_half((uint64_t)D, F, pw, E, ok);
           good[s] = good[s] && ok;
         } else {
-          int zh;
+          uint32_t zh;
           kv[s] = exp2_neg_scaled((uint64_t)D, F, Mi, cm->hj[c0 + c + s],
                                   ei + cm->e[c0 + c + s], E, zh);
-          if (good[s] && zh >= (1088 << 20)) kv[s] = 0.0;      // beyond 2^-1088: 0, times w
+          if (good[s] && zh >= 1088u << 21) kv[s] = 0.0;      // beyond 2^-1088: 0, times w
           else good[s] = good[s] && zh > 0;
         }
         mask = good[s] ? mask : mask | (1u << (c + s));
@@ -1356,7 +1356,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) sliced_tiles(TileArgs a)
       // (without the frame's norms the sum of many coordinates leaves two bits more)
       const int gb = G >= 0 ? G : guard_bits(a.kpad, fixed);
       const uint32_t bias = combine_bias<SIGN>(gb);
-      const ExpFrame E = KT == KS_GAUSSIAN ? exp_frame(max(fixed ? cp.F : 43, 43), tabS) : exp_frame52(tabS);
+      const ExpFrame E = KT == KS_GAUSSIAN ? exp_frame(max(fixed ? cp.F : 43, 43), tabS)
+                                           : exp_frame_floor(KT == KS_LAPLACE ? 52 : 53, tabS);
       const long long arow = __double_as_longlong(a.row_aa[i0]);
       const int unheld = (int)__reduce_or_sync(0xffffffffu, (unsigned)a.row_e[i0]);
       double racc[NR];
