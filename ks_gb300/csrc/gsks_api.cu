@@ -103,6 +103,20 @@ Ctx::~Ctx()
 
 static thread_local std::unique_ptr<Ctx> tl_ctx;
 
+// (made with the context: a stream that captures the thread's first asynchronous call
+// takes no new pool)
+static cudaError_t make_pool(Ctx *c)
+{
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = c->device;
+  const cudaError_t e = cudaMemPoolCreate(&c->pool, &props);
+  if (e != cudaSuccess) { c->pool = nullptr; return e; }
+  unsigned long long keep = POOL_KEEP;
+  return cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
 Ctx *get_ctx()
 {
   int dev = -1;
@@ -118,6 +132,7 @@ Ctx *get_ctx()
     cuda_status(e, "cudaStreamCreate");
     return nullptr;
   }
+  if ((e = make_pool(c.get())) != cudaSuccess) { cuda_status(e, "cudaMemPoolCreate"); return nullptr; }
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev);
   if (!c->err.ensure(sizeof(int))) { set_status(GSKS_ERR_ALLOC, "context"); return nullptr; }
   cudaMemset(c->err.p, 0, sizeof(int));
@@ -127,21 +142,6 @@ Ctx *get_ctx()
 
 cudaError_t stream_alloc(Ctx *c, void **p, size_t bytes, cudaStream_t s)
 {
-  if (!c->pool) {
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = c->device;
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = cudaMemPoolCreate(&pool, &props);
-    if (e != cudaSuccess) return e;
-    unsigned long long keep = POOL_KEEP;
-    if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
-      cudaMemPoolDestroy(pool);
-      return e;
-    }
-    c->pool = pool;
-  }
   return cudaMallocFromPoolAsync(p, bytes, c->pool, s);
 }
 
