@@ -1051,13 +1051,15 @@ __device__ __noinline__ void direct_cols(const TileArgs &a, const KParams &kp, i
     }
     const double *xs = (const double *)__shfl_sync(full, (unsigned long long)x, src);
     double s = 0.0;
+    const double *y = a.XB + (col >= 0 ? (size_t)pool_clamp(a.bmap, j0 + col, a.nxb) * a.k : 0);
     if (col >= 0) {
-      const double *y = a.XB + (size_t)pool_clamp(a.bmap, j0 + col, a.nxb) * a.k;
 #pragma unroll 8
       for (int p = sub; p < a.k; p += 8) s = fma(__ldg(xs + p), __ldg(y + p), s);
     }
 #pragma unroll
     for (int d = 4; d; d >>= 1) s += __shfl_xor_sync(full, s, d);
+    // (an overflow's sign is that of the sum in order; two partial sums' may cancel to NaN)
+    if (!(fabs(s) <= 1.79e308)) s = dot_direct(xs, y, a.k);
     const double kv = kvalue_call<KT>(a, kp, s);
 #pragma unroll
     for (int g = 0; g < 4; g++) {

@@ -130,3 +130,22 @@ def test_kernel_values(gpu, kind, k, power):
     # power or tanh and for numpy's own)
     curve = power * (power - 1) * (np.abs(c) + dc) ** max(power - 2, 0) if power else 1.0
     assert np.all(np.abs(got - val) <= slope * dc + curve * dc * dc + 8 * 2.0 ** -53 * np.abs(val))
+
+
+@pytest.mark.parametrize("how", ["single", "rhs", "list"])
+@pytest.mark.parametrize("k", [3, 20, 70, 300])
+def test_sums_beyond_the_range(gpu, k, how):
+    """x.y beyond FP64's range: a chain of fused multiply-adds has the sign of its first
+    overflow (and is a NaN only where a coordinate is), tanh of it 1 or -1."""
+    from ks_gb300 import gsks
+    rng = np.random.default_rng(k)
+    x, y = rng.standard_normal((40, k)) * 1e160, rng.standard_normal((6, k)) * 1e160
+    got = _pairs(gsks, gpu, gsks.make_kernel(gsks.KS_TANH, scal=1.0), x, y, how)
+    for i in range(40):
+        for j in range(6):
+            s = Fraction(0)
+            for a, b in zip(x[i], y[j]):
+                s += Fraction(a) * Fraction(b)
+                if abs(s) >= 2 ** 1024:
+                    break
+            assert got[i, j] == (1.0 if s > 0 else -1.0)
