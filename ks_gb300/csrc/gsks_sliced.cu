@@ -116,7 +116,7 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   a.ntm = ntm; a.ntn = ntn; a.nsc = nsc; a.chunk_tiles = 2 * chunk;
   a.imgA = p.imgA; a.imgB = p.imgB;
   a.row_aa = p.row_aa; a.row_hi = p.row_hi; a.row_e = p.row_e;
-  a.XA = XA; a.XB = XB; a.amap = amap; a.bmap = bmap; a.nxa = nxa; a.nxb = nxb;
+  a.XA = XA; a.XB = XB; a.XA2 = XA2; a.XB2 = XB2; a.amap = amap; a.bmap = bmap; a.nxa = nxa; a.nxb = nxb;
   a.kp = kp;
   a.kp.coinc = coincidence_eps(k);
   a.cp = p.cp;

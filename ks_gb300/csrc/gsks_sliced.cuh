@@ -24,6 +24,7 @@ constexpr int ELIM = 450;            // largest magnitude of a sliced point's ex
 constexpr int EBIAS = 2048;
 constexpr int NOT_COARSE = 1 << 20, NOT_LARGE = 1 << 21, NOT_DENSE = 1 << 22;
 constexpr int NOT_HELD = NOT_COARSE | NOT_LARGE | NOT_DENSE;   // also of a point without digits
+constexpr int NORM_GIVEN = 1 << 23;     // the point's norm, as given, is not that of its coordinates
 constexpr int ECLASS = 24;
 constexpr int ETAB = 2048;           // entries of the 2^-f table
 

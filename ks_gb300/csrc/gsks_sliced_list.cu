@@ -164,7 +164,7 @@ int sliced_list_run(const SlicedListPlan &Pl, Ctx *c, const double *XA, const do
   a.k = Pl.k; a.kpad = Pl.kpad; a.nrhs = 1; a.ntm = 1;
   a.imgA = p.imgA; a.imgB = p.imgB;
   a.row_aa = p.row_aa; a.row_hi = p.row_hi; a.row_e = p.row_e;
-  a.XA = XA; a.XB = XB; a.amap = a_idx; a.bmap = b_idx; a.nxa = nxa; a.nxb = nxb;
+  a.XA = XA; a.XB = XB; a.XA2 = XA2; a.XB2 = XB2; a.amap = a_idx; a.bmap = b_idx; a.nxa = nxa; a.nxb = nxb;
   a.partial = partial;
   a.err = err;
   a.next_item = p.next_item;

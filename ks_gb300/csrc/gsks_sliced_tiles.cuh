@@ -430,6 +430,7 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
 {
   __shared__ uint32_t s_max[8][32];
   __shared__ HeldStat s_held[8][32];
+  __shared__ double s_norm[8][32];
   __shared__ CallParam s_cp;
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int nbA = a.nta * (BM / 32);
@@ -498,11 +499,16 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     }
   };
 
-  double v[8];
+  double v[8], norm = 0.0;
   uint32_t mh = 0;
   const int nw = blockDim.x >> 5;
+  const bool dots = !kt_uses_norms(kt);
   for (int kg = wp; kg < kgs; kg += nw) {
     load8(kg, v);
+    if (!dots) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) norm = fma(v[q], v[q], norm);
+    }
     if (!fixed) {
 #pragma unroll
       for (int q = 0; q < 8; q++)
@@ -511,9 +517,10 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
   }
   int e = fixed ? s_cp.e : 0;
   bool flag = false;
+  s_max[wp][lane] = mh;
+  s_norm[wp][lane] = norm;
+  __syncthreads();
   if (!fixed) {
-    s_max[wp][lane] = mh;
-    __syncthreads();
 #pragma unroll
     for (int q = 0; q < 8; q++)
       if (q < nw) mh = max(mh, s_max[q][lane]);
@@ -526,7 +533,6 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
   }
   uint8_t *base = side ? a.imgB + (size_t)tile * btile_bytes(a.kpad, a.nr) : a.imgA + (size_t)tile * op_bytes(BM, a.kpad);
   const bool once = kgs <= nw;             // each thread's only group is still in registers
-  const bool dots = !kt_uses_norms(kt);
   HeldStat held{};
   for (int kg = wp; kg < kgs; kg += nw) {
     if (!once) load8(kg, v);
@@ -560,6 +566,11 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     }
     const bool norms = !dots, varbw = kt == KS_GAUSSIAN_VAR_BANDWIDTH;
     double nn = (valid && norms) ? (side ? a.XB2[p] : a.XA2[p]) : 0.0;
+    if (norms) {
+      // the point's own norm summed in any order, or another one
+      for (int q = 1; q < nw; q++) norm += s_norm[q][lane];
+      if (!(fabs(norm - nn) <= norm * ((double)(a.k + 16) * 0x1p-52) + 0x1p-1060)) bits |= NORM_GIVEN;
+    }
     if (fixed) {
       const double y = fma(nn, s_cp.ah, nn * s_cp.al) * ldexp(1.0, s_cp.F);
       nn = __longlong_as_double(__double2ll_rn(y));
@@ -577,14 +588,14 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
     if (!side) {
       a.row_aa[slot] = nn;
       a.row_hi[slot] = hb;
-      a.row_e[slot] = fixed ? e : (e + EBIAS) | bits;
+      a.row_e[slot] = fixed ? (e & 0xfffff) | bits : (e + EBIAS) | bits;
       if (a.row_n) a.row_n[slot] = 0;
     } else {
       ColMeta *cm = (ColMeta *)(base + op_bytes(BN, a.kpad));
       cm->bb[r] = nn;
       cm->hj[r] = hb;
       cm->e[r] = fixed ? e : (e + EBIAS) | bits;
-      const int any = (int)__reduce_or_sync(0xffffffffu, (unsigned)bits) & NOT_HELD;
+      const int any = (int)__reduce_or_sync(0xffffffffu, (unsigned)bits) & (NOT_HELD | NORM_GIVEN);
       if (lane == 0) { cm->flag = any; cm->pad[0] = cm->pad[1] = cm->pad[2] = 0; }
       const size_t wi = valid ? (size_t)(a.wmap ? a.wmap[pt] : pt) * a.nrhs : 0;
       for (int q = 0; q < a.nr; q++) cm->w[q][r] = (valid && q < a.nrhs) ? a.w[wi + q] : 0.0;
@@ -598,7 +609,7 @@ struct TileArgs {
   int ntm, ntn, nsc, chunk_tiles;   // items = ntm * nsc, chunk_tiles source tiles each
   const uint8_t *imgA, *imgB;
   const double *row_aa; const uint64_t *row_hi; const int *row_e;
-  const double *XA, *XB;            // pools and maps, for pairs formed directly
+  const double *XA, *XB, *XA2, *XB2;   // pools and maps, for pairs formed directly
   const int *amap, *bmap;
   int nxa, nxb;
   KParams kp;
@@ -774,6 +785,17 @@ static __device__ __noinline__ double near_d2(const TileArgs &a, int i, int j, d
   return s;
 }
 
+// The same from norms that are not the points' own: as given.
+static __device__ __noinline__ double given_d2(const TileArgs &a, int i, int j)
+{
+  const int pa = pool_clamp(a.amap, i, a.nxa), pb = pool_clamp(a.bmap, j, a.nxb);   // flagged by slice_kernel
+  const double *x = a.XA + (size_t)pa * a.k, *y = a.XB + (size_t)pb * a.k;
+  double s = 0.0;
+#pragma unroll 1   // (what a function called here needs in registers, every caller sets aside)
+  for (int p = 0; p < a.k; p++) s = fma(x[p], y[p], s);
+  return fma(-2.0, s, a.XA2[pa]) + a.XB2[pb];
+}
+
 // Row side of a pair: metadata, and the row's position in the call's maps (-1:
 // a padding row).
 struct RowMeta {
@@ -787,7 +809,7 @@ struct RowMeta {
 // cfold: y 2^53 per unit of d2 (Gaussian), times h_i (variable bandwidth).
 template <int KT>
 __device__ __forceinline__ double kvalue(const TileArgs &a, const KParams &kp, int j, double dot, const RowMeta &am,
-                                         double bb, double hj, double cfold, uint32_t tab)
+                                         double bb, double hj, double cfold, uint32_t tab, const ColMeta *cm)
 {
   double d2 = 0.0;
   bool near = false;
@@ -795,7 +817,7 @@ __device__ __forceinline__ double kvalue(const TileArgs &a, const KParams &kp, i
     d2 = fma(-2.0, dot, am.aa) + bb;
     // d2 at most about 2^-39 of the larger norm, by the high words
     near = __double2hiint(d2) <= max(__double2hiint(am.aa), __double2hiint(bb)) - (39 << 20);
-    if (KT != KS_LAPLACE && near && am.i >= 0) d2 = near_d2(a, am.i, j, d2);
+    if (KT != KS_LAPLACE && near && am.i >= 0 && !((am.e | cm->flag) & NORM_GIVEN)) d2 = near_d2(a, am.i, j, d2);
   }
   if constexpr (KT == KS_GAUSSIAN || KT == KS_GAUSSIAN_VAR_BANDWIDTH) {
     // max(d2, 0), also of NaN (fmax): anything not in (0, inf] becomes 0
@@ -844,34 +866,38 @@ __device__ __forceinline__ Place place_of(const TileArgs &a, int item, int row, 
 
 // A pair's distance where the fixed-point one does not do: nearly coincident
 // points (D at most about 2^-38 of the norms), two small norms.
-__device__ __forceinline__ double direct_d2(const TileArgs &a, const CallParam &cp, long long D, long long A, int i, int j)
+__device__ __forceinline__ double direct_d2(const TileArgs &a, const CallParam &cp, long long D, long long A, int i, int j,
+                                            bool given)
 {
-  if (D <= (A >> 38) || (cp.small && (int)(A >> 32) < cp.small)) return near_d2(a, i, j, 0.0);
+  if (D <= (A >> 38) || (cp.small && (int)(A >> 32) < cp.small)) return given ? given_d2(a, i, j) : near_d2(a, i, j, 0.0);
   return (double)D * ldexp(1.0, -cp.F);
 }
 
 // The fixed-point value of a pair outside the common range.  j: the column's
-// position (-1: a padding column).
+// position (-1: a padding column).  A's top bit: one of the norms
+// is not its point's own (NORM_GIVEN).
 template <int KT>
 __device__ __noinline__ double rare_value(const TileArgs &a, const KParams &kp, const CallParam &cp, uint32_t tab,
                                           long long y, long long A, int i, int j)
 {
   if (i < 0 || j < 0) return 0.0;   // padding: its weight is 0
+  const bool given = A < 0;
+  A &= 0x7fffffffffffffffll;
   if constexpr (KT == KS_GAUSSIAN) {
     if (y <= (A >> 38) || (cp.small && (int)(A >> 32) < cp.small))
-      y = __double2ll_rn(near_d2(a, i, j, 0.0) * cp.ah * ldexp(1.0, cp.F));
+      y = __double2ll_rn((given ? given_d2(a, i, j) : near_d2(a, i, j, 0.0)) * cp.ah * ldexp(1.0, cp.F));
     if (y <= 0) return 1.0;
     if ((int)(y >> 32) >= cp.end) return 0.0;
     return exp2_neg_deep((uint64_t)y << cp.pre, (int)(y >> 32) >= cp.lim, exp_frame(max(cp.F, 43), tab));
   } else {
-    double d2 = direct_d2(a, cp, y, A, i, j);
+    double d2 = direct_d2(a, cp, y, A, i, j, given);
     if constexpr (KT == KS_LAPLACE) {
       // (two coincident points have the same norm)
       if (d2 < fmax(1e-15, kp.coinc * 2.0 * ((double)A * ldexp(1.0, -cp.F)))) d2 = 1.79e308;
       return pow_call(d2, kp);      // the row's sum is multiplied by scal
     } else {
       const int pa = pool_clamp(a.amap, i, a.nxa), pb = pool_clamp(a.bmap, j, a.nxb);   // flagged by slice_kernel
-      return exp2_neg64(((d2 * (0.5 * 1.4426950408889634 * 0x1p53)) * kp.hi[pa]) * kp.hj[pb], tab);
+      return exp2_neg64(((fmax(d2, 0.0) * (0.5 * 1.4426950408889634 * 0x1p53)) * kp.hi[pa]) * kp.hj[pb], tab);
     }
   }
 }
@@ -946,7 +972,7 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp,
     int ei = 0;
     if constexpr (KT == KS_GAUSSIAN_VAR_BANDWIDTH) {
       Mi = a.row_hi[i0];
-      ei = a.row_e[i0];
+      ei = a.row_e[i0] << 12 >> 12;
     }
     const PowFrame pw = cp.pw;
     const int F = cp.F;
@@ -983,6 +1009,9 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp,
   }
   if (!mask) return;
   const Place P = place_of<LISTED>(a, item, row, tj, c0);
+  // (the row's place in the metadata, formed anew)
+  if ((a.row_e[item_geo<LISTED>(a, item).a_tile * BM + row] | cm->flag) & NORM_GIVEN)
+    A = (long long)((uint64_t)A | 0x8000000000000000ull);
   for (; mask; mask &= mask - 1) {
     const int c = __ffs(mask) - 1;
     long long y = W[0];
@@ -1003,7 +1032,7 @@ __device__ __forceinline__ void fixed_cols(const TileArgs &a, const KParams &kp,
 template <int KT>
 __device__ __noinline__ double kvalue_call(const TileArgs &a, const KParams &kp, double dot)
 {
-  return kvalue<KT>(a, kp, 0, dot, RowMeta{}, 0.0, 0.0, 0.0, 0);
+  return kvalue<KT>(a, kp, 0, dot, RowMeta{}, 0.0, 0.0, 0.0, 0, nullptr);
 }
 
 // The columns that dot_cols left (a bit each; the whole warp calls).  Few pairs among the
@@ -1109,7 +1138,7 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
         dot = dot_direct(a.XA + (size_t)pa * a.k, a.XB + (size_t)pb * a.k, a.k);
       }
       const double kv = kvalue<KT>(a, kp, j, dot, am, cm->bb[c0 + c],
-                                    __longlong_as_double((long long)cm->hj[c0 + c]), cfold, tab);
+                                    __longlong_as_double((long long)cm->hj[c0 + c]), cfold, tab, cm);
 #pragma unroll
       for (int r = 0; r < NR; r++)
         if (r == 0 || r < a.nrhs) sum[r] = fma(kv, cm->w[r][c0 + c], sum[r]);
