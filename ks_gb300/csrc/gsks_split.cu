@@ -1012,7 +1012,8 @@ __global__ void __launch_bounds__(256) pack_kernel(PackArgs g)
   mt.n_lo = (float)nl;
   mt.w = 0.0f;
   mt.h = 0.0f;
-  const size_t wi = valid ? (size_t)(g.wmap ? g.wmap[pt] : pt) * (nrhs > 1 ? nrhs : 1) : 0;   // weight column 0
+  // weight column 0 (wmap has an entry per source: none is read for a target)
+  const size_t wi = valid && side == 1 ? (size_t)(g.wmap ? g.wmap[pt] : pt) * (nrhs > 1 ? nrhs : 1) : 0;
   double wf = 1.0;                 // the Gaussian fast path's source factor
   if (side == 1 && valid) mt.w = (float)g.w[wi];
   if (gfast) {
