@@ -297,13 +297,13 @@ def roofline_split(per, peaks, rates):
 # warp instruction per SM cycle on GB300, i.e. 2 DFMA per SM per cycle; the
 # FP64 tensor-core MMA (DMMA) issues to the same pipe at 1.8 FMA per SM cycle
 # (profiles/fp64_pipe_peak.md).  The FP64 form's inner products run on the f16
-# tensor cores instead (k <= 1024): 21 exact digit products per coordinate; its
+# tensor cores instead (k <= 1024): 26 digit products per coordinate; its
 # kernel values run on integer instructions, which leaves the FP64 pipe the
 # weighted sum (and, for polynomials, scal x.y + cons).
 FP64_FMA_PER_SM_CYCLE = 2.0
 
 
-FP64_DIGIT_PRODUCTS = 21
+FP64_DIGIT_PRODUCTS = 26
 FP64_PIPE_PER_PAIR = {"gaussian": 1, "laplace": 1, "polynomial": 2}
 
 
@@ -415,7 +415,7 @@ def run_ours(args, ws, rank, local):
         roof = {"bound": "tensor", "kernel": f"sliced_tiles<{dom}>", "achieved": dk["executed_tflops"],
                 "peak": round(peaks.get("bf16_tflops", 1900.0), 1), "unit": "TFLOP/s",
                 "frac": dk["frac_executed_tensor"], "traffic": read_traffic(f"sliced_tiles_{dom}_general_stride"),
-                "flops": "executed f16 digit products (21 per coordinate pair); frac_fp64_pipe beside it",
+                "flops": "executed f16 digit products (26 per coordinate pair); frac_fp64_pipe beside it",
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst; f16 runs at the bf16 rate)"
                 if "bf16_tflops" in peaks else "fallback 1.9 PFLOP/s bf16"}
     roof["fp64_peak_tflops"] = round(p64 / 1e12, 4)
