@@ -443,7 +443,7 @@ extern "C" int dgsks_list(ks_t *kernel, ks_t *kernels, int ntask, int k,
     if (e != cudaSuccess) return cuda_status(e, "dgsks_list copy back");
   }
   // (kept for the next call, but no large one)
-  if (B.plan.lp.ws.cap > POOL_KEEP) B.plan.lp.ws.release();
+  if (B.plan.lp.ws.cap > SYNC_KEEP) B.plan.lp.ws.release();
   note_launches(launches);
   return set_status(GSKS_OK, nullptr);
 }

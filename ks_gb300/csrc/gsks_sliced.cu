@@ -74,7 +74,7 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   const size_t total = o_p + al((size_t)nrhs * nparts * ldp * 8);
   uint8_t *ws = nullptr;
   // (a synchronous call keeps its workspace for the next one, but no large one)
-  const bool from_pool = stream_ordered_alloc || total > POOL_KEEP;
+  const bool from_pool = stream_ordered_alloc || total > SYNC_KEEP;
   if (from_pool) {
     const cudaError_t e = stream_alloc(c, (void **)&ws, total, s);
     if (e == cudaErrorMemoryAllocation) {
