@@ -22,6 +22,7 @@ constexpr int ELIM = 450;            // largest magnitude of a sliced point's ex
 // EBIAS (twice of which leaves a double's high word unchanged), what the point's digits
 // do not promise for its inner products (held_bits), and the class of its length.
 constexpr int EBIAS = 2048;
+constexpr int EMASK = 12, EMASK_K = 8;  // up to 8 coordinates: a bit for each large one
 constexpr int NOT_COARSE = 1 << 20, NOT_LARGE = 1 << 21, NOT_DENSE = 1 << 22;
 constexpr int NOT_HELD = NOT_COARSE | NOT_LARGE | NOT_DENSE;   // also of a point without digits
 constexpr int NORM_GIVEN = 1 << 23;     // the point's norm, as given, is not that of its coordinates

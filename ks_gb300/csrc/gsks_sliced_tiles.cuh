@@ -390,7 +390,9 @@ __device__ __forceinline__ void slice8(const double (&v)[8], int e, bool live, u
 //   large ones (k up to 128: one or two roundings to W's unit): every coordinate that is
 //     not 0 is at least 2^-3, so that |xi_p eta_p| >= 2^-6 for each p that both have;
 //   dense ones: three quarters of the coordinates or more are at least 2^-5, so that half
-//     of them are in both points.
+//     of them are in both points;
+//   any with a coordinate of at least 2^-3 in both (k up to 8, whose points often have a
+//     small one: a mask of them.  Polynomial, 16384 x 16384 normal points, k = 7: 4.8 -> 2.6 ms).
 // Of other pairs dot_cols forms those with a small W directly: |W| < 2^-4 2^c, c the larger
 // class, 2^c >= |xi| (and the share of W's own roundings in long rows).
 struct HeldStat {
@@ -398,8 +400,9 @@ struct HeldStat {
   int count;                // that are not 0
   int sq;                   // |xi|^2 2^16, rounded down
   int fine;                 // one needs more than 26 bits
+  int mask;                 // the first eight of at least 2^-3
 };
-__device__ __forceinline__ void held_stat(const double (&v)[8], int e, HeldStat &t)
+__device__ __forceinline__ void held_stat(const double (&v)[8], int e, bool first, HeldStat &t)
 {
 #pragma unroll
   for (int q = 0; q < 8; q++) {
@@ -408,6 +411,7 @@ __device__ __forceinline__ void held_stat(const double (&v)[8], int e, HeldStat 
     const int sh = e + 1022 - (int)(b >> 52);          // 0 and more; xi = M 2^-(53 + sh)
     const int top = sh < 8 ? (int)(M >> (45 + sh)) : 0;
     t.large3 += sh < 3;
+    if (first) t.mask |= sh < 3 ? 1 << q : 0;
     t.large5 += sh < 5;
     t.count += b != 0;
     t.sq += top * top;
@@ -420,7 +424,7 @@ __device__ __forceinline__ int held_bits(const HeldStat &t, int k, int kpad)
   int c = t.sq <= 1 << 16 ? 0 : (17 - __clz(t.sq - 1)) / 2;            // 4^c >= |xi|^2
   c = max(c, kpad > 512 ? 3 : kpad > 256 ? 1 : 0);
   return (t.fine ? NOT_COARSE : 0) | (t.large3 < t.count || kpad > 128 ? NOT_LARGE : 0) |
-         (4 * t.large5 < 3 * k ? NOT_DENSE : 0) | c << ECLASS;
+         (4 * t.large5 < 3 * k ? NOT_DENSE : 0) | (k <= EMASK_K ? t.mask << EMASK : 0) | c << ECLASS;
 }
 
 // One block per 32 points: lane = point, each warp a group of eight coordinates
@@ -540,7 +544,7 @@ static __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a)
 #pragma unroll
       for (int q = 0; q < 8; q++) v[q] *= mul;
     }
-    if (dots) held_stat(v, e, held);
+    if (dots) held_stat(v, e, kg == 0, held);
     uint4 out[NS];
     slice8(v, e, !flag, out);
     const int c = kg / gpc, kgc = kg - c * gpc;
@@ -1122,6 +1126,7 @@ __device__ __forceinline__ void dot_cols(const TileArgs &a, const KParams &kp, c
       // (a point without digits: W = 0)
       const int lim = 1 << (16 + gb + (max(am.e, ej) >> ECLASS));          // 2^-4 2^class, high word
       if (c < P.nv && ((am.e | ej) & NOT_HELD) == NOT_HELD &&
+          !(am.e & ej & (((1 << EMASK_K) - 1) << EMASK)) &&
           (uint32_t)((int)(W[c] >> 32) + lim) < 2u * (uint32_t)lim)
         direct |= 1u << c;
     }
