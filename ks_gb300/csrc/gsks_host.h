@@ -84,8 +84,9 @@ Ctx *get_ctx();
 // rest is given back at the next synchronisation and mapped again by the next call.
 constexpr size_t POOL_KEEP = 512ull << 20;
 // Workspaces of the synchronous FP64 calls (single and one-shot lists) are kept for the
-// thread's next call up to this size.  (Mapping 2.6 GB anew took 2 ms of a list's 14.)
-constexpr size_t SYNC_KEEP = 4ull << 30;
+// thread's next call up to this size, a sixteenth of the device's memory.  (Mapping 2.6 GB
+// anew took 2 ms of a list's 14, the 9 GB of 20000 tasks at k = 16 4 of 102.)
+constexpr size_t SYNC_KEEP = 16ull << 30;
 cudaError_t stream_alloc(Ctx *c, void **p, size_t bytes, cudaStream_t s);
 int set_status(int s, const char *where);
 int cuda_status(cudaError_t e, const char *where);
