@@ -134,6 +134,8 @@ Ctx *get_ctx()
   }
   if ((e = make_pool(c.get())) != cudaSuccess) { cuda_status(e, "cudaMemPoolCreate"); return nullptr; }
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev);
+  size_t free_mem = 0;
+  if ((e = cudaMemGetInfo(&free_mem, &c->total_mem)) != cudaSuccess) { cuda_status(e, "cudaMemGetInfo"); return nullptr; }
   if (!c->err.ensure(sizeof(int))) { set_status(GSKS_ERR_ALLOC, "context"); return nullptr; }
   cudaMemset(c->err.p, 0, sizeof(int));
   tl_ctx = std::move(c);

@@ -40,6 +40,7 @@ struct Ctx {
   cudaStream_t side = nullptr;             // a batched call's second branch,
   cudaEvent_t fork = nullptr, join = nullptr;   // from and back to the call's stream
   int num_sms = 0;
+  size_t total_mem = 0;        // the device's
   DevBuf partial, err;
   DevBuf dA, dA2, dB, dB2, dw, du, dhi, dhj, dwork;
   DevBuf rmaps;                // per-rhs u and w maps of the multi-rhs calls

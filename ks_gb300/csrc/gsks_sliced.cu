@@ -72,6 +72,8 @@ int enqueue_sliced(Ctx *c, const ks_t *ker, int m, int n, int k, double *u, cons
   const size_t o_p = o_n + al((size_t)ldp * 4);
   const int nparts = nr > 1 ? nsc * GROUPS : nsc;          // partials per row and column
   const size_t total = o_p + al((size_t)nrhs * nparts * ldp * 8);
+  // (a capturing stream would only record the allocation, to fail with the graph)
+  if (total > c->total_mem) return GSKS_ERR_ALLOC;
   uint8_t *ws = nullptr;
   // (a synchronous call keeps its workspace for the next one, but no large one)
   const bool from_pool = stream_ordered_alloc || total > SYNC_KEEP;

@@ -51,6 +51,32 @@ def test_single_call(gpu, sync, nrhs):
     assert torch.all((u - ref[am.long()]).abs() <= 2.0 ** -53 * 64 * 3 * w[:n * nrhs].abs().max())
 
 
+def test_captured_call(gpu):
+    from ks_gb300 import gsks
+    torch, k, n = gpu, 1024, 3
+    X, X2, w = _pool(torch, k, np.random.default_rng(5))
+    m = _too_many(torch, k)
+    am = torch.randint(500, (m,), dtype=torch.int32, device="cuda")
+    bm = torch.arange(n, dtype=torch.int32, device="cuda")
+    ker = gsks.make_kernel(gsks.KS_GAUSSIAN, scal=-0.002)
+    ref, u = (torch.zeros(q, dtype=torch.float64, device="cuda") for q in (500, m))
+    row, every = torch.arange(500, dtype=torch.int32, device="cuda"), torch.arange(m, dtype=torch.int32, device="cuda")
+
+    def enqueue(out, um, a):
+        gsks.dgsks_device(ker, len(a), n, k, out, um, X, X2, a, X, X2, bm, w, bm, stream=torch.cuda.current_stream(),
+                          nxa=500, nxb=500)
+
+    enqueue(ref, row, row)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        enqueue(u, every, am)
+    g.replay()
+    torch.cuda.synchronize()
+    assert gsks.device_errors() == 0
+    assert torch.all((u - ref[am.long()]).abs() <= 2.0 ** -53 * 64 * 3 * w[:n].abs().max())
+
+
 @pytest.mark.parametrize("planned", [False, True])
 def test_list(gpu, planned):
     from ks_gb300 import gsks
