@@ -438,6 +438,21 @@ KParams make_kparams(const ks_t *ker, const double *hi, const double *hj)
 // |fl(aa - 2 x.y + bb) - d2| <= ~2k u (aa + bb) with u = 2^-53.
 double coincidence_eps(int k) { return 4.0 * (double)std::max(k, 1) * 0x1p-53; }
 
+// Calls of few pairs and few coordinates that the DFMA kernels take in less time than the
+// digit products, whose 128-row tiles then leave most SMs idle: tanh and general powers,
+// whose values are some 30 FP64 instructions in either form (us at k = 3, digits / DFMA:
+// tanh 3000 x 75 66 / 46, 75 x 3000 67 / 58, but 1000 x 1000 70 / 82; general powers 3000 x
+// 75 49 / 38; level at 16 to 20 coordinates for tanh, 8 to 20 for powers).  Powers 2 to 4 (25
+// / 24, 75 x 3000 27 / 31) stay; so do the kernels of distances, whose nearly coincident
+// points the digit form holds better (multiquadratic 26 / 23).
+static bool dfma_small(const ks_t *ker, int m, int n, int k)
+{
+  if ((long long)m * n > 1 << 19) return false;
+  if (ker->type == KS_TANH) return k <= 16;
+  return ker->type == KS_POLYNOMIAL && k <= 8 &&
+         !(ker->powe == 1.0 || ker->powe == 2.0 || ker->powe == 3.0 || ker->powe == 4.0);
+}
+
 // Enqueue one fused evaluation on stream s.  Maps may be nullptr (identity).
 int enqueue_fused(Ctx *c, const ks_t *ker, int m, int n, int k,
                   double *u, const int *umap,
@@ -451,7 +466,7 @@ int enqueue_fused(Ctx *c, const ks_t *ker, int m, int n, int k,
     return enqueue_split(c, ker, m, n, k, u, umap, XA, XA2, amap, nxa, XB, XB2, bmap, nxb,
                          w, wmap, hi, hj, s, stream_ordered_alloc, std::max(nrhs, 1));
   if (precision != GSKS_FP64) return GSKS_ERR_PRECISION;
-  if (sliced_takes(k)) {
+  if (sliced_takes(k) && !dfma_small(ker, m, n, k)) {
     const int st = enqueue_sliced(c, ker, m, n, k, u, umap, XA, XA2, amap, nxa, XB, XB2, bmap, nxb,
                                   w, wmap, hi, hj, s, stream_ordered_alloc, std::max(nrhs, 1));
     // (no room for the digits, 12 bytes a coordinate: the DFMA kernels need none)

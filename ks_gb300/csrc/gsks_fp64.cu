@@ -1,8 +1,8 @@
 // gsks_fp64.cu -- DFMA kernels of the fused kernel summation (sm_103a): the FP64
-// form beyond k = 1024, the allocation-free entry, and calls whose digits find no
-// room.  (Up to k = 1024 the digit products of gsks_sliced.cu are 7 to 45 times as
-// fast, 1.6 times for a call of 100 x 120 points; beyond it a row's digits no longer
-// fit the sums' 64 bits.)
+// form beyond k = 1024, the allocation-free entry, calls whose digits find no room, and
+// some calls of few pairs and coordinates (dfma_small).  (Else up to k = 1024 the digit
+// products of gsks_sliced.cu are 7 to 45 times as fast, 1.6 times for a call of 100 x 120
+// points; beyond it a row's digits no longer fit the sums' 64 bits.)
 //
 // A work item is (a tile of up to BM targets gathered through amap) x (a
 // chunk of sources gathered through bmap).  It forms the rank-k inner
